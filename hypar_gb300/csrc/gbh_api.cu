@@ -834,13 +834,12 @@ extern "C" int gb_solver_get_launch(gb_solver* s, int dir, int* seg, int* block)
   return GB_OK;
 }
 
-// Launch-shape autotuner.  The fused kernels are bound by the FP64 pipe, which
-// a few warps per SM saturate, so the shape mostly decides how evenly the
-// walk segments spread over the SMs (a partial last wave idles SMs) against the
-// per-segment overhead (a six-cell window warm-up and one extra interface).
-// Candidates: segment lengths that give 1..4 full waves of 4 warps per SM, plus
-// fixed lengths; each is timed on `reps` steps of the resident solution, which
-// is restored afterwards.
+// Launch-shape autotuner: each candidate is timed on `reps` steps of the resident
+// solution, which is restored afterwards.  The float-pair kernels take the most threads
+// per block from the shape (pair_cap_of); the FP64 ones (gravity, Steger-Warming, CRWENO5)
+// walk segments, where an even spread over the SMs (a partial last wave idles SMs) stands
+// against the per-segment overhead (a six-cell window warm-up and one extra interface):
+// segment lengths that give 1..4 full waves of 4 warps per SM, plus fixed lengths.
 extern "C" int gb_solver_autotune(gb_solver* s, int reps) {
   if (!s) { gbh_set_error("null solver"); return GB_ERR_ARG; }
   if (reps < 1) reps = 1;
@@ -870,26 +869,29 @@ extern "C" int gb_solver_autotune(gb_solver* s, int reps) {
     for (int e = 0; e < c.ndims; e++)
       if (e != d) ntrans *= c.dim[e];
     std::vector<int> segs;
-    for (int w = 1; w <= 4; w++) {
+    const bool pairs = !s->gravity && c.hyp_scheme == GB_SCHEME_WENO5 && c.upwind != UPW_SWFS;
+    for (int w = 1; w <= 4 && !pairs; w++) {
       double lanes = (double)w * sms * 4 * 32;
       long long nseg = (long long)(lanes / (double)ntrans + 0.5);
       if (nseg < 1) nseg = 1;
       int sg = (int)((N + nseg - 1) / nseg);
       segs.push_back(sg);
     }
-    for (int sg : {8, 16, 24, 32, 48, 64}) segs.push_back(sg);
+    if (pairs) segs = {32, -128};  // (32, 128): by the grid's size; (32, 64): 64; -128: 128
+    else
+      for (int sg : {8, 16, 24, 32, 48, 64}) segs.push_back(sg);
     // Small grids (at most four waves of 4 warps per SM at one interface per
     // thread) cannot fill the SMs with long segments: there, also 1-3
     // interfaces per thread and 32-thread blocks, spreading the few threads
     // over more SMs at the price of recomputing the segments' first interfaces.
-    const bool small = (double)ntrans * N <= 4.0 * sms * 4 * 32;
+    const bool small = !pairs && (double)ntrans * N <= 4.0 * sms * 4 * 32;
     if (small)
       for (int sg : {1, 2, 3}) segs.push_back(sg);
     std::vector<int> blocks = {128, 64};
     if (small) blocks.push_back(32);
     // shared-memory tiles of 32 / 64 / 128 interfaces (seg = -tile; not with gravity
     // or CRWENO5, whose kernels have no tile form)
-    if (!s->gravity && c.hyp_scheme == GB_SCHEME_WENO5)
+    if (!pairs && !s->gravity && c.hyp_scheme == GB_SCHEME_WENO5)
       for (int ti : {32, 64, 128}) segs.push_back(-ti);
     // lane groups of 8 / 16 interfaces (Euler1D component-wise: short lines)
     if (!s->gravity && c.hyp_scheme == GB_SCHEME_WENO5 && c.model == GB_MODEL_EULER1D &&
@@ -898,8 +900,8 @@ extern "C" int gb_solver_autotune(gb_solver* s, int reps) {
     double best = 1e30;
     HypLaunch bestL = s->hl[d];
     for (int sg : segs) {
-      if (sg > 0 && (sg < (small ? 1 : 4) || sg > N)) continue;
-      if (sg < 0 && -sg > 2 * (N + 1)) continue;
+      if (!pairs && sg > 0 && (sg < (small ? 1 : 4) || sg > N)) continue;
+      if (!pairs && sg < 0 && -sg > 2 * (N + 1)) continue;
       for (int blk : blocks) {
         if (sg < 0 && blk != blocks[0]) continue;  // a tile's block is the tile
         s->hl[d].seg = sg;

@@ -6,27 +6,24 @@
 // All members share the model, schemes, time step and Butcher table (as in the
 // reference, where they share solver.inp); sizes, boundaries and initial data
 // are per member.  Their arrays are concatenated; every Runge-Kutta stage is
-// one launch per direction over all members (each thread finds its member in a
-// table of thread offsets), and a whole step is captured once in a CUDA graph
-// and replayed.  The launch form per direction -- segment walker (one thread per
-// segment of a grid line) or tiles of 32/64/128 interfaces (one block per tile,
-// set as a negative segment length) -- is chosen by timing.
+// one launch per direction over all members (each block finds its member in a
+// table of block offsets), and a whole step is captured once in a CUDA graph
+// and replayed.  The launch shape (segment length, tile, block) sets the most threads
+// per block (pair_cap_of).
 #include <algorithm>
 #include <cstring>
 #include <vector>
 
 #include "gbh_internal.h"
+#include "gbh_pair_plan.h"
 
 namespace gbh {
-cudaError_t launch_batched_euler1d(int, int, int, const MemberDev*, int, long long, const double*, double*,
-                                   const double*, const PhysParams&, const StageEpi&, int, int, unsigned long long*,
-                                   cudaStream_t);
-cudaError_t launch_batched_euler2d(int, int, int, const MemberDev*, int, long long, const double*, double*,
-                                   const double*, const PhysParams&, const StageEpi&, int, int, unsigned long long*,
-                                   cudaStream_t);
-cudaError_t launch_batched_ns3d(int, int, int, const MemberDev*, int, long long, const double*, double*,
-                                const double*, const PhysParams&, const StageEpi&, int, int, unsigned long long*,
-                                cudaStream_t);
+cudaError_t launch_batched_euler1d(int, int, int, const MemberDev*, int, long long, int, const double*, double*,
+                                   const double*, const PhysParams&, const StageEpi&, cudaStream_t);
+cudaError_t launch_batched_euler2d(int, int, int, const MemberDev*, int, long long, int, const double*, double*,
+                                   const double*, const PhysParams&, const StageEpi&, cudaStream_t);
+cudaError_t launch_batched_ns3d(int, int, int, const MemberDev*, int, long long, int, const double*, double*,
+                                const double*, const PhysParams&, const StageEpi&, cudaStream_t);
 cudaError_t launch_pack(double*, const double*, const DevGeom&, int, int, cudaStream_t);
 }  // namespace gbh
 
@@ -56,12 +53,10 @@ struct gb_ensemble {
   double* d_stage = nullptr;
   size_t stage_vals = 0;
   long long total_vals = 0, total_dx = 0;
-  long long total_thr[3] = {0, 0, 0};
+  long long total_blk[3] = {0, 0, 0};
+  int threads[3] = {0, 0, 0};  // per block: the largest of the members' shapes
   int seg[3] = {32, 32, 32}, block[3] = {128, 128, 128};
-  // tile forms only: the persistent work-list kernel (one counter per stage and
-  // direction, cleared at the start of every step) instead of one block per tile
-  bool persist[3] = {false, false, false};
-  unsigned long long* d_ctr = nullptr;
+  bool persist[3] = {false, false, false};  // block = -1 was asked for (the same blocks)
   double* d_u = nullptr;
   double* d_acc = nullptr;
   double* d_P[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -82,26 +77,33 @@ struct gb_ensemble {
 };
 
 static void rebuild_table(gb_ensemble* e) {
-  for (int d = 0; d < 3; d++) e->total_thr[d] = 0;
+  long long cells = 0;
+  for (int m = 0; m < e->nm; m++) {
+    long long n = 1;
+    for (int k = 0; k < e->base.ndims; k++) n *= e->mem[m].G.dim[k];
+    cells += n;
+  }
+  for (int d = 0; d < 3; d++) {
+    e->total_blk[d] = 0;
+    e->threads[d] = 0;
+  }
   for (int m = 0; m < e->nm; m++) {
     MemberDev& md = e->mem[m];
     for (int d = 0; d < 3; d++) {
-      md.seg[d] = e->seg[d];
-      if (d >= e->base.ndims) {
-        md.ntrans[d] = 0;
-        md.nseg[d] = 0;
-        md.start[d] = e->total_thr[d];
-        continue;
-      }
+      md.start[d] = e->total_blk[d];
+      md.ntrans[d] = 0;
+      md.L[d] = md.XL[d] = 1;
+      if (d >= e->base.ndims) continue;
       long long ntr = 1;
       for (int k = 0; k < e->base.ndims; k++)
         if (k != d) ntr *= md.G.dim[k];
       md.ntrans[d] = ntr;
-      // walker: threads (segments x lines); tiles: blocks (tiles x lines)
-      const int ti = -e->seg[d];
-      md.nseg[d] = e->seg[d] > 0 ? (md.G.dim[d] + e->seg[d] - 1) / e->seg[d] : (md.G.dim[d] + ti - 2) / (ti - 1);
-      md.start[d] = e->total_thr[d];
-      e->total_thr[d] += ntr * md.nseg[d];
+      const int cap = pair_cap_of(e->seg[d], e->block[d]);
+      const PairPlan p = pair_plan(md.G.dim[d], ntr, d, cap > 0 ? cap : pair_cap(cells));
+      md.L[d] = p.L;
+      md.XL[d] = p.XL;
+      if (p.T > e->threads[d]) e->threads[d] = p.T;
+      e->total_blk[d] += (ntr + p.XL - 1) / p.XL * ((md.G.dim[d] + p.L - 1) / p.L);
     }
   }
 }
@@ -116,17 +118,15 @@ static int upload_table(gb_ensemble* e) {
 
 static cudaError_t launch_dir(gb_ensemble* e, int st, int d, const double* U, const StageEpi& ep) {
   const gb_config& c = e->base;
-  const int tile = e->seg[d] < 0 ? -e->seg[d] : 0;
-  unsigned long long* ctr = (tile && e->persist[d]) ? e->d_ctr + 3 * st + d : nullptr;
-  if (tile && !ctr && e->total_thr[d] > 0x7fffffffLL) return cudaErrorInvalidConfiguration;  // one block per tile
+  (void)st;
   if (c.model == GB_MODEL_EULER1D)
-    return launch_batched_euler1d(d, c.interp, c.upwind, e->d_mem, e->nm, e->total_thr[d], U, e->d_H, e->d_dx,
-                                  e->pp, ep, e->block[d], tile, ctr, e->stream);
+    return launch_batched_euler1d(d, c.interp, c.upwind, e->d_mem, e->nm, e->total_blk[d], e->threads[d], U, e->d_H,
+                                  e->d_dx, e->pp, ep, e->stream);
   if (c.model == GB_MODEL_EULER2D)
-    return launch_batched_euler2d(d, c.interp, c.upwind, e->d_mem, e->nm, e->total_thr[d], U, e->d_H, e->d_dx,
-                                  e->pp, ep, e->block[d], tile, ctr, e->stream);
-  return launch_batched_ns3d(d, c.interp, c.upwind, e->d_mem, e->nm, e->total_thr[d], U, e->d_H, e->d_dx, e->pp,
-                             ep, e->block[d], tile, ctr, e->stream);
+    return launch_batched_euler2d(d, c.interp, c.upwind, e->d_mem, e->nm, e->total_blk[d], e->threads[d], U, e->d_H,
+                                  e->d_dx, e->pp, ep, e->stream);
+  return launch_batched_ns3d(d, c.interp, c.upwind, e->d_mem, e->nm, e->total_blk[d], e->threads[d], U, e->d_H,
+                             e->d_dx, e->pp, ep, e->stream);
 }
 
 // The launches of one Runge-Kutta step (ns stages x ndims directions).
@@ -134,8 +134,6 @@ static int step_launches(gb_ensemble* e) {
   const gb_config& c = e->base;
   const int ns = c.rk_nstages;
   int touched[4] = {0, 0, 0, 0};
-  if (e->persist[0] || e->persist[1] || e->persist[2])
-    CK(cudaMemsetAsync(e->d_ctr, 0, sizeof(unsigned long long) * 12, e->stream));
   for (int st = 0; st < ns; st++) {
     double* U = (st == 0 || !touched[st]) ? e->d_u : e->d_P[st];
     StageEpi ep;
@@ -266,7 +264,6 @@ extern "C" int gb_ensemble_create(const gb_config* cfgs, const double* const* dx
   if (e->base.ndims > 1) A(&e->d_H, bytes);
   A(&e->d_dx, dxo * sizeof(double));
   if (ce == cudaSuccess) ce = cudaMalloc((void**)&e->d_mem, sizeof(MemberDev) * nsims);
-  if (ce == cudaSuccess) ce = cudaMalloc((void**)&e->d_ctr, sizeof(unsigned long long) * 12);
   if (ce == cudaSuccess) ce = cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking);
   if (ce == cudaSuccess) e->own_stream = true;
   for (int m = 0; m < nsims && ce == cudaSuccess; m++) {
@@ -299,7 +296,6 @@ extern "C" void gb_ensemble_destroy(gb_ensemble* e) {
   cudaFree(e->d_H);
   cudaFree(e->d_dx);
   cudaFree(e->d_mem);
-  cudaFree(e->d_ctr);
   cudaFree(e->d_bnd);
   cudaFree(e->d_red);
   if (e->own_stream && e->stream) cudaStreamDestroy(e->stream);
@@ -463,7 +459,7 @@ extern "C" int gb_ensemble_get_launch(gb_ensemble* e, int dir, int* seg, int* bl
 
 extern "C" double gb_ensemble_time(const gb_ensemble* e) { return e ? e->t : 0.0; }
 
-// Segment length / block per direction by timing whole graph-replayed steps
+// Threads per block and direction by timing whole graph-replayed steps
 // (directions tuned one after the other); the state is restored afterwards.
 extern "C" int gb_ensemble_autotune(gb_ensemble* e, int reps) {
   if (!e) { gbh_set_error("null ensemble"); return GB_ERR_ARG; }
@@ -480,40 +476,29 @@ extern "C" int gb_ensemble_autotune(gb_ensemble* e, int reps) {
   CK(cudaEventCreate(&a));
   CK(cudaEventCreate(&b));
   int rc = GB_OK;
-  const int cand[] = {8, 12, 16, 20, 24, 27, 32, 40, 48, 54, 64, -32, -64, -128};
+  // (32, 128): blocks of up to 256 threads on large ensembles; -128, -64: of up to 128 / 64
   for (int d = 0; d < e->base.ndims && !rc; d++) {
     float best = 1e30f;
-    int bs = e->seg[d], bb = e->block[d];
-    bool bp = e->persist[d];
-    for (int sg : cand) {
-      for (int blk : {128, 64, -1}) {
-        // a tile's block is its interfaces; -1: the tile's persistent work-list form
-        if (sg < 0 && blk == 64) continue;
-        if (sg > 0 && blk < 0) continue;
-        e->seg[d] = sg;
-        e->block[d] = blk > 0 ? blk : 128;
-        e->persist[d] = blk < 0;
-        rc = upload_table(e);
-        if (!rc) rc = gb_ensemble_step(e, 1);
-        if (rc) break;
-        CK(cudaEventRecord(a, e->stream));
-        rc = gb_ensemble_step(e, reps);
-        CK(cudaEventRecord(b, e->stream));
-        CK(cudaEventSynchronize(b));
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, a, b);
-        if (!rc && ms < best) {
-          best = ms;
-          bs = sg;
-          bb = e->block[d];
-          bp = e->persist[d];
-        }
-      }
+    int bs = e->seg[d];
+    e->block[d] = 128;
+    e->persist[d] = false;
+    for (int sg : {32, -128, -64}) {
+      e->seg[d] = sg;
+      rc = upload_table(e);
+      if (!rc) rc = gb_ensemble_step(e, 1);
       if (rc) break;
+      CK(cudaEventRecord(a, e->stream));
+      rc = gb_ensemble_step(e, reps);
+      CK(cudaEventRecord(b, e->stream));
+      CK(cudaEventSynchronize(b));
+      float ms = 0.f;
+      cudaEventElapsedTime(&ms, a, b);
+      if (!rc && ms < best) {
+        best = ms;
+        bs = sg;
+      }
     }
     e->seg[d] = bs;
-    e->block[d] = bb;
-    e->persist[d] = bp;
     if (!rc) rc = upload_table(e);
   }
   cudaEventDestroy(a);

@@ -17,6 +17,7 @@
 #pragma once
 
 #include "gbh_internal.h"
+#include "gbh_pair_plan.h"
 
 namespace gbh {
 
@@ -1037,122 +1038,23 @@ __device__ __forceinline__ const MemberDev& batched_member(const MemberDev* __re
   return m;
 }
 
+// All members in one launch (gbh_pair_flux.cuh): nblk blocks of T threads.
 template <int M, bool CHAR, int UPW, int DIR>
-__global__ void __launch_bounds__(128)
-hyp_batched_kernel(const MemberDev* __restrict__ mem, int nmem, long long total, const double* __restrict__ U,
-                   double* __restrict__ H, const double* __restrict__ dxinv, PhysParams pp, StageEpi ep) {
-  long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (tid >= total) return;
-  StageEpi e = ep;
-  const MemberDev& m = batched_member<DIR>(mem, nmem, tid, e);
-  long long lt = tid - m.start[DIR];
-  long long ntr = m.ntrans[DIR];
-  const long long o = m.off;
-  hyp_segment<M, CHAR, UPW, DIR>(U + o, H ? H + o : nullptr, dxinv + m.dx_off[DIR], m.G, pp, e, m.seg[DIR],
-                                 lt % ntr, (int)(lt / ntr));
-}
-
-// Tile form of the batched kernel: one block per tile of TI interfaces of one
-// member's grid line; the members' tables count blocks instead of threads.
-template <int M, bool CHAR, int UPW, int DIR, int TI>
-__global__ void __launch_bounds__(TI)
-hyp_batched_tile_kernel(const MemberDev* __restrict__ mem, int nmem, const double* __restrict__ U,
-                        double* __restrict__ H, const double* __restrict__ dxinv, PhysParams pp, StageEpi ep) {
-  StageEpi e = ep;
-  const long long b = blockIdx.x;
-  const MemberDev& m = batched_member<DIR>(mem, nmem, b, e);
-  const long long o = m.off;
-  hyp_tile_body<M, CHAR, UPW, DIR, false, TI, false>(U + o, H ? H + o : nullptr, dxinv + m.dx_off[DIR], m.G, pp,
-                                                     e, m.ntrans[DIR], b - m.start[DIR]);
-}
-
-// Persistent work-list form of the batched tile kernel: a grid of as many blocks as
-// the SMs hold at once pulls tile indices from a work counter (one atomicAdd per
-// tile, by one thread of the block) until the launch's `total` tiles are taken.  The
-// loop is bounded: every fetch takes a new index, so a block stops after at most
-// total / gridDim + 1 fetches.  `counter` is zero when the launch starts.
-template <int M, bool CHAR, int UPW, int DIR, int TI>
-__global__ void __launch_bounds__(TI)
-hyp_batched_worklist_kernel(const MemberDev* __restrict__ mem, int nmem, long long total,
-                            unsigned long long* __restrict__ counter, const double* __restrict__ U,
-                            double* __restrict__ H, const double* __restrict__ dxinv, PhysParams pp, StageEpi ep) {
-  __shared__ long long s_tile;
-  for (;;) {
-    if (threadIdx.x == 0) s_tile = (long long)atomicAdd(counter, 1ULL);
-    __syncthreads();
-    const long long b = s_tile;
-    __syncthreads();  // every thread holds b before thread 0 fetches the next one
-    if (b >= total) return;
-    StageEpi e = ep;
-    const MemberDev& m = batched_member<DIR>(mem, nmem, b, e);
-    const long long o = m.off;
-    hyp_tile_body<M, CHAR, UPW, DIR, false, TI, false>(U + o, H ? H + o : nullptr, dxinv + m.dx_off[DIR], m.G, pp,
-                                                       e, m.ntrans[DIR], b - m.start[DIR]);
-  }
-}
-
-template <typename K>
-unsigned worklist_grid(K kernel, int threads, long long total) {
-  int dev = 0, sms = 0, per = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, 0);
-  long long g = (long long)(per > 0 ? per : 1) * (sms > 0 ? sms : 1);
-  return (unsigned)(g < total ? g : total);
-}
-
-// total = threads (walker, tile == 0) or blocks (tiles of `tile` interfaces).
-// counter != nullptr with a tile form: the persistent work-list kernel.
-template <int M, bool CHAR, int UPW, int DIR>
-cudaError_t launch_batched_dir(const MemberDev* mem, int nmem, long long total, const double* U, double* H,
-                               const double* dxinv, const PhysParams& pp, const StageEpi& ep, int block, int tile,
-                               unsigned long long* counter, cudaStream_t s) {
-  if (total <= 0) return cudaSuccess;
-  if (counter && tile) {
-#define GBH_WL(TI)                                                                                       \
-  do {                                                                                                   \
-    auto k = hyp_batched_worklist_kernel<M, CHAR, UPW, DIR, TI>;                                         \
-    k<<<worklist_grid(k, TI, total), TI, 0, s>>>(mem, nmem, total, counter, U, H, dxinv, pp, ep);        \
-  } while (0)
-    if (tile == 32) GBH_WL(32);
-    else if (tile == 64) GBH_WL(64);
-    else if (tile == 128) GBH_WL(128);
-    else return cudaErrorInvalidValue;
-#undef GBH_WL
-    return cudaGetLastError();
-  }
-  if (tile == 32)
-    hyp_batched_tile_kernel<M, CHAR, UPW, DIR, 32><<<(unsigned)total, 32, 0, s>>>(mem, nmem, U, H, dxinv, pp, ep);
-  else if (tile == 64)
-    hyp_batched_tile_kernel<M, CHAR, UPW, DIR, 64><<<(unsigned)total, 64, 0, s>>>(mem, nmem, U, H, dxinv, pp, ep);
-  else if (tile == 128)
-    hyp_batched_tile_kernel<M, CHAR, UPW, DIR, 128><<<(unsigned)total, 128, 0, s>>>(mem, nmem, U, H, dxinv, pp, ep);
-  else if (tile != 0)
-    return cudaErrorInvalidValue;
-  else {
-    if (block <= 0) block = 128;
-    long long grid = (total + block - 1) / block;
-    hyp_batched_kernel<M, CHAR, UPW, DIR><<<(unsigned)grid, block, 0, s>>>(mem, nmem, total, U, H, dxinv, pp, ep);
-  }
-  return cudaGetLastError();
-}
+cudaError_t launch_batched_dir(const MemberDev* mem, int nmem, long long nblk, int T, const double* U, double* H,
+                               const double* dxinv, const PhysParams& pp, const StageEpi& ep, cudaStream_t s);
 
 template <int M>
-cudaError_t launch_batched_model(int dir, int chr, int upw, const MemberDev* mem, int nmem, long long total,
+cudaError_t launch_batched_model(int dir, int chr, int upw, const MemberDev* mem, int nmem, long long nblk, int T,
                                  const double* U, double* H, const double* dxinv, const PhysParams& pp,
-                                 const StageEpi& ep, int block, int tile, unsigned long long* counter,
-                                 cudaStream_t s) {
+                                 const StageEpi& ep, cudaStream_t s) {
   constexpr int ND = ModelTraits<M>::ND;
 #define GBH_B(C, W)                                                                                          \
   do {                                                                                                       \
-    if (dir == 0)                                                                                            \
-      return launch_batched_dir<M, C, W, 0>(mem, nmem, total, U, H, dxinv, pp, ep, block, tile, counter, s); \
+    if (dir == 0) return launch_batched_dir<M, C, W, 0>(mem, nmem, nblk, T, U, H, dxinv, pp, ep, s);         \
     if (ND > 1 && dir == 1)                                                                                  \
-      return launch_batched_dir<M, C, W, (ND > 1 ? 1 : 0)>(mem, nmem, total, U, H, dxinv, pp, ep, block, tile, \
-                                                           counter, s);                                      \
+      return launch_batched_dir<M, C, W, (ND > 1 ? 1 : 0)>(mem, nmem, nblk, T, U, H, dxinv, pp, ep, s);      \
     if (ND > 2 && dir == 2)                                                                                  \
-      return launch_batched_dir<M, C, W, (ND > 2 ? 2 : 0)>(mem, nmem, total, U, H, dxinv, pp, ep, block, tile, \
-                                                           counter, s);                                      \
+      return launch_batched_dir<M, C, W, (ND > 2 ? 2 : 0)>(mem, nmem, nblk, T, U, H, dxinv, pp, ep, s);      \
     return cudaErrorInvalidValue;                                                                            \
   } while (0)
   // Rusanov: Euler1D and NavierStokes3D (Euler2D offers none); the template
@@ -1172,6 +1074,11 @@ cudaError_t launch_batched_model(int dir, int chr, int upw, const MemberDev* mem
 #undef GBH_B
 }
 
+// The float-pair form (gbh_pair_flux.cuh), which the direction launcher prefers.
+template <int M, bool CHAR, int UPW, int DIR, bool ALTW>
+cudaError_t launch_pair(const double* U, double* H, const double* dxinv_dir, const DevGeom& G, const PhysParams& pp,
+                        const StageEpi& ep, long long ntrans, int cap, cudaStream_t s);
+
 // Host launcher for one direction.
 template <int M, bool CHAR, int UPW, int DIR, bool ALTW, bool GRAV = false, bool WT = false>
 cudaError_t launch_dir(const double* U, double* H, const double* dxinv_dir, const DevGeom& G,
@@ -1190,6 +1097,14 @@ cudaError_t launch_dir(const double* U, double* H, const double* dxinv_dir, cons
       return cudaGetLastError();
     }
   }
+  // Gravity, Steger-Warming and the adjoint's tapes: the FP64 kernels.
+  constexpr bool PAIR = !GRAV && !WT && UPW != UPW_SWFS;
+  constexpr bool TAPE = M == MODEL_EULER2D && !CHAR && UPW == UPW_ROE && !ALTW;
+  if constexpr (PAIR) {
+    if (!TAPE || !ep.tape)
+      return launch_pair<M, CHAR, UPW, DIR, ALTW>(U, H, dxinv_dir, G, pp, ep, ntrans, pair_cap_of(L.seg, L.block), s);
+  }
+  if constexpr (!PAIR || TAPE) {
   if (L.seg < 0 && !GRAV) {
     // tiles of -seg interfaces (32, 64 or 128), one block each
     const int ti = -L.seg;
@@ -1220,6 +1135,7 @@ cudaError_t launch_dir(const double* U, double* H, const double* dxinv_dir, cons
   hyp_dir_kernel<M, CHAR, UPW, DIR, ALTW, GRAV, WT><<<(unsigned)grid, block, 0, s>>>(U, H, dxinv_dir, G, pp, ep,
                                                                                   seg, nseg, ntrans);
   return cudaGetLastError();
+  }
 }
 
 template <int M, bool CHAR, int UPW, bool ALTW, bool GRAV = false>
@@ -1529,3 +1445,5 @@ cudaError_t launch_unfused_model(int kind, int dir, int upw, double* out, const 
 }
 
 }  // namespace gbh
+
+#include "gbh_pair_flux.cuh"

@@ -82,15 +82,15 @@ struct HypLaunch {
 };
 
 // Ensemble member as seen by the batched kernel: its geometry, where its
-// arrays start inside the batched arrays, and which threads of a launch along
-// each direction are its (start[d] .. start[d] + ntrans[d]*nseg[d]).
+// arrays start inside the batched arrays, which blocks of a launch along each direction
+// are its (from start[d]) and their shape (PairPlan in gbh_pair_flux.cuh).
 struct MemberDev {
   DevGeom G;
   long long off;         // first value of the member in every state array
   long long dx_off[3];   // first dxinv value of each direction
-  long long start[3];    // first thread of the member per direction
+  long long start[3];    // first block of the member per direction
   long long ntrans[3];
-  int nseg[3], seg[3];
+  int L[3], XL[3];
   long long bnd_off[3];  // the member's conservation-check accumulators per direction
 };
 

@@ -1,0 +1,679 @@
+// gbh_pair_flux.cuh -- the fused hyperbolic kernel with the small terms in float pairs.
+//
+// HyPar's interface flux (ReconstructHyperbolic, HyperbolicFunction.c:167-222: WENO5 of
+// fL, fR, uL, uR and the upwind scheme) is written as
+//   F_{j+1/2} = (-f_{j-1} + 7 f_j + 7 f_{j+1} - f_{j+2}) / 12 + G_{j+1/2},
+// the fourth-order central value and a correction G: the nonlinear weights' deviation from
+// it and the upwind dissipation.  Both parts of G are combinations of third differences
+// (gbh_pair.cuh), small against the flux wherever the solution is resolved.  The central
+// part (and the cells' fluxes and primitives) is computed in FP64, G in pairs of FP32
+// numbers, whose arithmetic has 64 times the FP64 pipe's throughput on GB300.
+//
+// What bounds the error: a pair carries 48 bits, the chain from the differences to G loses
+// two or three of them, so G is off by some 2^-46 of the magnitude of its terms.  Where
+// those terms exceed 2^-7 of the interface's flux scale (rho lam, rho lam^2, rho lam H
+// with lam = |u_n| + a), the scale leaves the range 2^-60 .. 2^100, a weight's sum leaves
+// its own, or anything is not finite, the interface takes the FP64 evaluation
+// (iface_flux) instead: shocks, contacts, under-resolved fields, odd units.  The decision
+// uses the interface's own window only, so every kernel that evaluates an interface takes
+// the same one and neighbouring blocks agree on the flux between them.
+#pragma once
+
+#include "gbh_pair.cuh"
+
+namespace gbh {
+
+// Eigen-system of a Roe average in pairs (Eig in gbh_device.cuh).
+struct PEig {
+  ff vel[3], un, a, ek, H, hac, rs, gi, lamn;  // gi = (gamma-1)/a^2
+};
+
+// Per-cell ingredients in pairs: sqrt(rho), velocity, enthalpy, wave speed.
+template <int M>
+struct PCell {
+  ff t, vel[3], H, c;
+};
+
+struct PParams {
+  ff gm1, gamma, eps4;
+};
+
+template <int M, int DIR>
+__device__ __forceinline__ void peig_finish(PEig& E, ff rho, const PParams& q) {
+  constexpr int ND = ModelTraits<M>::ND;
+  FAcc v2 = acc_mul(E.vel[0], E.vel[0]);
+#pragma unroll
+  for (int k = 1; k < ND; k++) acc_fma(v2, E.vel[k], E.vel[k]);
+  E.ek = mul2(acc_get(v2), 0.5f);
+  const ff a2 = q.gm1 * (E.H - E.ek);
+  const ff ia = rsqrt(a2);
+  E.a = a2 * ia;
+  const ff ia2 = sqr(ia);
+  E.un = E.vel[DIR];
+  E.hac = mul2(ia2, 0.5f);
+  E.rs = ff{1.0f, 0.0f};
+  if (M == MODEL_EULER1D) {  // hac = 1/(rho a), rs = rho/(2a)
+    E.hac = rcp(rho) * ia;
+    E.rs = mul2(rho * ia, 0.5f);
+  }
+  E.gi = q.gm1 * ia2;
+}
+
+// Roe average of two cells (or states) given by their ingredients.
+template <int M, int DIR>
+__device__ __forceinline__ PEig peig(const PCell<M>& L, const PCell<M>& R, const PParams& q) {
+  constexpr int ND = ModelTraits<M>::ND;
+  PEig E;
+  const ff th = R.t * rcp(L.t + R.t);  // weight of the right state
+#pragma unroll
+  for (int k = 0; k < ND; k++) E.vel[k] = L.vel[k] + th * (R.vel[k] - L.vel[k]);
+  E.H = L.H + th * (R.H - L.H);
+  peig_finish<M, DIR>(E, L.t * R.t, q);
+  return E;
+}
+
+// Ingredients of a conserved state (c: its sound speed).
+template <int M>
+__device__ __forceinline__ PCell<M> pcell(const ff* u, const PParams& q, bool want_c) {
+  constexpr int ND = ModelTraits<M>::ND, NV = ModelTraits<M>::NV;
+  PCell<M> s;
+  const ff rinv = rcp(u[0]);
+  s.t = u[0] * rsqrt(u[0]);
+#pragma unroll
+  for (int k = 0; k < ND; k++) s.vel[k] = u[1 + k] * rinv;
+  FAcc m = acc_mul(u[1], s.vel[0]);
+#pragma unroll
+  for (int k = 1; k < ND; k++) acc_fma(m, u[1 + k], s.vel[k]);
+  const ff P = q.gm1 * (u[NV - 1] - mul2(acc_get(m), 0.5f));
+  s.H = (u[NV - 1] + P) * rinv;
+  s.c = ff{0.0f, 0.0f};
+  if (want_c) {
+    const ff c2 = q.gamma * (P * rinv);
+    s.c = c2 * rsqrt(c2);
+  }
+  return s;
+}
+
+// R diag(c0, c1, c2, ..., c2) L x in the eigen-system E, fields as in projL (0: u_n - a,
+// 1: u_n + a, the rest u_n): since R L = I this is c2 x + (c0 - c2) w0 r0 + (c1 - c2) w1 r1.
+template <int M, int DIR>
+__device__ __forceinline__ void pdissip(const PEig& E, const PParams& q, const ff* x, ff c0, ff c1, ff c2, ff* y) {
+  constexpr int ND = ModelTraits<M>::ND, NV = ModelTraits<M>::NV;
+  FAcc sa = acc_mul(E.ek, x[0]);
+#pragma unroll
+  for (int k = 0; k < ND; k++) acc_fma(sa, neg(E.vel[k]), x[1 + k]);
+  acc_add(sa, x[NV - 1]);
+  const ff h2 = mul2(E.gi, 0.5f);  // (gamma-1)/(2 a^2)
+  const ff s = h2 * acc_get(sa);
+  // t/(2 a^2) = (u_n x_0 - x_n)/(2a), and 1/(2a) = a (gamma-1)/(2a^2) / (gamma-1)
+  const ff th = E.lamn * (E.un * x[0] - x[1 + DIR]);
+  const ff p0 = (c0 - c2) * (s + th), p1 = (c1 - c2) * (s - th);
+  const ff sum = p0 + p1, dif = E.a * (p1 - p0);
+  FAcc r = acc_mul(c2, x[0]);
+  acc_add(r, sum);
+  y[0] = acc_get(r);
+#pragma unroll
+  for (int k = 0; k < ND; k++) {
+    r = acc_mul(c2, x[1 + k]);
+    acc_fma(r, E.vel[k], sum);
+    if (k == DIR) acc_add(r, dif);
+    y[1 + k] = acc_get(r);
+  }
+  r = acc_mul(c2, x[NV - 1]);
+  acc_fma(r, E.H, sum);
+  acc_fma(r, E.un, dif);
+  y[NV - 1] = acc_get(r);
+}
+
+// 1/(2a), which pdissip's acoustic strengths need.
+__device__ __forceinline__ void peig_upwind(PEig& E, const PParams&) { E.lamn = mul2(rcp(E.a), 0.5f); }
+
+template <int M, int DIR>
+__device__ __forceinline__ void pprojL(const PEig& E, const PParams& q, const ff* x, ff* w) {
+  constexpr int ND = ModelTraits<M>::ND, NV = ModelTraits<M>::NV;
+  FAcc sa = acc_mul(E.ek, x[0]);
+#pragma unroll
+  for (int k = 0; k < ND; k++) acc_fma(sa, neg(E.vel[k]), x[1 + k]);
+  acc_add(sa, x[NV - 1]);
+  const ff s = acc_get(sa);
+  const ff gs = (q.gm1 * E.hac) * s, th = (E.a * E.hac) * (E.un * x[0] - x[1 + DIR]);
+  w[0] = gs + th;
+  w[1] = gs - th;
+  w[2] = x[0] - E.gi * s;
+  int j = 3;
+#pragma unroll
+  for (int k = 0; k < ND; k++)
+    if (k != DIR) w[j++] = E.vel[k] * x[0] - x[1 + k];
+}
+
+template <int M, int DIR>
+__device__ __forceinline__ void pprojR(const PEig& E, const ff* w, ff* y) {
+  constexpr int ND = ModelTraits<M>::ND, NV = ModelTraits<M>::NV;
+  ff Wm = w[0], Wp = w[1];
+  if (M == MODEL_EULER1D) {
+    Wm = Wm * E.rs;
+    Wp = Wp * E.rs;
+  }
+  const ff sa = Wm + Wp, da = E.a * (Wp - Wm);
+  const ff y0 = sa + w[2];
+  FAcc yE = acc_mul(E.H, sa);
+  acc_fma(yE, E.un, da);
+  acc_fma(yE, E.ek, w[2]);
+  int j = 3;
+#pragma unroll
+  for (int k = 0; k < ND; k++) {
+    FAcc r = acc_mul(E.vel[k], y0);
+    if (k == DIR) {
+      acc_add(r, da);
+    } else {
+      acc_add(r, neg(w[j]));
+      acc_fma(yE, neg(E.vel[k]), w[j]);
+      j++;
+    }
+    y[1 + k] = acc_get(r);
+  }
+  y[0] = y0;
+  y[NV - 1] = acc_get(yE);
+}
+
+__device__ __forceinline__ ff pharten(ff lam) {
+  ff d = ffabs(lam);
+  if (d.h < 0.000001f) d = mulf(sqr(d) + ffc(0.000001 * 0.000001), 500000.0f);
+  return d;
+}
+
+// The reconstructed states' mean central value + us6/12 of component v, from the cell's
+// value, its right difference and the second differences of the two cells.
+__device__ __forceinline__ ff pmean(ff u2, ff dr, ff d2, ff d3, ff us6) {
+  const ff tw = ffc(1.0 / 12.0);
+  return u2 + (mul2(dr, 0.5f) + tw * (us6 - (d2 + d3)));
+}
+
+// Coefficients of one field for LLF / RF: dissipation alpha, or the side taken (sg).
+template <int UPW>
+__device__ __forceinline__ void pfield(ff l, ff c, ff r, ff& al, float& sg) {
+  al = ffmax(ffmax(ffabs(l), ffabs(c)), ffabs(r));
+  sg = 0.0f;
+  if (UPW == UPW_RF) {
+    if (l.h > 0.0f && c.h > 0.0f && r.h > 0.0f) sg = 1.0f;
+    else if (l.h < 0.0f && c.h < 0.0f && r.h < 0.0f) sg = -1.0f;
+    if (sg != 0.0f) al = ff{0.0f, 0.0f};
+  }
+}
+
+// G of one interface times 12 from the conserved sums and differences of the
+// reconstructions (fs6 = 6 (fL + fR - 2 central), fd6 = 6 (fR - fL), ud6 = 6 (uR - uL)),
+// mean states um where the scheme averages the reconstructed states, and the cells'
+// ingredients.  lam, rho, H: the interface's scales.
+template <int M, int UPW, int DIR>
+__device__ __forceinline__ void pupwind(const ff* fs6, const ff* fd6, const ff* ud6, const ff* um, const PEig& Ecc,
+                                        const PCell<M>& cl, const PCell<M>& cr, const PParams& q, ff* g12, float& lam,
+                                        float& rho, float& Hs) {
+  constexpr int NV = ModelTraits<M>::NV, ND = ModelTraits<M>::ND;
+  constexpr bool STATES = (UPW == UPW_ROE && M == MODEL_EULER2D) ||
+                          ((UPW == UPW_LLF || UPW == UPW_RF) && M != MODEL_EULER1D);
+  PEig E;
+  PCell<M> sL, sR;
+  if (STATES) {
+    const ff tw = ffc(1.0 / 12.0);
+    ff a[NV], b[NV];
+#pragma unroll
+    for (int v = 0; v < NV; v++) {
+      const ff h = tw * ud6[v];
+      a[v] = um[v] - h;
+      b[v] = um[v] + h;
+    }
+    sL = pcell<M>(a, q, UPW != UPW_ROE);
+    sR = pcell<M>(b, q, UPW != UPW_ROE);
+    E = peig<M, DIR>(sL, sR, q);
+    rho = um[0].h;
+  } else {
+    E = Ecc;
+    sL = cl;
+    sR = cr;
+    rho = cl.t.h * cr.t.h;
+  }
+  lam = fadd(fabsf(E.un.h), E.a.h);
+  Hs = E.H.h;
+  if (UPW == UPW_RUS) {
+    const ff avg = (M == MODEL_EULER1D ? sqr(E.a) : E.a) + ffabs(E.un);
+    const ff al = ffmax(ffmax(cl.c, cr.c), avg);
+    lam = fmaxf(lam, al.h);
+#pragma unroll
+    for (int v = 0; v < NV; v++) g12[v] = fs6[v] - al * ud6[v];
+    return;
+  }
+  peig_upwind(E, q);
+  ff y[NV];
+  if (UPW == UPW_ROE) {
+    ff c0 = E.un - E.a, c1 = E.un + E.a, c2 = E.un;
+    if (M == MODEL_EULER1D) {
+      c0 = ffabs(c0);
+      c1 = ffabs(c1);
+      c2 = ffabs(c2);
+    } else {
+      c0 = pharten(c0);
+      c1 = pharten(c1);
+      c2 = pharten(c2);
+    }
+    pdissip<M, DIR>(E, q, ud6, c0, c1, c2, y);
+#pragma unroll
+    for (int v = 0; v < NV; v++) g12[v] = fs6[v] - y[v];
+    return;
+  }
+  ff al[3];
+  float sg[3];
+  pfield<UPW>(sL.vel[DIR] - sL.c, E.un - E.a, sR.vel[DIR] - sR.c, al[0], sg[0]);
+  pfield<UPW>(sL.vel[DIR] + sL.c, E.un + E.a, sR.vel[DIR] + sR.c, al[1], sg[1]);
+  pfield<UPW>(sL.vel[DIR], E.un, sR.vel[DIR], al[2], sg[2]);
+  lam = fmaxf(lam, fmaxf(al[0].h, al[1].h));
+  pdissip<M, DIR>(E, q, ud6, al[0], al[1], al[2], y);
+#pragma unroll
+  for (int v = 0; v < NV; v++) g12[v] = fs6[v] - y[v];
+  if (UPW == UPW_RF && (sg[0] != 0.0f || sg[1] != 0.0f || sg[2] != 0.0f)) {
+    // fields taken from one side: (fL - fR)/2 more, or less, than the mean
+    pdissip<M, DIR>(E, q, fd6, ff{sg[0], 0.0f}, ff{sg[1], 0.0f}, ff{sg[2], 0.0f}, y);
+#pragma unroll
+    for (int v = 0; v < NV; v++) g12[v] = g12[v] - y[v];
+  }
+  (void)ND;
+}
+
+// The FP64 evaluation of one interface (window in shared memory, own cell = slot w) as
+// the correction G, written to G[v S].
+template <int M, bool CHAR, int UPW, int DIR, bool ALTW>
+__device__ __forceinline__ void iface_fp64(const double* su, const double* sf, int S, int w, const PhysParams& pp,
+                                           double* G) {
+  constexpr int NV = ModelTraits<M>::NV;
+  double wu[6][NV], wf[6][NV], wuc[6], wgf[6], wgg[6], fI[NV], SI[NV];
+  CellAux<M> ax[6];
+#pragma unroll
+  for (int p = 0; p < 6; p++) {
+#pragma unroll
+    for (int v = 0; v < NV; v++) {
+      wu[p][v] = su[v * S + w - 2 + p];
+      wf[p][v] = sf[v * S + w - 2 + p];
+    }
+    const Prim<M> q = to_prim<M>(wu[p], pp);
+    wuc[p] = ufunc_energy<M>(q, pp, wu[p][NV - 1]);
+    if (p == 2 || p == 3) {
+      ax[p].rs = roe_side<M>(q);
+      if (UPW == UPW_RUS) ax[p].c = rusanov_speed<M, DIR>(q, pp);
+      else if (M == MODEL_EULER1D && UPW != UPW_ROE) ax[p].c = sound_speed<M>(q, pp);
+    }
+  }
+  StageEpi ep;
+  ep.tape = nullptr;
+  iface_flux<M, CHAR, UPW, DIR, ALTW, false, false>(wu, wf, wuc, wgf, wgg, ax, pp, ep, 4.0 * pp.eps, false, 0, fI, SI);
+#pragma unroll
+  for (int v = 0; v < NV; v++) {
+    const double d1 = wf[2][v] - wf[1][v], d2 = wf[3][v] - wf[2][v], d3 = wf[4][v] - wf[3][v];
+    G[v * S] = fI[v] - fma(6.0, d2, d1 - d3) * (1.0 / 12.0);
+  }
+}
+
+// Shared memory of a block of T threads (slots S = T + 4): u and f (doubles), their right
+// differences (pairs), the cells' ingredients, and for the component-wise form one
+// component's sub-stencil rows, double-buffered.
+template <int M, bool CHAR, int UPW, bool ALTW>
+struct PairLayout {
+  static constexpr int NV = ModelTraits<M>::NV, ND = ModelTraits<M>::ND;
+  static constexpr bool CC = NeedCC<M, CHAR, UPW>::value;
+  static constexpr bool NEEDC = UPW == UPW_RUS || (M == MODEL_EULER1D && UPW != UPW_ROE);
+  static constexpr int NA = (CC ? ND + 2 : 0) + (NEEDC ? 1 : 0);
+  static constexpr int NR = ALTW ? 6 : 4;                // pairs of a row
+  static constexpr int NROW = CHAR ? 0 : 2 * 2 * NR;     // two buffers of the f and u rows
+  static constexpr int WORDS = 2 * NV + 2 * NV + NA + NROW;  // 8-byte words per slot
+  static size_t bytes(int T) { return (size_t)WORDS * (T + 4) * 8; }
+};
+
+// One block: XL neighbouring grid lines times L cells of each, LL = L + 6 slots per line,
+// one thread per slot.  A thread owns a cell and the interface to its right.  sm is not
+// __restrict__: the barriers order other threads' accesses to it, and a pointer that is
+// said to have no alias lets the compiler move its loads and stores across them.
+template <int M, bool CHAR, int UPW, int DIR, bool ALTW>
+__device__ __forceinline__ void pair_body(const double* __restrict__ U, double* __restrict__ H,
+                                          const double* __restrict__ dxinv, const DevGeom& G, const PhysParams& pp,
+                                          const StageEpi& ep, long long ntrans, int L, int XL, long long blk,
+                                          double* sm) {
+  using LY = PairLayout<M, CHAR, UPW, ALTW>;
+  constexpr int NV = LY::NV, ND = LY::ND, NR = LY::NR;
+  constexpr bool CC = LY::CC, NEEDC = LY::NEEDC;
+  const int T = blockDim.x, S = T + 4, t = threadIdx.x;
+  double* su = sm;
+  double* sf = su + NV * S;
+  ff* sd = (ff*)(sf + NV * S);  // rows 0..NV-1: f, NV..2NV-1: u
+  ff* sa = sd + 2 * NV * S;
+  ff* sr = sa + LY::NA * S;
+  const int N = G.dim[DIR], LL = L + 6;
+  const long long sdir = G.stride[DIR];
+  const int lo = G.bclo[DIR], hi = G.bchi[DIR];
+  const unsigned ngrp = (unsigned)((ntrans + XL - 1) / XL), tile = (unsigned)blk / ngrp;
+  const long long l0 = (long long)((unsigned)blk - tile * ngrp) * XL;
+  const int a0 = (int)tile * L;
+  const int nl = (int)(ntrans - l0 < XL ? ntrans - l0 : XL), Lc = N - a0 < L ? N - a0 : L;
+  auto line_base = [&](long long tr) {
+    long long pb = (long long)G.g * sdir;
+#pragma unroll
+    for (int e = 0; e < ND; e++) {
+      if (e == DIR) continue;
+      const int ie = (int)(tr % G.dim[e]);
+      tr /= G.dim[e];
+      pb += (long long)(ie + G.g) * G.stride[e];
+    }
+    return pb;
+  };
+  // Cells a0-3 .. a0+Lc+2 of the lines, consecutive threads on consecutive doubles: along a
+  // line for DIR 0, else across the lines.
+  if (DIR == 0) {
+    for (int l = 0; l < nl; l++) {
+      const long long pb = line_base(l0 + l);
+      for (int i = t; i < (Lc + 6) * NV; i += T) {
+        const int c = i / NV, v = i - c * NV;
+        su[v * S + l * LL + c] = U[(pb + (long long)fold_index(a0 - 3 + c, N, lo, hi) * sdir) * NV + v];
+      }
+    }
+  } else {
+    const int R = nl * NV, c0 = t / R, r = t - c0 * R, l = r / NV, v = r - l * NV, step = T / R;
+    if (c0 < step) {
+      const long long pb = line_base(l0 + l);
+      for (int c = c0; c < Lc + 6; c += step)
+        su[v * S + l * LL + c] = U[(pb + (long long)fold_index(a0 - 3 + c, N, lo, hi) * sdir) * NV + v];
+    }
+  }
+  __syncthreads();
+  const int line = t / LL, q = t - line * LL, w = t;
+  // Every thread computes, also those whose slot holds no cell or no interface (their
+  // values, from whatever the slots hold, are not used): the warps stay converged from
+  // barrier to barrier, and the slots' padding keeps all indexes inside the arrays.
+  PParams P;
+  P.gm1 = to_pair(pp.gm1);
+  P.gamma = to_pair(pp.gamma);
+  P.eps4 = to_pair(4.0 * pp.eps);
+  {
+    double uu[NV], fv[NV];
+#pragma unroll
+    for (int v = 0; v < NV; v++) uu[v] = su[v * S + w];
+    const Prim<M> pr = to_prim<M>(uu, pp);
+    cell_flux<M, DIR>(pr, fv);
+#pragma unroll
+    for (int v = 0; v < NV; v++) sf[v * S + w] = fv[v];
+    if (CC) {
+      const ff r = to_pair(uu[0]);
+      sa[w] = r * rsqrt(r);
+#pragma unroll
+      for (int k = 0; k < ND; k++) sa[(1 + k) * S + w] = to_pair(pr.vel[k]);
+      sa[(1 + ND) * S + w] = to_pair((pr.e + pr.P) * pr.rinv);
+    }
+    if (NEEDC) {
+      const ff c2 = P.gamma * to_pair(pr.P * pr.rinv);
+      ff c = (UPW == UPW_RUS && M == MODEL_EULER1D) ? c2 : c2 * rsqrt(c2);
+      if (UPW == UPW_RUS) c = c + ffabs(to_pair(pr.vel[DIR]));
+      sa[(CC ? ND + 2 : 0) * S + w] = c;
+    }
+  }
+  __syncthreads();
+  {
+#pragma unroll
+    for (int v = 0; v < NV; v++) {
+      sd[v * S + w] = to_pair(sf[v * S + w + 1] - sf[v * S + w]);
+      sd[(NV + v) * S + w] = to_pair(su[v * S + w + 1] - su[v * S + w]);
+    }
+  }
+  __syncthreads();
+  const bool iface = line < nl && q >= 2 && q <= Lc + 2;
+  const bool own = line < nl && q >= 3 && q <= Lc + 2;
+  constexpr bool STATES = (UPW == UPW_ROE && M == MODEL_EULER2D) ||
+                          ((UPW == UPW_LLF || UPW == UPW_RF) && M != MODEL_EULER1D);
+  bool ok = true;
+  ff g12[NV];
+  float mag[NV], lam = 0.0f, rho = 0.0f, Hs = 0.0f;  // 6 x the terms of f per component, and of u
+  float magu[NV];
+  PCell<M> cl, cr;
+  PEig Ecc;
+  auto cell_of = [&](int x) {
+    PCell<M> c;
+    c.t = c.H = c.c = ff{1.0f, 0.0f};
+#pragma unroll
+    for (int k = 0; k < 3; k++) c.vel[k] = ff{0.0f, 0.0f};
+    if (CC) {
+      c.t = sa[x];
+#pragma unroll
+      for (int k = 0; k < ND; k++) c.vel[k] = sa[(1 + k) * S + x];
+      c.H = sa[(1 + ND) * S + x];
+    }
+    if (NEEDC) c.c = sa[(CC ? ND + 2 : 0) * S + x];
+    return c;
+  };
+  if (!CHAR) {
+    ff fs6[NV], fd6[NV], us6[NV], ud6[NV], um[NV];
+#pragma unroll
+    for (int v = 0; v < NV; v++) {
+      ff* rows = sr + (v & 1) * 2 * NR * S;
+      {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const ff* dd = sd + (h * NV + v) * S;
+          const PRow r = weno_row<ALTW>(dd[w - 1], dd[w], P.eps4, pp.wtype == PW_NONE);
+          ff* o = rows + h * NR * S + w;
+          o[0] = r.d;
+          o[S] = r.l;
+          o[2 * S] = r.c;
+          o[3 * S] = r.r;
+          if (ALTW) {
+            o[4 * S] = r.bl;
+            o[5 * S] = r.br;
+          }
+        }
+      }
+      __syncthreads();
+      {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const ff* o = rows + h * NR * S + w;
+          ff bl1, br3, br4, bl2;
+          bl1 = br3 = br4 = bl2 = ff{0.0f, 0.0f};
+          if (ALTW) {
+            bl1 = o[4 * S - 1];
+            bl2 = o[4 * S];
+            br3 = o[5 * S + 1];
+            br4 = o[5 * S + 2];
+          }
+          ok = weno_pair_corr<ALTW>(o[-1], o[0], o[1], o[2], o[S - 1], o[2 * S], o[3 * S + 1], o[3 * S + 2],
+                                    o[2 * S + 1], o[S], bl1, br3, br4, bl2, pp.wtype, h ? us6[v] : fs6[v],
+                                    h ? ud6[v] : fd6[v], h ? magu[v] : mag[v]) & ok;
+          if (h && STATES) um[v] = pmean(to_pair(su[v * S + w]), sd[(NV + v) * S + w], o[0], o[1], us6[v]);
+        }
+      }
+    }
+    {
+      if (CC || NEEDC) {
+        cl = cell_of(w);
+        cr = cell_of(w + 1);
+      }
+      if (CC) Ecc = peig<M, DIR>(cl, cr, P);
+      pupwind<M, UPW, DIR>(fs6, fd6, ud6, um, Ecc, cl, cr, P, g12, lam, rho, Hs);
+      const float s0 = rho * lam, sm1 = s0 * lam, sE = s0 * Hs;
+#pragma unroll
+      for (int v = 0; v < NV; v++) {
+        const float s = v == 0 ? s0 : (v == NV - 1 ? sE : sm1);
+        ok = ok & (ffma(lam, magu[v], mag[v]) <= 0.09375f * s) & (s >= 8.7e-19f) & (s <= 1.2e30f);
+      }
+    }
+  } else {
+    cl = cell_of(w);
+    cr = cell_of(w + 1);
+    Ecc = peig<M, DIR>(cl, cr, P);
+    ff xs[NV], xd[NV], us[NV], ud[NV];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      ff pj[5][NV];
+#pragma unroll
+      for (int k = 0; k < 5; k++) {
+        ff x[NV];
+#pragma unroll
+        for (int v = 0; v < NV; v++) x[v] = sd[(h * NV + v) * S + w - 2 + k];
+        pprojL<M, DIR>(Ecc, P, x, pj[k]);
+      }
+#pragma unroll
+      for (int v = 0; v < NV; v++) {
+        const ff dl[5] = {pj[0][v], pj[1][v], pj[2][v], pj[3][v], pj[4][v]};
+        ok = weno_window_corr<ALTW>(dl, P.eps4, pp.wtype, h ? us[v] : xs[v], h ? ud[v] : xd[v],
+                                    h ? magu[v] : mag[v]) & ok;
+      }
+    }
+    constexpr bool SAME_BASIS = UPW == UPW_RUS || M == MODEL_EULER1D || (M == MODEL_NS3D && UPW == UPW_ROE);
+    if (SAME_BASIS) {
+      rho = cl.t.h * cr.t.h;
+      lam = fadd(fabsf(Ecc.un.h), Ecc.a.h);
+      Hs = Ecc.H.h;
+      ff lm[3] = {Ecc.un - Ecc.a, Ecc.un + Ecc.a, Ecc.un};
+      float sg[3] = {0.0f, 0.0f, 0.0f};
+      if (UPW == UPW_RUS) {
+        const ff avg = (M == MODEL_EULER1D ? sqr(Ecc.a) : Ecc.a) + ffabs(Ecc.un);
+        lm[0] = lm[1] = lm[2] = ffmax(ffmax(cl.c, cr.c), avg);
+        lam = fmaxf(lam, lm[0].h);
+      } else if (UPW == UPW_ROE) {
+#pragma unroll
+        for (int k = 0; k < 3; k++) lm[k] = M == MODEL_EULER1D ? ffabs(lm[k]) : pharten(lm[k]);
+      } else {
+        const ff cv = cl.vel[DIR], rv = cr.vel[DIR];
+        pfield<UPW>(cv - cl.c, lm[0], rv - cr.c, lm[0], sg[0]);
+        pfield<UPW>(cv + cl.c, lm[1], rv + cr.c, lm[1], sg[1]);
+        pfield<UPW>(cv, lm[2], rv, lm[2], sg[2]);
+        lam = fmaxf(lam, fmaxf(lm[0].h, lm[1].h));
+      }
+#pragma unroll
+      for (int k = 0; k < NV; k++) {
+        const int m = k < 2 ? k : 2;
+        FAcc r = acc_mul(neg(lm[m]), ud[k]);
+        acc_add(r, xs[k]);
+        if (UPW == UPW_RF && sg[m] != 0.0f) acc_add(r, mul2(xd[k], -sg[m]));
+        xs[k] = acc_get(r);
+      }
+      pprojR<M, DIR>(Ecc, xs, g12);
+    } else {
+      ff fs6[NV], fd6[NV], us6[NV], ud6[NV], um[NV];
+      pprojR<M, DIR>(Ecc, xs, fs6);
+      pprojR<M, DIR>(Ecc, us, us6);
+      pprojR<M, DIR>(Ecc, ud, ud6);
+      if (UPW == UPW_RF) pprojR<M, DIR>(Ecc, xd, fd6);
+#pragma unroll
+      for (int v = 0; v < NV; v++) {
+        const ff* dd = sd + (NV + v) * S + w;
+        um[v] = pmean(to_pair(su[v * S + w]), dd[0], dd[0] - dd[-1], dd[1] - dd[0], us6[v]);
+      }
+      pupwind<M, UPW, DIR>(fs6, fd6, ud6, um, Ecc, cl, cr, P, g12, lam, rho, Hs);
+    }
+    // the fields' strengths are densities (shear: momenta) times a speed for f
+    const float s0 = rho * lam, sm1 = s0 * lam;
+    const float sE = s0 * Hs;
+    ok = ok & (s0 >= 8.7e-19f) & (s0 <= 1.2e30f) & (sm1 >= 8.7e-19f) & (sm1 <= 1.2e30f) & (sE >= 8.7e-19f) &
+         (sE <= 1.2e30f);
+#pragma unroll
+    for (int k = 0; k < NV; k++) {
+      const float sc = (M == MODEL_EULER1D && k < 2) ? Ecc.rs.h : 1.0f;
+      ok = ok & (ffma(lam, magu[k], mag[k]) * sc <= 0.09375f * (k < 3 ? s0 : sm1));
+    }
+  }
+  __syncthreads();  // the differences are read no more: their place takes G and the cells' sums
+  double* sg = sf + NV * S;
+  double* sh = sg + NV * S;
+  if (iface) {
+    if (ok) {
+#pragma unroll
+      for (int v = 0; v < NV; v++) sg[v * S + w] = to_double(ffc(1.0 / 12.0) * g12[v]);
+    } else {
+      iface_fp64<M, CHAR, UPW, DIR, ALTW>(su, sf, S, w, pp, sg + w);
+    }
+    const int I = a0 - 2 + q;  // the interface right of the own cell
+    if (ep.bnd && (I == 0 || I == N)) {
+      double Fb[NV];
+#pragma unroll
+      for (int v = 0; v < NV; v++) {
+        const double* f = sf + v * S + w;
+        Fb[v] = fma(7.0, f[0] + f[1], -(f[-1] + f[2])) * (1.0 / 12.0) + sg[v * S + w];
+      }
+      boundary_flux<NV>(ep, I, N, l0 + line, ntrans, Fb);
+    }
+  }
+  __syncthreads();
+  if (own) {
+    const double dxi = dxinv[G.g + a0 - 3 + q];
+#pragma unroll
+    for (int v = 0; v < NV; v++) {
+      const double* f = sf + v * S + w;
+      const double c4 = fma(2.0 / 3.0, f[1] - f[-1], (f[2] - f[-2]) * (-1.0 / 12.0));
+      sh[v * S + w] = dxi * (c4 + (sg[v * S + w] - sg[v * S + w - 1]));
+    }
+  }
+  __syncthreads();
+  // Stage epilogue, value by value in the order of memory.
+  if (DIR == 0) {
+    for (int l = 0; l < nl; l++) {
+      const long long ob = (line_base(l0 + l) + (long long)a0 * sdir) * NV;
+      for (int i = t; i < Lc * NV; i += T) {
+        const int c = i / NV, v = i - c * NV;
+        stage_epilogue<1>(ep, H, ob + i, &sh[v * S + l * LL + c + 3]);
+      }
+    }
+  } else {
+    const int R = nl * NV, c0 = t / R, r = t - c0 * R, l = r / NV, v = r - l * NV, step = T / R;
+    if (c0 < step) {
+      const long long ob = (line_base(l0 + l) + (long long)a0 * sdir) * NV + v;
+      for (int c = c0; c < Lc; c += step) stage_epilogue<1>(ep, H, ob + (long long)c * sdir * NV, &sh[v * S + l * LL + c + 3]);
+    }
+  }
+}
+
+template <int M, bool CHAR, int UPW, int DIR, bool ALTW>
+__global__ void __launch_bounds__(256, 2)
+hyp_pair_kernel(const double* __restrict__ U, double* __restrict__ H, const double* __restrict__ dxinv, DevGeom G,
+                PhysParams pp, StageEpi ep, long long ntrans, int L, int XL) {
+  extern __shared__ double pair_smem[];
+  pair_body<M, CHAR, UPW, DIR, ALTW>(U, H, dxinv, G, pp, ep, ntrans, L, XL, blockIdx.x, pair_smem);
+}
+
+template <int M, bool CHAR, int UPW, int DIR, bool ALTW>
+cudaError_t launch_pair(const double* U, double* H, const double* dxinv_dir, const DevGeom& G, const PhysParams& pp,
+                        const StageEpi& ep, long long ntrans, int cap, cudaStream_t s) {
+  const int N = G.dim[DIR];
+  const PairPlan p = pair_plan(N, ntrans, DIR, cap > 0 ? cap : pair_cap(ntrans * N));
+  const long long nblk = (ntrans + p.XL - 1) / p.XL * ((N + p.L - 1) / p.L);
+  if (nblk > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+  auto k = hyp_pair_kernel<M, CHAR, UPW, DIR, ALTW>;
+  const size_t sm = PairLayout<M, CHAR, UPW, ALTW>::bytes(p.T);
+  if (sm > 48 * 1024)
+    if (cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) return e;
+  k<<<(unsigned)nblk, p.T, sm, s>>>(U, H, dxinv_dir, G, pp, ep, ntrans, p.L, p.XL);
+  return cudaGetLastError();
+}
+
+// Ensemble: the blocks of all members in one launch.
+template <int M, bool CHAR, int UPW, int DIR>
+__global__ void __launch_bounds__(256, 2)
+hyp_batched_pair_kernel(const MemberDev* __restrict__ mem, int nmem, const double* __restrict__ U,
+                        double* __restrict__ H, const double* __restrict__ dxinv, PhysParams pp, StageEpi ep) {
+  extern __shared__ double pair_smem[];
+  StageEpi e = ep;
+  const long long b = blockIdx.x;
+  const MemberDev& m = batched_member<DIR>(mem, nmem, b, e);
+  const long long o = m.off;
+  pair_body<M, CHAR, UPW, DIR, false>(U + o, H ? H + o : nullptr, dxinv + m.dx_off[DIR], m.G, pp, e, m.ntrans[DIR],
+                                      m.L[DIR], m.XL[DIR], b - m.start[DIR], pair_smem);
+}
+
+template <int M, bool CHAR, int UPW, int DIR>
+cudaError_t launch_batched_dir(const MemberDev* mem, int nmem, long long nblk, int T, const double* U, double* H,
+                               const double* dxinv, const PhysParams& pp, const StageEpi& ep, cudaStream_t s) {
+  if (nblk <= 0) return cudaSuccess;
+  if (nblk > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+  auto k = hyp_batched_pair_kernel<M, CHAR, UPW, DIR>;
+  const size_t sm = PairLayout<M, CHAR, UPW, false>::bytes(T);
+  if (sm > 48 * 1024)
+    if (cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) return e;
+  k<<<(unsigned)nblk, T, sm, s>>>(mem, nmem, U, H, dxinv, pp, ep);
+  return cudaGetLastError();
+}
+
+}  // namespace gbh

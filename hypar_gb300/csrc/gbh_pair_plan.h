@@ -1,0 +1,45 @@
+// gbh_pair_plan.h -- block shapes of the float-pair kernels (gbh_pair_flux.cuh).
+#pragma once
+
+namespace gbh {
+
+// The block shape of one direction: XL lines of L cells each, T threads (T >= XL (L + 6)).
+struct PairPlan {
+  int L, XL, T;
+};
+
+// The shape that covers nlines lines of N cells with the fewest threads, at most `cap` per
+// block.  Slots are lost to the six halo cells of each piece of a line, to the last piece
+// of a line and to the last block of lines; along the strided directions fewer than four
+// neighbouring lines read less than a 128-byte line of memory at a time, which is weighed
+// as an eighth more.
+inline PairPlan pair_plan(int N, long long nlines, int dir, int cap) {
+  PairPlan best = {1, 1, 32};
+  double cost = 1e300;
+  for (int XL = 1; XL <= 16 && XL <= nlines; XL++) {
+    const int Lmax = cap / XL - 6;
+    if (Lmax < 1) break;
+    const int n0 = (N + Lmax - 1) / Lmax;
+    for (int n = n0; n < n0 + 3; n++) {
+      const int L = (N + n - 1) / n, nt = (N + L - 1) / L;
+      const int T = (XL * (L + 6) + 31) / 32 * 32;
+      double c = (double)((nlines + XL - 1) / XL) * nt * T;
+      if (dir > 0 && XL < 4) c *= 1.125;
+      if (c < cost) {
+        cost = c;
+        best = {L, XL, T};
+      }
+    }
+  }
+  return best;
+}
+
+// Threads per block: large blocks lose fewer slots, small ones spread a small grid over
+// the 152 SMs.
+inline int pair_cap(long long cells) { return cells >= 150000 ? 256 : (cells >= 30000 ? 128 : 64); }
+
+// Threads per block asked for by a launch shape: a tile of t interfaces (seg = -t) or a
+// block below 128 threads is taken as the cap, anything else leaves it to pair_cap (0).
+inline int pair_cap_of(int seg, int block) { return seg <= -32 ? -seg : (block > 0 && block < 128 ? block : 0); }
+
+}  // namespace gbh
