@@ -869,7 +869,7 @@ extern "C" int gb_solver_autotune(gb_solver* s, int reps) {
     for (int e = 0; e < c.ndims; e++)
       if (e != d) ntrans *= c.dim[e];
     std::vector<int> segs;
-    const bool pairs = !s->gravity && c.hyp_scheme == GB_SCHEME_WENO5 && c.upwind != UPW_SWFS;
+    const bool pairs = c.hyp_scheme == GB_SCHEME_WENO5 && c.upwind != UPW_SWFS;
     for (int w = 1; w <= 4 && !pairs; w++) {
       double lanes = (double)w * sms * 4 * 32;
       long long nseg = (long long)(lanes / (double)ntrans + 0.5);

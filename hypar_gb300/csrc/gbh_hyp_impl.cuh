@@ -41,6 +41,17 @@ __device__ __forceinline__ double sound_speed(const Prim<M>& q, const PhysParams
   return nr_sqrt(pp.gamma * q.P * q.rinv);
 }
 
+// Energy component of the well-balanced modified solution: Euler1D u / S (f holds 1/S,
+// Euler1DModifiedSolution.c:48); NavierStokes3D P/(gamma-1)/g + f rho|v|^2/2
+// (NavierStokes3DModifiedSolution.c:52-66).
+template <int M>
+__device__ __forceinline__ double modified_energy(const Prim<M>& q, double e, double f, double g,
+                                                  const PhysParams& pp) {
+  if (M == MODEL_EULER1D) return e * f;
+  const double vsq = q.vel[0] * q.vel[0] + q.vel[1] * q.vel[1] + q.vel[2] * q.vel[2];
+  return fma(q.P * pp.inv_gm1, nr_rcp(g), (0.5 * q.rho * vsq) * f);
+}
+
 template <int M>
 struct CellAux {
   RoeSide rs;
@@ -1075,7 +1086,7 @@ cudaError_t launch_batched_model(int dir, int chr, int upw, const MemberDev* mem
 }
 
 // The float-pair form (gbh_pair_flux.cuh), which the direction launcher prefers.
-template <int M, bool CHAR, int UPW, int DIR, bool ALTW>
+template <int M, bool CHAR, int UPW, int DIR, bool ALTW, bool GRAV>
 cudaError_t launch_pair(const double* U, double* H, const double* dxinv_dir, const DevGeom& G, const PhysParams& pp,
                         const StageEpi& ep, long long ntrans, int cap, cudaStream_t s);
 
@@ -1097,12 +1108,12 @@ cudaError_t launch_dir(const double* U, double* H, const double* dxinv_dir, cons
       return cudaGetLastError();
     }
   }
-  // Gravity, Steger-Warming and the adjoint's tapes: the FP64 kernels.
-  constexpr bool PAIR = !GRAV && !WT && UPW != UPW_SWFS;
-  constexpr bool TAPE = M == MODEL_EULER2D && !CHAR && UPW == UPW_ROE && !ALTW;
+  // Steger-Warming and the adjoint's tapes: the FP64 kernels.
+  constexpr bool PAIR = !WT && UPW != UPW_SWFS;
+  constexpr bool TAPE = M == MODEL_EULER2D && !CHAR && UPW == UPW_ROE && !ALTW && !GRAV;
   if constexpr (PAIR) {
     if (!TAPE || !ep.tape)
-      return launch_pair<M, CHAR, UPW, DIR, ALTW>(U, H, dxinv_dir, G, pp, ep, ntrans, pair_cap_of(L.seg, L.block), s);
+      return launch_pair<M, CHAR, UPW, DIR, ALTW, GRAV>(U, H, dxinv_dir, G, pp, ep, ntrans, pair_cap_of(L.seg, L.block), s);
   }
   if constexpr (!PAIR || TAPE) {
   if (L.seg < 0 && !GRAV) {

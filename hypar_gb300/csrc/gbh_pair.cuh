@@ -295,14 +295,16 @@ GBH_HD bool side_weights(ff i1, ff i2, ff i3, ff tau, int wtype, ff& w1, ff& w3)
   return (S.h >= 7.888609e-31f) & (S.h <= 1.0e36f);  // 2^-100; false for NaN
 }
 
-// Six times (mean of the two sides - central value) * 2 = `sum6` and six times the right
-// value minus the left one = `dif6`, from the second differences d1..d4 of window cells
-// 1..4 and the sub-stencils' terms.  mag6: the sum of the terms' magnitudes, which bounds
-// the rounding of both (some 2^-47 of it), cancellation or not.
+// The weights of a pair: the farthest upwind sub-stencils' doubled, the downwind ones'.
+struct PWeights {
+  ff l1, l3, r1, r3;  // 2 w1 and w3 of the left-biased side, of the right-biased side
+};
+
+// From the third differences t1, t2, t3 of the values the weights are formed from
+// (Yamaleev-Carpenter's tau) and the sub-stencils' terms.
 template <bool ALTW>
-GBH_HD bool weno_pair_corr(ff d1, ff d2, ff d3, ff d4, ff l1, ff c2, ff r3, ff r4, ff c3, ff l2, ff bl1, ff br3,
-                           ff br4, ff bl2, int wtype, ff& sum6, ff& dif6, float& mag6) {
-  const ff t1 = d2 - d1, t2 = d3 - d2, t3 = d4 - d3;
+GBH_HD bool weno_pair_weights(ff t1, ff t2, ff t3, ff l1, ff c2, ff r3, ff r4, ff c3, ff l2, ff bl1, ff br3, ff br4,
+                              ff bl2, int wtype, PWeights& W) {
   ff tauL = {0.0f, 0.0f}, tauR = {0.0f, 0.0f};
   if (ALTW && wtype == PW_BORGES) {
     tauL = bl1 - br3;
@@ -311,26 +313,50 @@ GBH_HD bool weno_pair_corr(ff d1, ff d2, ff d3, ff d4, ff l1, ff c2, ff r3, ff r
     tauL = mul2(sqr(t2 - t1), 4.0f);
     tauR = mul2(sqr(t3 - t2), 4.0f);
   }
-  ff w1L, w3L, w1R, w3R;
-  bool ok = side_weights<ALTW>(l1, c2, mulf(r3, 3.0f), tauL, wtype, w1L, w3L);
-  ok = side_weights<ALTW>(r4, c3, mulf(l2, 3.0f), tauR, wtype, w1R, w3R) & ok;
-  w1L = mul2(w1L, 2.0f);
-  w1R = mul2(w1R, 2.0f);
-  FAcc s = acc_mul(w1R, t3), d = s;
-  acc_fma(s, w1L, neg(t1));
-  acc_fma(s, w3R - w3L, t2);
-  acc_fma(d, w1L, t1);
-  acc_fma(d, (w3R + w3L) - ff{1.0f, 0.0f}, t2);
-  sum6 = acc_get(s);
-  dif6 = acc_get(d);
-  mag6 = ffma(fabsf(w1R.h), fabsf(t3.h), ffma(fabsf(w1L.h), fabsf(t1.h), fmul(fadd(w3R.h, w3L.h), fabsf(t2.h))));
+  bool ok = side_weights<ALTW>(l1, c2, mulf(r3, 3.0f), tauL, wtype, W.l1, W.l3);
+  ok = side_weights<ALTW>(r4, c3, mulf(l2, 3.0f), tauR, wtype, W.r1, W.r3) & ok;
+  W.l1 = mul2(W.l1, 2.0f);
+  W.r1 = mul2(W.r1, 2.0f);
+  return ok;
+}
+// Twice the mean of the two sides less the central value, and the right value less the
+// left one, times 6, of values with the third differences t1, t2, t3.
+GBH_HD ff weno_sum6(const PWeights& W, ff t1, ff t2, ff t3) {
+  FAcc s = acc_mul(W.r1, t3);
+  acc_fma(s, W.l1, neg(t1));
+  acc_fma(s, W.r3 - W.l3, t2);
+  return acc_get(s);
+}
+GBH_HD ff weno_dif6(const PWeights& W, ff t1, ff t2, ff t3) {
+  FAcc d = acc_mul(W.r1, t3);
+  acc_fma(d, W.l1, t1);
+  acc_fma(d, (W.r3 + W.l3) - ff{1.0f, 0.0f}, t2);
+  return acc_get(d);
+}
+// The sum of the terms' magnitudes, which bounds the rounding of both (some 2^-47 of it),
+// cancellation or not.
+GBH_HD float weno_mag6(const PWeights& W, ff t1, ff t2, ff t3) {
+  return ffma(fabsf(W.r1.h), fabsf(t3.h), ffma(fabsf(W.l1.h), fabsf(t1.h), fmul(fadd(W.r3.h, W.l3.h), fabsf(t2.h))));
+}
+
+// All three from the second differences d1..d4 of window cells 1..4 where weights and
+// values come from the same array.
+template <bool ALTW>
+GBH_HD bool weno_pair_corr(ff d1, ff d2, ff d3, ff d4, ff l1, ff c2, ff r3, ff r4, ff c3, ff l2, ff bl1, ff br3,
+                           ff br4, ff bl2, int wtype, ff& sum6, ff& dif6, float& mag6) {
+  const ff t1 = d2 - d1, t2 = d3 - d2, t3 = d4 - d3;
+  PWeights W;
+  const bool ok = weno_pair_weights<ALTW>(t1, t2, t3, l1, c2, r3, r4, c3, l2, bl1, br3, br4, bl2, wtype, W);
+  sum6 = weno_sum6(W, t1, t2, t3);
+  dif6 = weno_dif6(W, t1, t2, t3);
+  mag6 = weno_mag6(W, t1, t2, t3);
   return ok;
 }
 
-// The same from the five differences of a window whose sub-stencils no other interface
-// shares (characteristic fields).
+// The weights from the five differences of a window whose sub-stencils no other interface
+// shares (characteristic fields), with its third differences.
 template <bool ALTW>
-GBH_HD bool weno_window_corr(const ff* dl, ff eps4, int wtype, ff& sum6, ff& dif6, float& mag6) {
+GBH_HD bool weno_window_weights(const ff* dl, ff eps4, int wtype, PWeights& W, ff& t1, ff& t2, ff& t3) {
   ff d[4], l1, c2, l2, c3, r3, r4, bl1, bl2, br3, br4;
 #pragma unroll
   for (int k = 0; k < 4; k++) d[k] = dl[k + 1] - dl[k];
@@ -355,8 +381,27 @@ GBH_HD bool weno_window_corr(const ff* dl, ff eps4, int wtype, ff& sum6, ff& dif
       }
     }
   }
-  return weno_pair_corr<ALTW>(d[0], d[1], d[2], d[3], l1, c2, r3, r4, c3, l2, bl1, br3, br4, bl2, wtype, sum6, dif6,
-                              mag6);
+  t1 = d[1] - d[0];
+  t2 = d[2] - d[1];
+  t3 = d[3] - d[2];
+  return weno_pair_weights<ALTW>(t1, t2, t3, l1, c2, r3, r4, c3, l2, bl1, br3, br4, bl2, wtype, W);
+}
+template <bool ALTW>
+GBH_HD bool weno_window_corr(const ff* dl, ff eps4, int wtype, ff& sum6, ff& dif6, float& mag6) {
+  PWeights W;
+  ff t1, t2, t3;
+  const bool ok = weno_window_weights<ALTW>(dl, eps4, wtype, W, t1, t2, t3);
+  sum6 = weno_sum6(W, t1, t2, t3);
+  dif6 = weno_dif6(W, t1, t2, t3);
+  mag6 = weno_mag6(W, t1, t2, t3);
+  return ok;
+}
+// Third differences of a window from its five differences.
+GBH_HD void third_differences(const ff* dl, ff& t1, ff& t2, ff& t3) {
+  const ff d1 = dl[1] - dl[0], d2 = dl[2] - dl[1], d3 = dl[3] - dl[2], d4 = dl[4] - dl[3];
+  t1 = d2 - d1;
+  t2 = d3 - d2;
+  t3 = d4 - d3;
 }
 
 }  // namespace gbh

@@ -204,11 +204,12 @@ __device__ __forceinline__ void pfield(ff l, ff c, ff r, ff& al, float& sg) {
 // G of one interface times 12 from the conserved sums and differences of the
 // reconstructions (fs6 = 6 (fL + fR - 2 central), fd6 = 6 (fR - fL), ud6 = 6 (uR - uL)),
 // mean states um where the scheme averages the reconstructed states, and the cells'
-// ingredients.  lam, rho, H: the interface's scales.
+// ingredients.  lam, rho, H: the interface's scales.  kappa: gravity's factor of the
+// dissipation.
 template <int M, int UPW, int DIR>
 __device__ __forceinline__ void pupwind(const ff* fs6, const ff* fd6, const ff* ud6, const ff* um, const PEig& Ecc,
                                         const PCell<M>& cl, const PCell<M>& cr, const PParams& q, ff* g12, float& lam,
-                                        float& rho, float& Hs) {
+                                        float& rho, float& Hs, const ff* kappa = nullptr) {
   constexpr int NV = ModelTraits<M>::NV, ND = ModelTraits<M>::ND;
   constexpr bool STATES = (UPW == UPW_ROE && M == MODEL_EULER2D) ||
                           ((UPW == UPW_LLF || UPW == UPW_RF) && M != MODEL_EULER1D);
@@ -237,7 +238,8 @@ __device__ __forceinline__ void pupwind(const ff* fs6, const ff* fd6, const ff* 
   Hs = E.H.h;
   if (UPW == UPW_RUS) {
     const ff avg = (M == MODEL_EULER1D ? sqr(E.a) : E.a) + ffabs(E.un);
-    const ff al = ffmax(ffmax(cl.c, cr.c), avg);
+    ff al = ffmax(ffmax(cl.c, cr.c), avg);
+    if (kappa) al = al * *kappa;
     lam = fmaxf(lam, al.h);
 #pragma unroll
     for (int v = 0; v < NV; v++) g12[v] = fs6[v] - al * ud6[v];
@@ -256,6 +258,12 @@ __device__ __forceinline__ void pupwind(const ff* fs6, const ff* fd6, const ff* 
       c1 = pharten(c1);
       c2 = pharten(c2);
     }
+    if (kappa) {  // Euler1D with gravity
+      c0 = c0 * *kappa;
+      c1 = c1 * *kappa;
+      c2 = c2 * *kappa;
+      lam = fmul(lam, kappa->h);
+    }
     pdissip<M, DIR>(E, q, ud6, c0, c1, c2, y);
 #pragma unroll
     for (int v = 0; v < NV; v++) g12[v] = fs6[v] - y[v];
@@ -266,6 +274,10 @@ __device__ __forceinline__ void pupwind(const ff* fs6, const ff* fd6, const ff* 
   pfield<UPW>(sL.vel[DIR] - sL.c, E.un - E.a, sR.vel[DIR] - sR.c, al[0], sg[0]);
   pfield<UPW>(sL.vel[DIR] + sL.c, E.un + E.a, sR.vel[DIR] + sR.c, al[1], sg[1]);
   pfield<UPW>(sL.vel[DIR], E.un, sR.vel[DIR], al[2], sg[2]);
+  if (kappa) {
+#pragma unroll
+    for (int k = 0; k < 3; k++) al[k] = al[k] * *kappa;
+  }
   lam = fmaxf(lam, fmaxf(al[0].h, al[1].h));
   pdissip<M, DIR>(E, q, ud6, al[0], al[1], al[2], y);
 #pragma unroll
@@ -280,10 +292,11 @@ __device__ __forceinline__ void pupwind(const ff* fs6, const ff* fd6, const ff* 
 }
 
 // The FP64 evaluation of one interface (window in shared memory, own cell = slot w) as
-// the correction G, written to G[v S].
-template <int M, bool CHAR, int UPW, int DIR, bool ALTW>
-__device__ __forceinline__ void iface_fp64(const double* su, const double* sf, int S, int w, const PhysParams& pp,
-                                           double* G) {
+// the correction G, written to G[v S]; with gravity (sgf, sgg: the hydrostatic fields)
+// also the source function's interface values as corrections of its central value, to Gs.
+template <int M, bool CHAR, int UPW, int DIR, bool ALTW, bool GRAV>
+__device__ __forceinline__ void iface_fp64(const double* su, const double* sf, const double* sgf, const double* sgg,
+                                           int S, int w, const PhysParams& pp, bool src_dir, double* G, double* Gs) {
   constexpr int NV = ModelTraits<M>::NV;
   double wu[6][NV], wf[6][NV], wuc[6], wgf[6], wgg[6], fI[NV], SI[NV];
   CellAux<M> ax[6];
@@ -295,7 +308,13 @@ __device__ __forceinline__ void iface_fp64(const double* su, const double* sf, i
       wf[p][v] = sf[v * S + w - 2 + p];
     }
     const Prim<M> q = to_prim<M>(wu[p], pp);
-    wuc[p] = ufunc_energy<M>(q, pp, wu[p][NV - 1]);
+    if (GRAV) {
+      wgf[p] = sgf[w - 2 + p];
+      wgg[p] = sgg[w - 2 + p];
+      wuc[p] = modified_energy<M>(q, wu[p][NV - 1], wgf[p], wgg[p], pp);
+    } else {
+      wuc[p] = ufunc_energy<M>(q, pp, wu[p][NV - 1]);
+    }
     if (p == 2 || p == 3) {
       ax[p].rs = roe_side<M>(q);
       if (UPW == UPW_RUS) ax[p].c = rusanov_speed<M, DIR>(q, pp);
@@ -304,18 +323,25 @@ __device__ __forceinline__ void iface_fp64(const double* su, const double* sf, i
   }
   StageEpi ep;
   ep.tape = nullptr;
-  iface_flux<M, CHAR, UPW, DIR, ALTW, false, false>(wu, wf, wuc, wgf, wgg, ax, pp, ep, 4.0 * pp.eps, false, 0, fI, SI);
+  iface_flux<M, CHAR, UPW, DIR, ALTW, GRAV, false>(wu, wf, wuc, wgf, wgg, ax, pp, ep, 4.0 * pp.eps, src_dir, 0, fI, SI);
 #pragma unroll
   for (int v = 0; v < NV; v++) {
     const double d1 = wf[2][v] - wf[1][v], d2 = wf[3][v] - wf[2][v], d3 = wf[4][v] - wf[3][v];
-    G[v * S] = fI[v] - fma(6.0, d2, d1 - d3) * (1.0 / 12.0);
+    // without gravity fI is relative to the left cell's flux
+    G[v * S] = (GRAV ? fI[v] - wf[2][v] : fI[v]) - fma(6.0, d2, d1 - d3) * (1.0 / 12.0);
+  }
+  if (GRAV && src_dir) {
+    const double d1 = wgg[2] - wgg[1], d2 = wgg[3] - wgg[2], d3 = wgg[4] - wgg[3];
+    const double c = fma(6.0, d2, d1 - d3) * (1.0 / 12.0);
+    Gs[0] = (SI[1 + DIR] - wgg[2]) - c;
+    Gs[S] = (SI[NV - 1] - wgg[2]) - c;
   }
 }
 
 // Shared memory of a block of T threads (slots S = T + 4): u and f (doubles), their right
 // differences (pairs), the cells' ingredients, and for the component-wise form one
-// component's sub-stencil rows, double-buffered.
-template <int M, bool CHAR, int UPW, bool ALTW>
+// component's sub-stencil rows, double-buffered; with gravity the hydrostatic fields.
+template <int M, bool CHAR, int UPW, bool ALTW, bool GRAV>
 struct PairLayout {
   static constexpr int NV = ModelTraits<M>::NV, ND = ModelTraits<M>::ND;
   static constexpr bool CC = NeedCC<M, CHAR, UPW>::value;
@@ -323,7 +349,9 @@ struct PairLayout {
   static constexpr int NA = (CC ? ND + 2 : 0) + (NEEDC ? 1 : 0);
   static constexpr int NR = ALTW ? 6 : 4;                // pairs of a row
   static constexpr int NROW = CHAR ? 0 : 2 * 2 * NR;     // two buffers of the f and u rows
-  static constexpr int WORDS = 2 * NV + 2 * NV + NA + NROW;  // 8-byte words per slot
+  // differences: f, u; with gravity also of the modified solution and of g
+  static constexpr int ND_ROWS = 2 * NV + (GRAV ? NV + 1 : 0);
+  static constexpr int WORDS = 2 * NV + ND_ROWS + NA + NROW + (GRAV ? 2 : 0);  // 8-byte words per slot
   static size_t bytes(int T) { return (size_t)WORDS * (T + 4) * 8; }
 };
 
@@ -331,20 +359,23 @@ struct PairLayout {
 // one thread per slot.  A thread owns a cell and the interface to its right.  sm is not
 // __restrict__: the barriers order other threads' accesses to it, and a pointer that is
 // said to have no alias lets the compiler move its loads and stores across them.
-template <int M, bool CHAR, int UPW, int DIR, bool ALTW>
+template <int M, bool CHAR, int UPW, int DIR, bool ALTW, bool GRAV = false>
 __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* __restrict__ H,
                                           const double* __restrict__ dxinv, const DevGeom& G, const PhysParams& pp,
                                           const StageEpi& ep, long long ntrans, int L, int XL, long long blk,
                                           double* sm) {
-  using LY = PairLayout<M, CHAR, UPW, ALTW>;
+  using LY = PairLayout<M, CHAR, UPW, ALTW, GRAV>;
   constexpr int NV = LY::NV, ND = LY::ND, NR = LY::NR;
   constexpr bool CC = LY::CC, NEEDC = LY::NEEDC;
   const int T = blockDim.x, S = T + 4, t = threadIdx.x;
   double* su = sm;
   double* sf = su + NV * S;
-  ff* sd = (ff*)(sf + NV * S);  // rows 0..NV-1: f, NV..2NV-1: u
-  ff* sa = sd + 2 * NV * S;
+  ff* sd = (ff*)(sf + NV * S);  // rows 0..NV-1: f, NV..2NV-1: u, then the modified solution and g
+  ff* sa = sd + LY::ND_ROWS * S;
   ff* sr = sa + LY::NA * S;
+  double* sgf = (double*)(sr + LY::NROW * S);
+  double* sgg = sgf + S;
+  const bool src_dir = GRAV && pp.grav[DIR] != 0.0 && (ep.mode != EPI_HYP || ep.with_source);
   const int N = G.dim[DIR], LL = L + 6;
   const long long sdir = G.stride[DIR];
   const int lo = G.bclo[DIR], hi = G.bchi[DIR];
@@ -383,6 +414,7 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
   }
   __syncthreads();
   const int line = t / LL, q = t - line * LL, w = t;
+  double term[2] = {0.0, 0.0};  // gravity's source per unit difference of g: momentum, energy
   // Every thread computes, also those whose slot holds no cell or no interface (their
   // values, from whatever the slots hold, are not used): the warps stay converged from
   // barrier to barrier, and the slots' padding keeps all indexes inside the arrays.
@@ -398,6 +430,26 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
     cell_flux<M, DIR>(pr, fv);
 #pragma unroll
     for (int v = 0; v < NV; v++) sf[v * S + w] = fv[v];
+    if (GRAV) {
+      const int i = a0 - 3 + q;
+      double f = 1.0, g = 1.0;
+      if (line < nl && i <= N + 2) {
+        const long long pt = line_base(l0 + line) + (long long)fold_index(i, N, lo, hi) * sdir;
+        f = pp.gf[pt];
+        g = pp.gg[pt];
+      }
+      sgf[w] = f;
+      sgg[w] = g;
+      // the modified solution, in the place its differences take
+      double* sc = (double*)(sd + 2 * NV * S);
+#pragma unroll
+      for (int v = 0; v < NV - 1; v++) sc[v * S + w] = uu[v] * f;
+      sc[(NV - 1) * S + w] = modified_energy<M>(pr, uu[NV - 1], f, g, pp);
+      // [0, rho RT e_DIR, rho RT v_DIR] f (NavierStokes3DSource.c:92-97)
+      const double rRT = pr.rho * pp.RT;
+      term[0] = rRT * f;
+      term[1] = (rRT * (pr.rho == 0.0 ? 0.0 : uu[1 + DIR] * pr.rinv)) * f;
+    }
     if (CC) {
       const ff r = to_pair(uu[0]);
       sa[w] = r * rsqrt(r);
@@ -413,6 +465,16 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
     }
   }
   __syncthreads();
+  if (GRAV) {
+    const double* sc = (const double*)(sd + 2 * NV * S);
+    ff dc[NV];
+#pragma unroll
+    for (int v = 0; v < NV; v++) dc[v] = to_pair(sc[v * S + w + 1] - sc[v * S + w]);
+    __syncthreads();
+#pragma unroll
+    for (int v = 0; v < NV; v++) sd[(2 * NV + v) * S + w] = dc[v];
+    sd[3 * NV * S + w] = to_pair(sgg[w + 1] - sgg[w]);
+  }
   {
 #pragma unroll
     for (int v = 0; v < NV; v++) {
@@ -445,6 +507,14 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
     if (NEEDC) c.c = sa[(CC ? ND + 2 : 0) * S + x];
     return c;
   };
+  ff gs6[NV], tg1, tg2, tg3, kap;  // gravity: the source function's corrections, the dissipation's factor
+  float magg[NV];
+  if (GRAV) {
+    const ff* dd = sd + 3 * NV * S + w;
+    const ff dl[5] = {dd[-2], dd[-1], dd[0], dd[1], dd[2]};
+    third_differences(dl, tg1, tg2, tg3);
+    kap = to_pair(fmax(sgg[w], sgg[w + 1]));
+  }
   if (!CHAR) {
     ff fs6[NV], fd6[NV], us6[NV], ud6[NV], um[NV];
 #pragma unroll
@@ -479,6 +549,27 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
             br3 = o[5 * S + 1];
             br4 = o[5 * S + 2];
           }
+          if (GRAV) {
+            ff t1 = o[0] - o[-1], t2 = o[1] - o[0], t3 = o[2] - o[1];
+            PWeights W;
+            ok = weno_pair_weights<ALTW>(t1, t2, t3, o[S - 1], o[2 * S], o[3 * S + 1], o[3 * S + 2], o[2 * S + 1],
+                                         o[S], bl1, br3, br4, bl2, pp.wtype, W) & ok;
+            if (h) {  // weights of u, values of the modified solution
+              const ff* dd = sd + (2 * NV + v) * S + w;
+              const ff dl[5] = {dd[-2], dd[-1], dd[0], dd[1], dd[2]};
+              third_differences(dl, t1, t2, t3);
+              ud6[v] = weno_dif6(W, t1, t2, t3);
+              magu[v] = weno_mag6(W, t1, t2, t3);
+            } else {
+              fs6[v] = weno_sum6(W, t1, t2, t3);
+              mag[v] = weno_mag6(W, t1, t2, t3);
+              if (v == 1 + DIR || v == NV - 1) {
+                gs6[v] = weno_sum6(W, tg1, tg2, tg3);
+                magg[v] = weno_mag6(W, tg1, tg2, tg3);
+              }
+            }
+            continue;
+          }
           ok = weno_pair_corr<ALTW>(o[-1], o[0], o[1], o[2], o[S - 1], o[2 * S], o[3 * S + 1], o[3 * S + 2],
                                     o[2 * S + 1], o[S], bl1, br3, br4, bl2, pp.wtype, h ? us6[v] : fs6[v],
                                     h ? ud6[v] : fd6[v], h ? magu[v] : mag[v]) & ok;
@@ -492,12 +583,16 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
         cr = cell_of(w + 1);
       }
       if (CC) Ecc = peig<M, DIR>(cl, cr, P);
-      pupwind<M, UPW, DIR>(fs6, fd6, ud6, um, Ecc, cl, cr, P, g12, lam, rho, Hs);
+      pupwind<M, UPW, DIR>(fs6, fd6, ud6, um, Ecc, cl, cr, P, g12, lam, rho, Hs, GRAV ? &kap : nullptr);
       const float s0 = rho * lam, sm1 = s0 * lam, sE = s0 * Hs;
 #pragma unroll
       for (int v = 0; v < NV; v++) {
         const float s = v == 0 ? s0 : (v == NV - 1 ? sE : sm1);
         ok = ok & (ffma(lam, magu[v], mag[v]) <= 0.09375f * s) & (s >= 8.7e-19f) & (s <= 1.2e30f);
+      }
+      if (GRAV && src_dir) {
+        const float rt = (float)term[0];
+        ok = ok & (magg[1 + DIR] * rt <= 0.09375f * sm1) & (magg[NV - 1] * rt * lam <= 0.09375f * sE);
       }
     }
   } else {
@@ -505,9 +600,25 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
     cr = cell_of(w + 1);
     Ecc = peig<M, DIR>(cl, cr, P);
     ff xs[NV], xd[NV], us[NV], ud[NV];
+    ff lcol[NV], sch[NV];  // L (e_{1+DIR} + e_E): the source function's projection per unit of g
+    if (GRAV) {
+      ff ev[NV];
+#pragma unroll
+      for (int v = 0; v < NV; v++) ev[v] = ff{(v == 1 + DIR || v == NV - 1) ? 1.0f : 0.0f, 0.0f};
+      pprojL<M, DIR>(Ecc, P, ev, lcol);
+    }
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-      ff pj[5][NV];
+      ff pj[5][NV], pc[GRAV ? 5 : 1][NV];
+      if (GRAV && h) {
+#pragma unroll
+        for (int k = 0; k < 5; k++) {
+          ff x[NV];
+#pragma unroll
+          for (int v = 0; v < NV; v++) x[v] = sd[(2 * NV + v) * S + w - 2 + k];
+          pprojL<M, DIR>(Ecc, P, x, pc[GRAV ? k : 0]);
+        }
+      }
 #pragma unroll
       for (int k = 0; k < 5; k++) {
         ff x[NV];
@@ -518,6 +629,24 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
 #pragma unroll
       for (int v = 0; v < NV; v++) {
         const ff dl[5] = {pj[0][v], pj[1][v], pj[2][v], pj[3][v], pj[4][v]};
+        if (GRAV) {
+          PWeights W;
+          ff t1, t2, t3;
+          ok = weno_window_weights<ALTW>(dl, P.eps4, pp.wtype, W, t1, t2, t3) & ok;
+          if (h) {
+            const ff dc[5] = {pc[0][v], pc[GRAV ? 1 : 0][v], pc[GRAV ? 2 : 0][v], pc[GRAV ? 3 : 0][v],
+                              pc[GRAV ? 4 : 0][v]};
+            third_differences(dc, t1, t2, t3);
+            ud[v] = weno_dif6(W, t1, t2, t3);
+            magu[v] = weno_mag6(W, t1, t2, t3);
+          } else {
+            xs[v] = weno_sum6(W, t1, t2, t3);
+            mag[v] = weno_mag6(W, t1, t2, t3);
+            sch[v] = weno_sum6(W, tg1, tg2, tg3) * lcol[v];
+            magg[v] = weno_mag6(W, tg1, tg2, tg3) * fabsf(lcol[v].h);
+          }
+          continue;
+        }
         ok = weno_window_corr<ALTW>(dl, P.eps4, pp.wtype, h ? us[v] : xs[v], h ? ud[v] : xd[v],
                                     h ? magu[v] : mag[v]) & ok;
       }
@@ -532,15 +661,24 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
       if (UPW == UPW_RUS) {
         const ff avg = (M == MODEL_EULER1D ? sqr(Ecc.a) : Ecc.a) + ffabs(Ecc.un);
         lm[0] = lm[1] = lm[2] = ffmax(ffmax(cl.c, cr.c), avg);
+        if (GRAV) lm[0] = lm[1] = lm[2] = lm[0] * kap;
         lam = fmaxf(lam, lm[0].h);
       } else if (UPW == UPW_ROE) {
 #pragma unroll
-        for (int k = 0; k < 3; k++) lm[k] = M == MODEL_EULER1D ? ffabs(lm[k]) : pharten(lm[k]);
+        for (int k = 0; k < 3; k++) {
+          lm[k] = M == MODEL_EULER1D ? ffabs(lm[k]) : pharten(lm[k]);
+          if (GRAV) lm[k] = lm[k] * kap;
+        }
+        if (GRAV) lam = fmul(lam, kap.h);
       } else {
         const ff cv = cl.vel[DIR], rv = cr.vel[DIR];
         pfield<UPW>(cv - cl.c, lm[0], rv - cr.c, lm[0], sg[0]);
         pfield<UPW>(cv + cl.c, lm[1], rv + cr.c, lm[1], sg[1]);
         pfield<UPW>(cv, lm[2], rv, lm[2], sg[2]);
+        if (GRAV) {
+#pragma unroll
+          for (int k = 0; k < 3; k++) lm[k] = lm[k] * kap;
+        }
         lam = fmaxf(lam, fmaxf(lm[0].h, lm[1].h));
       }
 #pragma unroll
@@ -552,6 +690,7 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
         xs[k] = acc_get(r);
       }
       pprojR<M, DIR>(Ecc, xs, g12);
+      if (GRAV) pprojR<M, DIR>(Ecc, sch, gs6);
     } else {
       ff fs6[NV], fd6[NV], us6[NV], ud6[NV], um[NV];
       pprojR<M, DIR>(Ecc, xs, fs6);
@@ -574,17 +713,23 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
     for (int k = 0; k < NV; k++) {
       const float sc = (M == MODEL_EULER1D && k < 2) ? Ecc.rs.h : 1.0f;
       ok = ok & (ffma(lam, magu[k], mag[k]) * sc <= 0.09375f * (k < 3 ? s0 : sm1));
+      if (GRAV && src_dir) ok = ok & (magg[k] * (float)term[0] * sc <= 0.09375f * (k < 3 ? s0 : sm1));
     }
   }
   __syncthreads();  // the differences are read no more: their place takes G and the cells' sums
   double* sg = sf + NV * S;
   double* sh = sg + NV * S;
+  double* ss = sh + NV * S;  // gravity: the source function's corrections, momentum and energy
   if (iface) {
     if (ok) {
 #pragma unroll
       for (int v = 0; v < NV; v++) sg[v * S + w] = to_double(ffc(1.0 / 12.0) * g12[v]);
+      if (GRAV && src_dir) {
+        ss[w] = to_double(ffc(1.0 / 12.0) * gs6[1 + DIR]);
+        ss[S + w] = to_double(ffc(1.0 / 12.0) * gs6[NV - 1]);
+      }
     } else {
-      iface_fp64<M, CHAR, UPW, DIR, ALTW>(su, sf, S, w, pp, sg + w);
+      iface_fp64<M, CHAR, UPW, DIR, ALTW, GRAV>(su, sf, sgf, sgg, S, w, pp, src_dir, sg + w, ss + w);
     }
     const int I = a0 - 2 + q;  // the interface right of the own cell
     if (ep.bnd && (I == 0 || I == N)) {
@@ -604,7 +749,14 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
     for (int v = 0; v < NV; v++) {
       const double* f = sf + v * S + w;
       const double c4 = fma(2.0 / 3.0, f[1] - f[-1], (f[2] - f[-2]) * (-1.0 / 12.0));
-      sh[v * S + w] = dxi * (c4 + (sg[v * S + w] - sg[v * S + w - 1]));
+      double h = dxi * (c4 + (sg[v * S + w] - sg[v * S + w - 1]));
+      if (GRAV && src_dir && (v == 1 + DIR || v == NV - 1)) {
+        const int k = v == 1 + DIR ? 0 : 1;
+        const double* g = sgg + w;
+        const double g4 = fma(2.0 / 3.0, g[1] - g[-1], (g[2] - g[-2]) * (-1.0 / 12.0));
+        h = fma(-term[k] * (g4 + (ss[k * S + w] - ss[k * S + w - 1])), dxi, h);  // rhs = -hyp + source
+      }
+      sh[v * S + w] = h;
     }
   }
   __syncthreads();
@@ -626,23 +778,23 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
   }
 }
 
-template <int M, bool CHAR, int UPW, int DIR, bool ALTW>
+template <int M, bool CHAR, int UPW, int DIR, bool ALTW, bool GRAV>
 __global__ void __launch_bounds__(256, 2)
 hyp_pair_kernel(const double* __restrict__ U, double* __restrict__ H, const double* __restrict__ dxinv, DevGeom G,
                 PhysParams pp, StageEpi ep, long long ntrans, int L, int XL) {
   extern __shared__ double pair_smem[];
-  pair_body<M, CHAR, UPW, DIR, ALTW>(U, H, dxinv, G, pp, ep, ntrans, L, XL, blockIdx.x, pair_smem);
+  pair_body<M, CHAR, UPW, DIR, ALTW, GRAV>(U, H, dxinv, G, pp, ep, ntrans, L, XL, blockIdx.x, pair_smem);
 }
 
-template <int M, bool CHAR, int UPW, int DIR, bool ALTW>
+template <int M, bool CHAR, int UPW, int DIR, bool ALTW, bool GRAV>
 cudaError_t launch_pair(const double* U, double* H, const double* dxinv_dir, const DevGeom& G, const PhysParams& pp,
                         const StageEpi& ep, long long ntrans, int cap, cudaStream_t s) {
   const int N = G.dim[DIR];
   const PairPlan p = pair_plan(N, ntrans, DIR, cap > 0 ? cap : pair_cap(ntrans * N));
   const long long nblk = (ntrans + p.XL - 1) / p.XL * ((N + p.L - 1) / p.L);
   if (nblk > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-  auto k = hyp_pair_kernel<M, CHAR, UPW, DIR, ALTW>;
-  const size_t sm = PairLayout<M, CHAR, UPW, ALTW>::bytes(p.T);
+  auto k = hyp_pair_kernel<M, CHAR, UPW, DIR, ALTW, GRAV>;
+  const size_t sm = PairLayout<M, CHAR, UPW, ALTW, GRAV>::bytes(p.T);
   if (sm > 48 * 1024)
     if (cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) return e;
   k<<<(unsigned)nblk, p.T, sm, s>>>(U, H, dxinv_dir, G, pp, ep, ntrans, p.L, p.XL);
@@ -669,7 +821,7 @@ cudaError_t launch_batched_dir(const MemberDev* mem, int nmem, long long nblk, i
   if (nblk <= 0) return cudaSuccess;
   if (nblk > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
   auto k = hyp_batched_pair_kernel<M, CHAR, UPW, DIR>;
-  const size_t sm = PairLayout<M, CHAR, UPW, false>::bytes(T);
+  const size_t sm = PairLayout<M, CHAR, UPW, false, false>::bytes(T);
   if (sm > 48 * 1024)
     if (cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) return e;
   k<<<(unsigned)nblk, T, sm, s>>>(mem, nmem, U, H, dxinv, pp, ep);
