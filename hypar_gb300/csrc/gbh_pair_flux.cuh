@@ -291,20 +291,24 @@ __device__ __forceinline__ void pupwind(const ff* fs6, const ff* fd6, const ff* 
   (void)ND;
 }
 
-// The FP64 evaluation of one interface (window in shared memory, own cell = slot w) as
-// the correction G, written to G[v S]; with gravity (sgf, sgg: the hydrostatic fields)
-// also the source function's interface values as corrections of its central value, to Gs.
+// The FP64 evaluation of one interface as the correction G, written to G[v S]; with
+// gravity (sgf, sgg: the hydrostatic fields) also the source function's interface values
+// as corrections of its central value, to Gs.  Window: cells i-2 .. i+3 of the line with
+// base point pb (states from memory), own cell = slot w (fluxes in shared memory).
 template <int M, bool CHAR, int UPW, int DIR, bool ALTW, bool GRAV>
-__device__ __forceinline__ void iface_fp64(const double* su, const double* sf, const double* sgf, const double* sgg,
-                                           int S, int w, const PhysParams& pp, bool src_dir, double* G, double* Gs) {
+__device__ __forceinline__ void iface_fp64(const double* __restrict__ U, long long pb, int i, const DevGeom& geo,
+                                           const double* sf, const double* sgf, const double* sgg, int S, int w,
+                                           const PhysParams& pp, bool src_dir, double* G, double* Gs) {
   constexpr int NV = ModelTraits<M>::NV;
   double wu[6][NV], wf[6][NV], wuc[6], wgf[6], wgg[6], fI[NV], SI[NV];
   CellAux<M> ax[6];
 #pragma unroll
   for (int p = 0; p < 6; p++) {
+    const double* src = U + (pb + (long long)fold_index(i - 2 + p, geo.dim[DIR], geo.bclo[DIR], geo.bchi[DIR]) *
+                                      geo.stride[DIR]) * NV;
 #pragma unroll
     for (int v = 0; v < NV; v++) {
-      wu[p][v] = su[v * S + w - 2 + p];
+      wu[p][v] = src[v];
       wf[p][v] = sf[v * S + w - 2 + p];
     }
     const Prim<M> q = to_prim<M>(wu[p], pp);
@@ -338,20 +342,71 @@ __device__ __forceinline__ void iface_fp64(const double* su, const double* sf, c
   }
 }
 
-// Shared memory of a block of T threads (slots S = T + 4): u and f (doubles), their right
-// differences (pairs), the cells' ingredients, and for the component-wise form one
-// component's sub-stencil rows, double-buffered; with gravity the hydrostatic fields.
+// stage_epilogue of NB values at once: all reads are issued before the first write, so
+// that their latencies overlap.
+template <int NB>
+__device__ __forceinline__ void stage_epilogue_batch(const StageEpi& ep, double* __restrict__ H, const long long* off,
+                                                     const double* h, const bool* on) {
+  const bool finish = ep.last && ep.mode != EPI_HYP, rk = finish && ep.mode != EPI_RHS;
+  double x[NB], par[NB], u[NB], a[NB], p[NB][4];
+#pragma unroll
+  for (int k = 0; k < NB; k++) {
+    if (!on[k]) continue;
+    x[k] = ep.first ? 0.0 : H[off[k]];
+    par[k] = (finish && ep.par) ? ep.par[off[k]] : 0.0;
+    u[k] = (rk && ep.need_u) ? ep.u[off[k]] : 0.0;
+    a[k] = (rk && ep.stage != 0) ? ep.acc[off[k]] : u[k];
+#pragma unroll
+    for (int t = 1; t < 4; t++)
+      p[k][t] = (rk && t > ep.stage && t < ep.nstages && ep.ca[t] != 0.0 && ep.touched[t]) ? ep.P[t][off[k]] : u[k];
+  }
+#pragma unroll
+  for (int k = 0; k < NB; k++) {
+    if (!on[k]) continue;
+    const double hyp = ep.first ? h[k] : x[k] + h[k];
+    if (!finish) {
+      H[off[k]] = hyp;
+      continue;
+    }
+    const double kv = par[k] - hyp;
+    if (!rk) {
+      ep.rhs[off[k]] = kv;
+      continue;
+    }
+    const double av = fma(ep.cb, kv, a[k]);
+    if (ep.stage == ep.nstages - 1) ep.uout[off[k]] = av;
+    else ep.acc[off[k]] = av;
+#pragma unroll
+    for (int t = 1; t < 4; t++)
+      if (t > ep.stage && t < ep.nstages && ep.ca[t] != 0.0) ep.P[t][off[k]] = fma(ep.ca[t], kv, p[k][t]);
+  }
+}
+
+// Shared memory of a block of T threads (slots S = T + 4), in 8-byte words per slot:
+//   f (doubles);
+//   the right differences of f and u (pairs; with gravity also of the modified solution
+//   and of g); component-wise, a component's two rows take its results once its
+//   sub-stencils are done;
+//   the cells' ingredients;
+//   u (doubles) and, component-wise, the sub-stencils of one component of f and u, which
+//   take u's place unless the mean states are still formed from it;
+//   characteristic: the fields' results; mean states and RF's differences where needed;
+//   with gravity the hydrostatic fields.
 template <int M, bool CHAR, int UPW, bool ALTW, bool GRAV>
 struct PairLayout {
   static constexpr int NV = ModelTraits<M>::NV, ND = ModelTraits<M>::ND;
   static constexpr bool CC = NeedCC<M, CHAR, UPW>::value;
   static constexpr bool NEEDC = UPW == UPW_RUS || (M == MODEL_EULER1D && UPW != UPW_ROE);
+  static constexpr bool STATES = (UPW == UPW_ROE && M == MODEL_EULER2D) ||
+                                 ((UPW == UPW_LLF || UPW == UPW_RF) && M != MODEL_EULER1D);
   static constexpr int NA = (CC ? ND + 2 : 0) + (NEEDC ? 1 : 0);
-  static constexpr int NR = ALTW ? 6 : 4;                // pairs of a row
-  static constexpr int NROW = CHAR ? 0 : 2 * 2 * NR;     // two buffers of the f and u rows
-  // differences: f, u; with gravity also of the modified solution and of g
-  static constexpr int ND_ROWS = 2 * NV + (GRAV ? NV + 1 : 0);
-  static constexpr int WORDS = 2 * NV + ND_ROWS + NA + NROW + (GRAV ? 2 : 0);  // 8-byte words per slot
+  static constexpr int NR = ALTW ? 6 : 4;  // pairs of a sub-stencil row
+  static constexpr int NDIF = 2 * NV + (GRAV ? NV + 1 : 0);
+  static constexpr bool KEEP_U = CHAR || STATES;
+  static constexpr int NROW = CHAR ? 0 : 2 * NR;
+  static constexpr int NU = KEEP_U ? NV + NROW : (NV > NROW ? NV : NROW);
+  static constexpr int NRES = (CHAR ? 2 * NV : 0) + (STATES ? NV : 0) + (UPW == UPW_RF ? NV : 0);
+  static constexpr int WORDS = NV + NDIF + NA + NU + NRES + (GRAV ? 2 : 0);
   static size_t bytes(int T) { return (size_t)WORDS * (T + 4) * 8; }
 };
 
@@ -366,14 +421,17 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
                                           double* sm) {
   using LY = PairLayout<M, CHAR, UPW, ALTW, GRAV>;
   constexpr int NV = LY::NV, ND = LY::ND, NR = LY::NR;
-  constexpr bool CC = LY::CC, NEEDC = LY::NEEDC;
+  constexpr bool CC = LY::CC, NEEDC = LY::NEEDC, STATES = LY::STATES;
   const int T = blockDim.x, S = T + 4, t = threadIdx.x;
-  double* su = sm;
-  double* sf = su + NV * S;
+  double* sf = sm;
   ff* sd = (ff*)(sf + NV * S);  // rows 0..NV-1: f, NV..2NV-1: u, then the modified solution and g
-  ff* sa = sd + LY::ND_ROWS * S;
-  ff* sr = sa + LY::NA * S;
-  double* sgf = (double*)(sr + LY::NROW * S);
+  ff* sa = sd + LY::NDIF * S;
+  double* su = (double*)(sa + LY::NA * S);
+  ff* sr = (ff*)su + (LY::KEEP_U ? NV * S : 0);  // rows of f's component, then of u's
+  ff* sx = (ff*)su + LY::NU * S;                 // characteristic: 2 NV results; mean states; RF's differences
+  ff* sum = sx + (CHAR ? 2 * NV * S : 0);
+  ff* sfd = sum + (STATES ? NV * S : 0);
+  double* sgf = (double*)(sx + LY::NRES * S);
   double* sgg = sgf + S;
   const bool src_dir = GRAV && pp.grav[DIR] != 0.0 && (ep.mode != EPI_HYP || ep.with_source);
   const int N = G.dim[DIR], LL = L + 6;
@@ -399,6 +457,7 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
   if (DIR == 0) {
     for (int l = 0; l < nl; l++) {
       const long long pb = line_base(l0 + l);
+#pragma unroll 4
       for (int i = t; i < (Lc + 6) * NV; i += T) {
         const int c = i / NV, v = i - c * NV;
         su[v * S + l * LL + c] = U[(pb + (long long)fold_index(a0 - 3 + c, N, lo, hi) * sdir) * NV + v];
@@ -408,6 +467,7 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
     const int R = nl * NV, c0 = t / R, r = t - c0 * R, l = r / NV, v = r - l * NV, step = T / R;
     if (c0 < step) {
       const long long pb = line_base(l0 + l);
+#pragma unroll 4
       for (int c = c0; c < Lc + 6; c += step)
         su[v * S + l * LL + c] = U[(pb + (long long)fold_index(a0 - 3 + c, N, lo, hi) * sdir) * NV + v];
     }
@@ -475,24 +535,17 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
     for (int v = 0; v < NV; v++) sd[(2 * NV + v) * S + w] = dc[v];
     sd[3 * NV * S + w] = to_pair(sgg[w + 1] - sgg[w]);
   }
-  {
 #pragma unroll
-    for (int v = 0; v < NV; v++) {
-      sd[v * S + w] = to_pair(sf[v * S + w + 1] - sf[v * S + w]);
-      sd[(NV + v) * S + w] = to_pair(su[v * S + w + 1] - su[v * S + w]);
-    }
+  for (int v = 0; v < NV; v++) {
+    sd[v * S + w] = to_pair(sf[v * S + w + 1] - sf[v * S + w]);
+    sd[(NV + v) * S + w] = to_pair(su[v * S + w + 1] - su[v * S + w]);
   }
   __syncthreads();
   const bool iface = line < nl && q >= 2 && q <= Lc + 2;
   const bool own = line < nl && q >= 3 && q <= Lc + 2;
-  constexpr bool STATES = (UPW == UPW_ROE && M == MODEL_EULER2D) ||
-                          ((UPW == UPW_LLF || UPW == UPW_RF) && M != MODEL_EULER1D);
   bool ok = true;
   ff g12[NV];
-  float mag[NV], lam = 0.0f, rho = 0.0f, Hs = 0.0f;  // 6 x the terms of f per component, and of u
-  float magu[NV];
-  PCell<M> cl, cr;
-  PEig Ecc;
+  float lam, rho, Hs;
   auto cell_of = [&](int x) {
     PCell<M> c;
     c.t = c.H = c.c = ff{1.0f, 0.0f};
@@ -507,8 +560,8 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
     if (NEEDC) c.c = sa[(CC ? ND + 2 : 0) * S + x];
     return c;
   };
-  ff gs6[NV], tg1, tg2, tg3, kap;  // gravity: the source function's corrections, the dissipation's factor
-  float magg[NV];
+  // gravity: the source function's corrections (momentum, energy), the dissipation's factor
+  ff gsm = {0.0f, 0.0f}, gse = {0.0f, 0.0f}, tg1, tg2, tg3, kap;
   if (GRAV) {
     const ff* dd = sd + 3 * NV * S + w;
     const ff dl[5] = {dd[-2], dd[-1], dd[0], dd[1], dd[2]};
@@ -516,90 +569,105 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
     kap = to_pair(fmax(sgg[w], sgg[w + 1]));
   }
   if (!CHAR) {
-    ff fs6[NV], fd6[NV], us6[NV], ud6[NV], um[NV];
-#pragma unroll
+    // 6 x the terms of density, the momenta (largest), energy: of f, of u
+    float m0 = 0.0f, mm = 0.0f, mE = 0.0f, u0 = 0.0f, um = 0.0f, uE = 0.0f, magsm = 0.0f, magse = 0.0f;
+#pragma unroll 1
     for (int v = 0; v < NV; v++) {
-      ff* rows = sr + (v & 1) * 2 * NR * S;
-      {
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-          const ff* dd = sd + (h * NV + v) * S;
-          const PRow r = weno_row<ALTW>(dd[w - 1], dd[w], P.eps4, pp.wtype == PW_NONE);
-          ff* o = rows + h * NR * S + w;
-          o[0] = r.d;
-          o[S] = r.l;
-          o[2 * S] = r.c;
-          o[3 * S] = r.r;
-          if (ALTW) {
-            o[4 * S] = r.bl;
-            o[5 * S] = r.br;
-          }
+      for (int h = 0; h < 2; h++) {
+        const ff* dd = sd + (h * NV + v) * S;
+        const PRow r = weno_row<ALTW>(dd[w - 1], dd[w], P.eps4, pp.wtype == PW_NONE);
+        ff* o = sr + h * NR * S + w;
+        o[0] = r.d;
+        o[S] = r.l;
+        o[2 * S] = r.c;
+        o[3 * S] = r.r;
+        if (ALTW) {
+          o[4 * S] = r.bl;
+          o[5 * S] = r.br;
         }
       }
       __syncthreads();
-      {
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-          const ff* o = rows + h * NR * S + w;
-          ff bl1, br3, br4, bl2;
-          bl1 = br3 = br4 = bl2 = ff{0.0f, 0.0f};
-          if (ALTW) {
-            bl1 = o[4 * S - 1];
-            bl2 = o[4 * S];
-            br3 = o[5 * S + 1];
-            br4 = o[5 * S + 2];
-          }
-          if (GRAV) {
-            ff t1 = o[0] - o[-1], t2 = o[1] - o[0], t3 = o[2] - o[1];
-            PWeights W;
-            ok = weno_pair_weights<ALTW>(t1, t2, t3, o[S - 1], o[2 * S], o[3 * S + 1], o[3 * S + 2], o[2 * S + 1],
-                                         o[S], bl1, br3, br4, bl2, pp.wtype, W) & ok;
-            if (h) {  // weights of u, values of the modified solution
-              const ff* dd = sd + (2 * NV + v) * S + w;
-              const ff dl[5] = {dd[-2], dd[-1], dd[0], dd[1], dd[2]};
-              third_differences(dl, t1, t2, t3);
-              ud6[v] = weno_dif6(W, t1, t2, t3);
-              magu[v] = weno_mag6(W, t1, t2, t3);
+      for (int h = 0; h < 2; h++) {
+        const ff* o = sr + h * NR * S + w;
+        ff bl1, br3, br4, bl2;
+        bl1 = br3 = br4 = bl2 = ff{0.0f, 0.0f};
+        if (ALTW) {
+          bl1 = o[4 * S - 1];
+          bl2 = o[4 * S];
+          br3 = o[5 * S + 1];
+          br4 = o[5 * S + 2];
+        }
+        const ff d2 = o[0], d3 = o[1];
+        ff t1 = d2 - o[-1], t2 = d3 - d2, t3 = o[2] - d3;
+        PWeights W;
+        ok = weno_pair_weights<ALTW>(t1, t2, t3, o[S - 1], o[2 * S], o[3 * S + 1], o[3 * S + 2], o[2 * S + 1], o[S],
+                                     bl1, br3, br4, bl2, pp.wtype, W) & ok;
+        ff* res = sd + (h * NV + v) * S + w;  // this component's differences are read no more
+        float mag;
+        if (h == 0) {
+          mag = weno_mag6(W, t1, t2, t3);
+          if (UPW == UPW_RF) sfd[v * S + w] = weno_dif6(W, t1, t2, t3);
+          if (GRAV && (v == 1 + DIR || v == NV - 1)) {
+            const ff g = weno_sum6(W, tg1, tg2, tg3);
+            const float mg = weno_mag6(W, tg1, tg2, tg3);
+            if (v == NV - 1) {
+              gse = g;
+              magse = mg;
             } else {
-              fs6[v] = weno_sum6(W, t1, t2, t3);
-              mag[v] = weno_mag6(W, t1, t2, t3);
-              if (v == 1 + DIR || v == NV - 1) {
-                gs6[v] = weno_sum6(W, tg1, tg2, tg3);
-                magg[v] = weno_mag6(W, tg1, tg2, tg3);
-              }
+              gsm = g;
+              magsm = mg;
             }
-            continue;
           }
-          ok = weno_pair_corr<ALTW>(o[-1], o[0], o[1], o[2], o[S - 1], o[2 * S], o[3 * S + 1], o[3 * S + 2],
-                                    o[2 * S + 1], o[S], bl1, br3, br4, bl2, pp.wtype, h ? us6[v] : fs6[v],
-                                    h ? ud6[v] : fd6[v], h ? magu[v] : mag[v]) & ok;
-          if (h && STATES) um[v] = pmean(to_pair(su[v * S + w]), sd[(NV + v) * S + w], o[0], o[1], us6[v]);
+          *res = weno_sum6(W, t1, t2, t3);
+          m0 = v == 0 ? mag : m0;
+          mm = (v > 0 && v < NV - 1 && !(mag <= mm)) ? mag : mm;  // a NaN stays
+          mE = v == NV - 1 ? mag : mE;
+        } else {
+          if (STATES) sum[v * S + w] = pmean(to_pair(su[v * S + w]), *res, d2, d3, weno_sum6(W, t1, t2, t3));
+          if (GRAV) {  // weights of u, values of the modified solution
+            const ff* dd = sd + (2 * NV + v) * S + w;
+            const ff dl[5] = {dd[-2], dd[-1], dd[0], dd[1], dd[2]};
+            third_differences(dl, t1, t2, t3);
+          }
+          mag = weno_mag6(W, t1, t2, t3);
+          *res = weno_dif6(W, t1, t2, t3);
+          u0 = v == 0 ? mag : u0;
+          um = (v > 0 && v < NV - 1 && !(mag <= um)) ? mag : um;
+          uE = v == NV - 1 ? mag : uE;
         }
       }
+      __syncthreads();
     }
-    {
-      if (CC || NEEDC) {
-        cl = cell_of(w);
-        cr = cell_of(w + 1);
-      }
-      if (CC) Ecc = peig<M, DIR>(cl, cr, P);
-      pupwind<M, UPW, DIR>(fs6, fd6, ud6, um, Ecc, cl, cr, P, g12, lam, rho, Hs, GRAV ? &kap : nullptr);
-      const float s0 = rho * lam, sm1 = s0 * lam, sE = s0 * Hs;
+    ff fs6[NV], fd6[NV], ud6[NV], us[NV];
 #pragma unroll
-      for (int v = 0; v < NV; v++) {
-        const float s = v == 0 ? s0 : (v == NV - 1 ? sE : sm1);
-        ok = ok & (ffma(lam, magu[v], mag[v]) <= 0.09375f * s) & (s >= 8.7e-19f) & (s <= 1.2e30f);
-      }
-      if (GRAV && src_dir) {
-        const float rt = (float)term[0];
-        ok = ok & (magg[1 + DIR] * rt <= 0.09375f * sm1) & (magg[NV - 1] * rt * lam <= 0.09375f * sE);
-      }
+    for (int v = 0; v < NV; v++) {
+      fs6[v] = sd[v * S + w];
+      ud6[v] = sd[(NV + v) * S + w];
+      if (UPW == UPW_RF) fd6[v] = sfd[v * S + w];
+      if (STATES) us[v] = sum[v * S + w];
+    }
+    PCell<M> cl, cr;
+    PEig Ecc;
+    if (CC || NEEDC) {
+      cl = cell_of(w);
+      cr = cell_of(w + 1);
+    }
+    if (CC) Ecc = peig<M, DIR>(cl, cr, P);
+    pupwind<M, UPW, DIR>(fs6, fd6, ud6, us, Ecc, cl, cr, P, g12, lam, rho, Hs, GRAV ? &kap : nullptr);
+    const float s0 = rho * lam, sm1 = s0 * lam, sE = s0 * Hs;
+    ok = ok & (ffma(lam, u0, m0) <= 0.09375f * s0) & (ffma(lam, um, mm) <= 0.09375f * sm1) &
+         (ffma(lam, uE, mE) <= 0.09375f * sE);
+    ok = ok & (s0 >= 8.7e-19f) & (s0 <= 1.2e30f) & (sm1 >= 8.7e-19f) & (sm1 <= 1.2e30f) & (sE >= 8.7e-19f) &
+         (sE <= 1.2e30f);
+    if (GRAV && src_dir) {
+      const float rt = (float)term[0];
+      ok = ok & (magsm * rt <= 0.09375f * sm1) & (magse * rt * lam <= 0.09375f * sE);
     }
   } else {
-    cl = cell_of(w);
-    cr = cell_of(w + 1);
-    Ecc = peig<M, DIR>(cl, cr, P);
-    ff xs[NV], xd[NV], us[NV], ud[NV];
+    PCell<M> cl = cell_of(w), cr = cell_of(w + 1);
+    PEig Ecc = peig<M, DIR>(cl, cr, P);
     ff lcol[NV], sch[NV];  // L (e_{1+DIR} + e_E): the source function's projection per unit of g
     if (GRAV) {
       ff ev[NV];
@@ -607,49 +675,81 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
       for (int v = 0; v < NV; v++) ev[v] = ff{(v == 1 + DIR || v == NV - 1) ? 1.0f : 0.0f, 0.0f};
       pprojL<M, DIR>(Ecc, P, ev, lcol);
     }
-#pragma unroll
+    // Per unit of g, the source function's terms; 6 x the terms of fields 0-2, of the shear
+    // fields, of f, of u (the largest of each).
+    float ma = 0.0f, ms = 0.0f, ua = 0.0f, us = 0.0f, magg = 0.0f;
+    const float sc01 = M == MODEL_EULER1D ? Ecc.rs.h : 1.0f;
+    const ff gh = P.gm1 * Ecc.hac, ah = Ecc.a * Ecc.hac;
+#pragma unroll 1
     for (int h = 0; h < 2; h++) {
-      ff pj[5][NV], pc[GRAV ? 5 : 1][NV];
-      if (GRAV && h) {
+      // the projections' common parts at the five faces: s/(gamma-1) times (gamma-1) hac, t hac
+      const ff* x = sd + h * NV * S + w - 2;
+      const ff* xc = sd + 2 * NV * S + w - 2;  // gravity: the modified solution
+      ff gs[5], th[5], gc[GRAV ? 5 : 1], tc[GRAV ? 5 : 1];
+      auto parts = [&](const ff* y, ff& a, ff& b) {
+        FAcc acc = acc_mul(Ecc.ek, y[0]);
 #pragma unroll
-        for (int k = 0; k < 5; k++) {
-          ff x[NV];
-#pragma unroll
-          for (int v = 0; v < NV; v++) x[v] = sd[(2 * NV + v) * S + w - 2 + k];
-          pprojL<M, DIR>(Ecc, P, x, pc[GRAV ? k : 0]);
-        }
-      }
+        for (int e = 0; e < ND; e++) acc_fma(acc, neg(Ecc.vel[e]), y[(1 + e) * S]);
+        acc_add(acc, y[(NV - 1) * S]);
+        a = acc_get(acc);
+        b = ah * (Ecc.un * y[0] - y[(1 + DIR) * S]);
+      };
+      // field v of the difference at one face, from its common parts
+      auto field = [&](const ff* y, int v, ff a, ff b) {
+        if (v == 0) return gh * a + b;
+        if (v == 1) return gh * a - b;
+        if (v == 2) return y[0] - Ecc.gi * a;
+        const int e = (v - 3) + ((v - 3) >= DIR ? 1 : 0);  // the shear fields: transverse directions ascending
+        return Ecc.vel[e < ND ? e : 0] * y[0] - y[(1 + e) * S];
+      };
 #pragma unroll
       for (int k = 0; k < 5; k++) {
-        ff x[NV];
-#pragma unroll
-        for (int v = 0; v < NV; v++) x[v] = sd[(h * NV + v) * S + w - 2 + k];
-        pprojL<M, DIR>(Ecc, P, x, pj[k]);
+        parts(x + k, gs[k], th[k]);
+        if (GRAV) {
+          if (h) parts(xc + k, gc[GRAV ? k : 0], tc[GRAV ? k : 0]);
+        }
       }
 #pragma unroll
       for (int v = 0; v < NV; v++) {
-        const ff dl[5] = {pj[0][v], pj[1][v], pj[2][v], pj[3][v], pj[4][v]};
+        const ff dl[5] = {field(x, v, gs[0], th[0]), field(x + 1, v, gs[1], th[1]), field(x + 2, v, gs[2], th[2]),
+                          field(x + 3, v, gs[3], th[3]), field(x + 4, v, gs[4], th[4])};
+        PWeights W;
+        ff t1, t2, t3;
+        ok = weno_window_weights<ALTW>(dl, P.eps4, pp.wtype, W, t1, t2, t3) & ok;
         if (GRAV) {
-          PWeights W;
-          ff t1, t2, t3;
-          ok = weno_window_weights<ALTW>(dl, P.eps4, pp.wtype, W, t1, t2, t3) & ok;
           if (h) {
-            const ff dc[5] = {pc[0][v], pc[GRAV ? 1 : 0][v], pc[GRAV ? 2 : 0][v], pc[GRAV ? 3 : 0][v],
-                              pc[GRAV ? 4 : 0][v]};
+            const ff dc[5] = {field(xc, v, gc[0], tc[0]), field(xc + 1, v, gc[GRAV ? 1 : 0], tc[GRAV ? 1 : 0]),
+                              field(xc + 2, v, gc[GRAV ? 2 : 0], tc[GRAV ? 2 : 0]),
+                              field(xc + 3, v, gc[GRAV ? 3 : 0], tc[GRAV ? 3 : 0]),
+                              field(xc + 4, v, gc[GRAV ? 4 : 0], tc[GRAV ? 4 : 0])};
             third_differences(dc, t1, t2, t3);
-            ud[v] = weno_dif6(W, t1, t2, t3);
-            magu[v] = weno_mag6(W, t1, t2, t3);
           } else {
-            xs[v] = weno_sum6(W, t1, t2, t3);
-            mag[v] = weno_mag6(W, t1, t2, t3);
             sch[v] = weno_sum6(W, tg1, tg2, tg3) * lcol[v];
-            magg[v] = weno_mag6(W, tg1, tg2, tg3) * fabsf(lcol[v].h);
+            const float mg = weno_mag6(W, tg1, tg2, tg3) * fabsf(lcol[v].h) * (v < 2 ? sc01 : 1.0f);
+            magg = !(mg <= magg) ? mg : magg;
           }
-          continue;
         }
-        ok = weno_window_corr<ALTW>(dl, P.eps4, pp.wtype, h ? us[v] : xs[v], h ? ud[v] : xd[v],
-                                    h ? magu[v] : mag[v]) & ok;
+        float mag = weno_mag6(W, t1, t2, t3);
+        if (v < 2) mag = mag * sc01;
+        if (h == 0) {
+          sx[v * S + w] = weno_sum6(W, t1, t2, t3);
+          if (UPW == UPW_RF) sfd[v * S + w] = weno_dif6(W, t1, t2, t3);
+          if (v < 3) ma = !(mag <= ma) ? mag : ma;
+          else ms = !(mag <= ms) ? mag : ms;
+        } else {
+          sx[(NV + v) * S + w] = weno_dif6(W, t1, t2, t3);
+          if (STATES) sum[v * S + w] = weno_sum6(W, t1, t2, t3);
+          if (v < 3) ua = !(mag <= ua) ? mag : ua;
+          else us = !(mag <= us) ? mag : us;
+        }
       }
+    }
+    ff xs[NV], xd[NV], ud[NV];
+#pragma unroll
+    for (int v = 0; v < NV; v++) {
+      xs[v] = sx[v * S + w];
+      ud[v] = sx[(NV + v) * S + w];
+      if (UPW == UPW_RF) xd[v] = sfd[v * S + w];
     }
     constexpr bool SAME_BASIS = UPW == UPW_RUS || M == MODEL_EULER1D || (M == MODEL_NS3D && UPW == UPW_ROE);
     if (SAME_BASIS) {
@@ -686,17 +786,24 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
         const int m = k < 2 ? k : 2;
         FAcc r = acc_mul(neg(lm[m]), ud[k]);
         acc_add(r, xs[k]);
-        if (UPW == UPW_RF && sg[m] != 0.0f) acc_add(r, mul2(xd[k], -sg[m]));
+        if (UPW == UPW_RF) acc_add(r, mul2(xd[k], -sg[m]));
         xs[k] = acc_get(r);
       }
       pprojR<M, DIR>(Ecc, xs, g12);
-      if (GRAV) pprojR<M, DIR>(Ecc, sch, gs6);
+      if (GRAV) {
+        ff y[NV];
+        pprojR<M, DIR>(Ecc, sch, y);
+        gsm = y[1 + DIR];
+        gse = y[NV - 1];
+      }
     } else {
       ff fs6[NV], fd6[NV], us6[NV], ud6[NV], um[NV];
       pprojR<M, DIR>(Ecc, xs, fs6);
-      pprojR<M, DIR>(Ecc, us, us6);
       pprojR<M, DIR>(Ecc, ud, ud6);
       if (UPW == UPW_RF) pprojR<M, DIR>(Ecc, xd, fd6);
+#pragma unroll
+      for (int v = 0; v < NV; v++) xs[v] = STATES ? sum[v * S + w] : xs[v];
+      pprojR<M, DIR>(Ecc, xs, us6);
 #pragma unroll
       for (int v = 0; v < NV; v++) {
         const ff* dd = sd + (NV + v) * S + w;
@@ -708,30 +815,27 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
     const float s0 = rho * lam, sm1 = s0 * lam;
     const float sE = s0 * Hs;
     ok = ok & (s0 >= 8.7e-19f) & (s0 <= 1.2e30f) & (sm1 >= 8.7e-19f) & (sm1 <= 1.2e30f) & (sE >= 8.7e-19f) &
-         (sE <= 1.2e30f);
-#pragma unroll
-    for (int k = 0; k < NV; k++) {
-      const float sc = (M == MODEL_EULER1D && k < 2) ? Ecc.rs.h : 1.0f;
-      ok = ok & (ffma(lam, magu[k], mag[k]) * sc <= 0.09375f * (k < 3 ? s0 : sm1));
-      if (GRAV && src_dir) ok = ok & (magg[k] * (float)term[0] * sc <= 0.09375f * (k < 3 ? s0 : sm1));
-    }
+         (sE <= 1.2e30f) & (ffma(lam, ua, ma) <= 0.09375f * s0) & (ffma(lam, us, ms) <= 0.09375f * sm1);
+    if (GRAV && src_dir) ok = ok & (magg * (float)term[0] <= 0.09375f * s0);
   }
   __syncthreads();  // the differences are read no more: their place takes G and the cells' sums
   double* sg = sf + NV * S;
   double* sh = sg + NV * S;
   double* ss = sh + NV * S;  // gravity: the source function's corrections, momentum and energy
   if (iface) {
+    const int i = a0 - 3 + q;  // the own cell
     if (ok) {
 #pragma unroll
       for (int v = 0; v < NV; v++) sg[v * S + w] = to_double(ffc(1.0 / 12.0) * g12[v]);
       if (GRAV && src_dir) {
-        ss[w] = to_double(ffc(1.0 / 12.0) * gs6[1 + DIR]);
-        ss[S + w] = to_double(ffc(1.0 / 12.0) * gs6[NV - 1]);
+        ss[w] = to_double(ffc(1.0 / 12.0) * gsm);
+        ss[S + w] = to_double(ffc(1.0 / 12.0) * gse);
       }
     } else {
-      iface_fp64<M, CHAR, UPW, DIR, ALTW, GRAV>(su, sf, sgf, sgg, S, w, pp, src_dir, sg + w, ss + w);
+      iface_fp64<M, CHAR, UPW, DIR, ALTW, GRAV>(U, line_base(l0 + line), i, G, sf, sgf, sgg, S, w, pp, src_dir, sg + w,
+                                                ss + w);
     }
-    const int I = a0 - 2 + q;  // the interface right of the own cell
+    const int I = i + 1;  // the interface to its right
     if (ep.bnd && (I == 0 || I == N)) {
       double Fb[NV];
 #pragma unroll
@@ -761,25 +865,51 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
   }
   __syncthreads();
   // Stage epilogue, value by value in the order of memory.
+  constexpr int NB = 3;
+  long long off[NB];
+  double hv[NB];
+  bool on[NB];
   if (DIR == 0) {
     for (int l = 0; l < nl; l++) {
       const long long ob = (line_base(l0 + l) + (long long)a0 * sdir) * NV;
-      for (int i = t; i < Lc * NV; i += T) {
-        const int c = i / NV, v = i - c * NV;
-        stage_epilogue<1>(ep, H, ob + i, &sh[v * S + l * LL + c + 3]);
+      for (int i0 = t; i0 < Lc * NV; i0 += NB * T) {
+#pragma unroll
+        for (int k = 0; k < NB; k++) {
+          const int i = i0 + k * T, c = i / NV, v = i - c * NV;
+          on[k] = i < Lc * NV;
+          off[k] = ob + i;
+          hv[k] = on[k] ? sh[v * S + l * LL + c + 3] : 0.0;
+        }
+        stage_epilogue_batch<NB>(ep, H, off, hv, on);
       }
     }
   } else {
     const int R = nl * NV, c0 = t / R, r = t - c0 * R, l = r / NV, v = r - l * NV, step = T / R;
     if (c0 < step) {
       const long long ob = (line_base(l0 + l) + (long long)a0 * sdir) * NV + v;
-      for (int c = c0; c < Lc; c += step) stage_epilogue<1>(ep, H, ob + (long long)c * sdir * NV, &sh[v * S + l * LL + c + 3]);
+      for (int cc = c0; cc < Lc; cc += NB * step) {
+#pragma unroll
+        for (int k = 0; k < NB; k++) {
+          const int c = cc + k * step;
+          on[k] = c < Lc;
+          off[k] = ob + (long long)c * sdir * NV;
+          hv[k] = on[k] ? sh[v * S + l * LL + c + 3] : 0.0;
+        }
+        stage_epilogue_batch<NB>(ep, H, off, hv, on);
+      }
     }
   }
 }
 
+// Blocks of 256 threads per SM the kernels are held to.  Bound by issue slots and latency
+// (some 6000 mostly FP32 instructions per thread against 75 FP64 ones): two blocks (128
+// registers) left the schedulers idle half of the time; three (80 registers; spills in the
+// FP64 evaluation only) take the Taylor-Green 256^3 directions from 75.9 to 61.4 ms per RK4
+// step and the 1024^2 vortex from 3.12 to 2.56 ms per step, four (64 registers) are no
+// faster (61.7 and 2.54 ms; shared memory allows three).
+constexpr int PAIR_MINB = 3;
 template <int M, bool CHAR, int UPW, int DIR, bool ALTW, bool GRAV>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(256, PAIR_MINB)
 hyp_pair_kernel(const double* __restrict__ U, double* __restrict__ H, const double* __restrict__ dxinv, DevGeom G,
                 PhysParams pp, StageEpi ep, long long ntrans, int L, int XL) {
   extern __shared__ double pair_smem[];
@@ -803,7 +933,7 @@ cudaError_t launch_pair(const double* U, double* H, const double* dxinv_dir, con
 
 // Ensemble: the blocks of all members in one launch.
 template <int M, bool CHAR, int UPW, int DIR>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(256, PAIR_MINB)
 hyp_batched_pair_kernel(const MemberDev* __restrict__ mem, int nmem, const double* __restrict__ U,
                         double* __restrict__ H, const double* __restrict__ dxinv, PhysParams pp, StageEpi ep) {
   extern __shared__ double pair_smem[];
