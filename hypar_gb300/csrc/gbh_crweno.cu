@@ -116,6 +116,42 @@ __device__ __forceinline__ void cr_weights(const double* s, double c1, double c2
   cr_norm<ALT>(B1, B2, B3, t, c1, c2, c3, wtype, w1, w2, w3);
 }
 
+// The same weights of an interior interface in float pairs (gbh_pair.cuh) from the
+// sub-stencils' 1/B^2 (farthest upwind, central, downwind), optimal weights (0.2, 0.5,
+// 0.3); tau = 4 tau of the side (Borges, Yamaleev-Carpenter).  False where their sum
+// leaves the pairs' range.
+template <bool ALT>
+__device__ __forceinline__ bool cr_weights_pair(ff i1, ff i2, ff i3, ff tau, int wtype, ff& w1, ff& w2, ff& w3) {
+  if (ALT && wtype == WENO_W_NONE) {
+    w1 = ffc(0.2);
+    w2 = ffc(0.5);
+    w3 = ffc(0.3);
+    return true;
+  }
+  if (ALT && (wtype == WENO_W_BORGES || wtype == WENO_W_YC)) {
+    const ff T = sqr(tau), one = {1.0f, 0.0f};
+    i1 = T * i1 + one;
+    i2 = T * i2 + one;
+    i3 = T * i3 + one;
+  }
+  i1 = mul2(i1, 2.0f);  // x 10 of the optimal weights
+  i2 = mulf(i2, 5.0f);
+  i3 = mulf(i3, 3.0f);
+  const ff S = addu(addu(i1, i2), i3);
+  const ff r = rcp(S);
+  w1 = i1 * r;
+  w2 = i2 * r;
+  w3 = i3 * r;
+  if (ALT && wtype == WENO_W_MAPPED) {
+    const ff m1 = mapped_weight(w1, 0.2), m2 = mapped_weight(w2, 0.5), m3 = mapped_weight(w3, 0.3);
+    const ff n = rcp(addu(addu(m1, m2), m3));
+    w1 = m1 * n;
+    w2 = m2 * n;
+    w3 = m3 * n;
+  }
+  return (S.h >= 7.888609e-31f) & (S.h <= 1.0e36f);
+}
+
 // Grid line `tr` along DIR: offset (in points) of its cell 0.
 template <int ND, int DIR>
 __device__ __forceinline__ long long line_base(const DevGeom& G, long long tr) {
@@ -181,14 +217,7 @@ __device__ __forceinline__ void cr_cell(const double* __restrict__ src, const do
 #pragma unroll
     for (int e = 1; e < NV; e++)
       if (v == e) x = uu[e];
-    wv = x;
-    if (M == MODEL_NS3D && v == NV - 1) {
-      // the modified solution's energy (NavierStokes3DModifiedSolution.c:65)
-      Prim<M> q = to_prim<M>(uu, pp);
-      val = ufunc_energy<M>(q, pp, uu[NV - 1]);
-    } else {
-      val = x;
-    }
+    val = wv = x;  // the modified solution without gravity is u (its energy up to rounding)
   }
 }
 
@@ -219,6 +248,17 @@ cr_solve_kernel(const double* __restrict__ U, const double* __restrict__ F, DevG
   };
 #pragma unroll
   for (int p = 0; p < 5; p++) load(p - 3, p + 1);
+  // the sub-stencils of window cells 1 .. 4 (I-2 .. I+1) and the last right difference
+  const ff peps4 = to_pair(eps4);
+  const bool none = ALTW && pp.wtype == WENO_W_NONE;
+  PRow row[5];
+  ff dlast = to_pair(wwv[2] - wwv[1]);
+#pragma unroll
+  for (int p = 2; p < 5; p++) {
+    const ff dn = to_pair(wwv[p + 1] - wwv[p]);
+    row[p] = weno_row<ALTW, false>(dlast, dn, peps4, none);
+    dlast = dn;
+  }
 
   double cprev = 0.0, xprev = 0.0;
   for (int I = 0; I <= N; I++) {
@@ -227,18 +267,50 @@ cr_solve_kernel(const double* __restrict__ U, const double* __restrict__ F, DevG
       wval[p] = wval[p + 1];
       wwv[p] = wwv[p + 1];
     }
+    row[1] = row[2];
+    row[2] = row[3];
+    row[3] = row[4];
     load(I + 2, 5);
-    // the biased stencil (f_{j-2}, f_{j-1}, f_j, f_{j+1}, f_{j+2}) of this interface
-    double sw[5], sv[5];
-#pragma unroll
-    for (int p = 0; p < 5; p++) {
-      sw[p] = left ? wwv[p] : wwv[5 - p];
-      sv[p] = left ? wval[p] : wval[5 - p];
+    {
+      const ff dn = to_pair(wwv[5] - wwv[4]);
+      row[4] = weno_row<ALTW, false>(dlast, dn, peps4, none);
+      dlast = dn;
     }
+    // the biased stencil (f_{j-2}, f_{j-1}, f_j, f_{j+1}, f_{j+2}) of this interface
+    double sv[5];
+#pragma unroll
+    for (int p = 0; p < 5; p++) sv[p] = left ? wval[p] : wval[5 - p];
     const bool bnd = (I == 0) || (I == N);
+    // Weights in pairs: an error e of a weight moves the interface value by about e/20 of
+    // the stencil's third differences; where those exceed 1/16 of its values (or the pairs'
+    // range is left, or something is not finite), and for gravity's source function, whose
+    // values are not the weights', the weights are formed in FP64.
     double w1, w2, w3;
-    if (bnd) cr_weights<ALTW>(sw, 0.1, 0.6, 0.3, eps4, pp.wtype, w1, w2, w3);
-    else cr_weights<ALTW>(sw, 0.2, 0.5, 0.3, eps4, pp.wtype, w1, w2, w3);
+    bool ok;
+    {
+      const ff t1 = left ? row[2].d - row[1].d : row[3].d - row[4].d;
+      const ff t2 = left ? row[3].d - row[2].d : row[2].d - row[3].d;
+      ff tau = {0.0f, 0.0f};
+      if (ALTW && pp.wtype == WENO_W_BORGES) tau = left ? row[1].bl - row[3].br : row[4].br - row[2].bl;
+      if (ALTW && pp.wtype == WENO_W_YC) tau = mul2(sqr(t2 - t1), 4.0f);
+      ff p1, p2, p3;
+      ok = cr_weights_pair<ALTW>(left ? row[1].l : row[4].r, left ? row[2].c : row[3].c, left ? row[3].r : row[2].l,
+                                 tau, pp.wtype, p1, p2, p3);
+      float m = 0.0f;
+#pragma unroll
+      for (int p = 0; p < 6; p++) m = fmaxf(m, d2f_mag(wval[p]));
+      ok = ok & (fadd(fabsf(t1.h), fabsf(t2.h)) <= 0.0625f * m) & (m >= 8.7e-19f) & (m <= 1.2e30f) & !(GRAV && k >= 4);
+      w1 = to_double(p1);
+      w2 = to_double(p2);
+      w3 = to_double(p3);
+    }
+    if (bnd || !ok) {
+      double sw[5];
+#pragma unroll
+      for (int p = 0; p < 5; p++) sw[p] = left ? wwv[p] : wwv[5 - p];
+      const double c1 = bnd ? 0.1 : 0.2, c2 = bnd ? 0.6 : 0.5;
+      cr_weights<ALTW>(sw, c1, c2, 0.3, eps4, pp.wtype, w1, w2, w3);
+    }
     double cI, xI;
     if (bnd) {
       // explicit WENO5 value: identity row
@@ -537,6 +609,24 @@ cr_char_solve_kernel(const double* __restrict__ U, DevGeom G, PhysParams pp, dou
   }
 }
 
+// A cell's ingredients as pairs.
+template <int M, int UPW>
+__device__ __forceinline__ PCell<M> pair_cell(const CellAux<M>& a) {
+  constexpr int ND = ModelTraits<M>::ND;
+  PCell<M> c;
+  c.t = c.H = c.c = ff{1.0f, 0.0f};
+#pragma unroll
+  for (int k = 0; k < 3; k++) c.vel[k] = ff{0.0f, 0.0f};
+  if (NeedCC<M, false, UPW>::value) {
+    c.t = to_pair(a.rs.t);
+#pragma unroll
+    for (int k = 0; k < ND; k++) c.vel[k] = to_pair(a.rs.vel[k]);
+    c.H = to_pair(a.rs.H);
+  }
+  if (UPW == UPW_RUS || (M == MODEL_EULER1D && UPW != UPW_ROE)) c.c = to_pair(a.c);
+  return c;
+}
+
 // GRAV: the dissipation scaled by max(g_L, g_R) of the gravity field (Euler1DUpwind.c:79-82,
 // NavierStokes3DUpwind.c:407) and, along a direction with gravity, the well-balanced
 // source term (Euler1DSource.c:58-76, NavierStokes3DSource.c:73-101): the average of
@@ -576,6 +666,12 @@ cr_flux_kernel(const double* __restrict__ U, double* __restrict__ H, const doubl
     if (GRAV) gv = pp.gg[pt];
     return a;
   };
+  constexpr bool STATES = (UPW == UPW_ROE && M == MODEL_EULER2D) ||
+                          ((UPW == UPW_LLF || UPW == UPW_RF) && M != MODEL_EULER1D);
+  PParams P;
+  P.gm1 = to_pair(pp.gm1);
+  P.gamma = to_pair(pp.gamma);
+  P.eps4 = to_pair(4.0 * pp.eps);
   double gL = 1.0, gR = 1.0;
   CellAux<M> axL = aux(I0 - 1, gL);
   double fIp[NV], SI[NV], SIp[NV];
@@ -593,10 +689,39 @@ cr_flux_kernel(const double* __restrict__ U, double* __restrict__ H, const doubl
       uR[v] = q[(3 * NV + v) * ntrans];
       if (src_dir) SI[v] = 0.5 * (q[(4 * NV + v) * ntrans] + q[(5 * NV + v) * ntrans]);
     }
-    Eig Ecc;
-    if (CC) Ecc = roe_eig<M, DIR>(axL.rs, axR.rs, pp);
+    // The dissipation in float pairs where it is small against the flux (the rule of
+    // gbh_pair_flux.cuh), else the FP64 upwinding.
     double fI[NV];
-    upwind_iface<M, false, UPW, DIR>(fL, fR, uL, uR, Ecc, axL, axR, pp, fI, GRAV ? fmax(gL, gR) : 1.0);
+    bool ok = false;
+    if constexpr (UPW != UPW_SWFS) {
+      const ff six = {6.0f, 0.0f}, zero = {0.0f, 0.0f};
+      ff fs6[NV], fd6[NV], ud6[NV], um[NV], g12[NV];
+      float lam, rho, Hs;
+#pragma unroll
+      for (int v = 0; v < NV; v++) {
+        fs6[v] = zero;
+        fd6[v] = UPW == UPW_RF ? six * to_pair(fR[v] - fL[v]) : zero;
+        ud6[v] = six * to_pair(uR[v] - uL[v]);
+        um[v] = STATES ? to_pair(0.5 * (uL[v] + uR[v])) : zero;
+      }
+      const PCell<M> cl = pair_cell<M, UPW>(axL), cr = pair_cell<M, UPW>(axR);
+      PEig E;
+      if (CC) E = peig<M, DIR>(cl, cr, P);
+      const ff kap = GRAV ? to_pair(fmax(gL, gR)) : zero;
+      pupwind<M, UPW, DIR>(fs6, fd6, ud6, um, E, cl, cr, P, g12, lam, rho, Hs, GRAV ? &kap : nullptr);
+      const float s0 = rho * lam, sm = s0 * lam, sE = s0 * Hs;
+      ok = (s0 >= 8.7e-19f) & (s0 <= 1.2e30f) & (sm >= 8.7e-19f) & (sm <= 1.2e30f) & (sE >= 8.7e-19f) & (sE <= 1.2e30f);
+#pragma unroll
+      for (int v = 0; v < NV; v++) {
+        ok = ok & (ffma(lam, fabsf(ud6[v].h), fabsf(fd6[v].h)) <= 0.09375f * (v == 0 ? s0 : (v == NV - 1 ? sE : sm)));
+        fI[v] = fma(0.5, fL[v] + fR[v], to_double(ffc(1.0 / 12.0) * g12[v]));
+      }
+    }
+    if (!ok) {
+      Eig Ecc;
+      if (CC) Ecc = roe_eig<M, DIR>(axL.rs, axR.rs, pp);
+      upwind_iface<M, false, UPW, DIR>(fL, fR, uL, uR, Ecc, axL, axR, pp, fI, GRAV ? fmax(gL, gR) : 1.0);
+    }
     boundary_flux<NV>(ep, I, N, line, ntrans, fI);
     if (I > I0) {
       const int c = I - 1;

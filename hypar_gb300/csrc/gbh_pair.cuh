@@ -165,6 +165,14 @@ GBH_HD ff to_pair(double x) {
   r.l = fmul(fmul(u32tof(L & 0x1fffffffu), 1.862645149230957e-9f), s);
   return r;
 }
+// The magnitude of a double as a float, rounded down (0 below 2^-126, infinity for what is
+// too large or not finite).
+GBH_HD float d2f_mag(double x) {
+  const uint32_t H = dhi(x) & 0x7fffffffu;
+  const int32_t e = (int32_t)(H & 0x7ff00000u) - (896 << 20);
+  const uint32_t m = shl64hi(H, dlo(x), 3) & 0x7fffffu;
+  return e <= 0 ? 0.0f : (e >= (255 << 20) ? u2f(0x7f800000u) : u2f(((uint32_t)e << 3) | m));
+}
 GBH_HD double f2d(float a) {
   const uint32_t b = f2u(a);
   const uint32_t hi = (((b >> 3) & 0x0fffffffu) + 0x38000000u) | (b & 0x80000000u);
@@ -237,20 +245,21 @@ struct PRow {
 };
 GBH_HD ff inv_sq(ff B) { return sqr(rcp(B)); }
 
-template <bool ALTW>
+// SIX: with the factor 6 (the optimal weights' ratio) in c.
+template <bool ALTW, bool SIX = true>
 GBH_HD PRow weno_row(ff dm, ff dp, ff eps4, bool none) {
   PRow o;
   o.d = dp - dm;
   if (ALTW && none) {
     o.l = o.r = o.bl = o.br = ff{1.0f, 0.0f};
-    o.c = ff{6.0f, 0.0f};
+    o.c = ff{SIX ? 6.0f : 1.0f, 0.0f};
     return o;
   }
   const ff s = dp + dm, d2 = mul2(o.d, 2.0f);
   const ff base = addu(ffc(13.0 / 3.0) * sqr(o.d), eps4);
   const ff Bl = addu(base, sqr(s + d2)), Bc = addu(base, sqr(s)), Br = addu(base, sqr(s - d2));
   o.l = inv_sq(Bl);
-  o.c = mulf(inv_sq(Bc), 6.0f);
+  o.c = SIX ? mulf(inv_sq(Bc), 6.0f) : inv_sq(Bc);
   o.r = inv_sq(Br);
   if (ALTW) {
     o.bl = Bl;
