@@ -281,8 +281,10 @@ cr_solve_kernel(const double* __restrict__ U, const double* __restrict__ F, DevG
 #pragma unroll
     for (int p = 0; p < 5; p++) sv[p] = left ? wval[p] : wval[5 - p];
     const bool bnd = (I == 0) || (I == N);
-    // Weights in pairs: an error e of a weight moves the interface value by about e/20 of
-    // the stencil's third differences; where those exceed 1/16 of its values (or the pairs'
+    // Weights in pairs: an error e of a weight moves the interface value by the residual of
+    // a sub-stencil's compact relation, about a twentieth of the stencil's third
+    // differences, times e / 3, i.e. by 2^-46 / 60 of them; where those exceed half of its
+    // values (or the pairs'
     // range is left, or something is not finite), and for gravity's source function, whose
     // values are not the weights', the weights are formed in FP64.
     double w1, w2, w3;
@@ -299,7 +301,7 @@ cr_solve_kernel(const double* __restrict__ U, const double* __restrict__ F, DevG
       float m = 0.0f;
 #pragma unroll
       for (int p = 0; p < 6; p++) m = fmaxf(m, d2f_mag(wval[p]));
-      ok = ok & (fadd(fabsf(t1.h), fabsf(t2.h)) <= 0.0625f * m) & (m >= 8.7e-19f) & (m <= 1.2e30f) & !(GRAV && k >= 4);
+      ok = ok & (fadd(fabsf(t1.h), fabsf(t2.h)) <= 0.5f * m) & (m >= 8.7e-19f) & (m <= 1.2e30f) & !(GRAV && k >= 4);
       w1 = to_double(p1);
       w2 = to_double(p2);
       w3 = to_double(p3);
@@ -779,7 +781,11 @@ static cudaError_t cr_dir(bool chr, const double* U, double* H, const double* dx
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  const int seg = L.seg > 0 ? L.seg : 32;
+  int seg = L.seg > 0 ? L.seg : 32;
+  // The back half walks short segments: 16 warps per SM hide the latency of its reads
+  // (64^3: two segments of 32 per line left 256 warps in all, 117 / 162 / 247 us).
+  const long long fill = G.dim[DIR] * ntrans / (152LL * 16 * 32);
+  if (seg > fill) seg = fill < 2 ? 2 : (int)fill;
   const int nseg = (G.dim[DIR] + seg - 1) / seg;
   const long long nthr = ntrans * nseg;
   const int block = L.block > 0 ? L.block : 128;

@@ -98,8 +98,9 @@ static void rebuild_table(gb_ensemble* e) {
       for (int k = 0; k < e->base.ndims; k++)
         if (k != d) ntr *= md.G.dim[k];
       md.ntrans[d] = ntr;
-      const int cap = pair_cap_of(e->seg[d], e->block[d]);
-      const PairPlan p = pair_plan(md.G.dim[d], ntr, d, cap > 0 ? cap : pair_cap(cells));
+      int cap = pair_cap_of(e->seg[d], e->block[d]);
+      if (cap <= 0) cap = pair_cap(cells);
+      const PairPlan p = pair_plan(md.G.dim[d], ntr, d, cap, true);
       md.L[d] = p.L;
       md.XL[d] = p.XL;
       if (p.T > e->threads[d]) e->threads[d] = p.T;

@@ -13,7 +13,8 @@ struct PairPlan {
 // of a line and to the last block of lines; along the strided directions fewer than four
 // neighbouring lines read less than a 128-byte line of memory at a time, which is weighed
 // as an eighth more.
-inline PairPlan pair_plan(int N, long long nlines, int dir, int cap) {
+// fixed: every block of the launch has `cap` threads (ensembles), so blocks are counted.
+inline PairPlan pair_plan(int N, long long nlines, int dir, int cap, bool fixed = false) {
   PairPlan best = {1, 1, 32};
   double cost = 1e300;
   for (int XL = 1; XL <= 16 && XL <= nlines; XL++) {
@@ -23,7 +24,7 @@ inline PairPlan pair_plan(int N, long long nlines, int dir, int cap) {
     for (int n = n0; n < n0 + 3; n++) {
       const int L = (N + n - 1) / n, nt = (N + L - 1) / L;
       const int T = (XL * (L + 6) + 31) / 32 * 32;
-      double c = (double)((nlines + XL - 1) / XL) * nt * T;
+      double c = (double)((nlines + XL - 1) / XL) * nt * (fixed ? cap : T);
       if (dir > 0 && XL < 4) c *= 1.125;
       if (c < cost) {
         cost = c;

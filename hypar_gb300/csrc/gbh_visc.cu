@@ -6,12 +6,26 @@
 // FirstDerivativeFourthOrderCentral (src/FirstDerivative/FirstDerivativeFourthOrder.c:36-129),
 // including its single-rank behaviour: a derivative along d is formed only on
 // lines whose other indices are interior, so at a ghost point the derivatives
-// across the ghost direction are zero.  Three passes:
-//   visc_q      : Q = (rho, u, v, w, T = gamma P / rho) and mu = T^0.76 at every point
-//   visc_grad   : dQ/dx_d * dxinv_d for the velocity and temperature, with the rule above
-//   visc_dir<d> : viscous flux along d on each line (window of five points) and
-//                 par += dxinv_d * d/dx_d (flux) at interior points.
+// across the ghost direction are zero.  Three passes over arrays of one component each
+// (consecutive threads, consecutive addresses):
+//   visc_q    : velocity, T = gamma P / rho and mu = T^0.76 at every point
+//   visc_flux : the scaled derivatives of velocity and temperature, with the rule above,
+//               and from them the stress tensor (6) and the energy fluxes (3)
+//   visc_div  : par = sum over d of dxinv_d d/dx_d (flux along d) at interior points.
+//
+// All three are bound by arithmetic, the FP64 pipe above all (2 operations per clock and
+// SM), so the passes share what the three directions have in common (162 FP64 operations
+// per point against the 310 of one flux pass per direction) and, where the viscous flux is
+// small against the convective one, work in pairs of FP32 numbers (gbh_pair.cuh): the
+// derivatives of the velocity, the stresses, the energy flux and their divergence.
+// Velocities hold 48 bits as pairs, so their derivatives are off by 2^-50 |v| / h and the
+// stress by 2^-50 mu |v| / (Re h); where mu / (Re h) is at most rho a / 32 at every point
+// that is below a quarter of the rounding of the convective flux (rho a^2) it is added to.
+// visc_q checks this, and any point that fails (or leaves the pairs' range, or is not
+// finite) turns the whole evaluation to FP64.  Temperature derivatives stay in FP64.
+// 256^3: 8.30 -> 1.65 ms per evaluation.
 #include "gbh_internal.h"
+#include "gbh_pair.cuh"
 
 namespace gbh {
 
@@ -22,12 +36,33 @@ __device__ __forceinline__ int fold1(int i, int N, int lo, int hi) {
 }
 
 
-// Q (5) and mu at all points including ghosts; ghost points read through the fold.
-__global__ void visc_q_kernel(const double* __restrict__ u, double* __restrict__ Q, DevGeom G, ViscParams vp) {
-  long long n = (long long)(G.dim[0] + 2 * G.g) * (G.dim[1] + 2 * G.g) * (G.dim[2] + 2 * G.g);
+// T^0.76 (raiseto, include/math_ops.h:37).  y = T^(19/25) from an FP32 estimate y0 and
+// z = y0^25 / T^19: y = y0 z^(-1/25) = y0 (1 + e/25 + 13 e^2/625 + ...), e = 1 - z.  The
+// estimate's error of some 1e-6 leaves 1e-17 after these terms, and the rounding of z
+// (some ten units) counts a 25th: 20 FP64 operations against about 90 of exp(0.76 log T),
+// at its accuracy.
+__device__ __forceinline__ double pow076(double T) {
+  const float t = d2f_mag(T);
+  if (!(T > 0.0) || !(t > 1e-8f) || !(t < 1e8f)) return exp(0.76 * log(T));
+  const double y = (double)exp2f(0.76f * log2f(t)), r = nr_rcp(T);
+  const double y2 = y * y, y4 = y2 * y2, y8 = y4 * y4, y16 = y8 * y8;
+  const double r2 = r * r, r4 = r2 * r2, r8 = r4 * r4, r16 = r8 * r8;
+  const double e = fma(-((y16 * y8) * y), (r16 * r2) * r, 1.0);
+  return fma(y * e, fma(13.0 / 625.0, e, 0.04), y);
+}
+
+// Arrays of one component each, n points: doubles u, v, w, T, mu, then pairs u, v, w, mu.
+enum { VQ_T = 3, VQ_MU = 4, VQ_PAIR = 5 };
+
+// At all points including ghosts; ghost points read through the fold.  *flag takes `id`
+// where the pairs' bound fails.
+__global__ void __launch_bounds__(256)
+visc_q_kernel(const double* __restrict__ u, double* __restrict__ Q, const double* __restrict__ dxinv, DevGeom G,
+              ViscParams vp, int* __restrict__ flag, int id) {
+  const int ng0 = G.dim[0] + 2 * G.g, ng1 = G.dim[1] + 2 * G.g, ng2 = G.dim[2] + 2 * G.g;
+  const long long n = (long long)ng0 * ng1 * ng2;
   long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n) return;
-  int ng0 = G.dim[0] + 2 * G.g, ng1 = G.dim[1] + 2 * G.g;
   int i = (int)(p % ng0) - G.g;
   int j = (int)((p / ng0) % ng1) - G.g;
   int k = (int)(p / ((long long)ng0 * ng1)) - G.g;
@@ -39,19 +74,33 @@ __global__ void visc_q_kernel(const double* __restrict__ u, double* __restrict__
   const double* uu = u + q * 5;
   double rho = uu[0];
   double ri = nr_rcp(rho);
-  double vx = rho == 0.0 ? 0.0 : uu[1] * ri;
-  double vy = rho == 0.0 ? 0.0 : uu[2] * ri;
-  double vz = rho == 0.0 ? 0.0 : uu[3] * ri;
-  double vsq = vx * vx + vy * vy + vz * vz;
+  double v[3];
+#pragma unroll
+  for (int d = 0; d < 3; d++) v[d] = rho == 0.0 ? 0.0 : uu[1 + d] * ri;
+  double vsq = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
   double P = (uu[4] - 0.5 * rho * vsq) * vp.gm1;
   double T = vp.gamma * P * ri;
-  double* out = Q + p * 6;
-  out[0] = rho;
-  out[1] = vx;
-  out[2] = vy;
-  out[3] = vz;
-  out[4] = T;
-  out[5] = exp(0.76 * log(T));  // raiseto(T, 0.76), include/math_ops.h:37
+  const double mu = pow076(T);
+#pragma unroll
+  for (int d = 0; d < 3; d++) Q[d * n + p] = v[d];
+  Q[VQ_T * n + p] = T;
+  Q[VQ_MU * n + p] = mu;
+  if (!flag) return;
+  ff* R = (ff*)(Q + VQ_PAIR * n);
+  const ff pm = to_pair(mu);
+  float vm = 0.0f;
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    const ff pv = to_pair(v[d]);
+    R[d * n + p] = pv;
+    vm = fadd(vm, fabsf(pv.h));
+  }
+  R[3 * n + p] = pm;
+  const float h = fmaxf(d2f_mag(dxinv[G.g + i]), fmaxf(d2f_mag(dxinv[ng0 + G.g + j]), d2f_mag(dxinv[ng0 + ng1 + G.g + k])));
+  const float t = d2f_mag(T), r = d2f_mag(rho);
+  const bool ok = (T > 0.0) & (pm.h * (float)vp.inv_Re * h <= 0.03125f * r * sqrtf(t)) & (t >= 1e-18f) & (t <= 1e18f) &
+                  (r >= 1e-18f) & (vm <= 1e18f) & (h <= 1e18f);
+  if (!ok) *flag = id;
 }
 
 // Fourth-order first derivative of one Q component at position i of a line of
@@ -78,144 +127,171 @@ __device__ __forceinline__ double d1(int i, int N, int g, int bias, F f) {
                     : __dsub_rn(__dadd_rn(__dmul_rn(0.0, f(1)), f(0)), f(-1));
 }
 
-// Scaled gradients of (u, v, w, T): Gr[p*12 + d*4 + c].
-__global__ void visc_grad_kernel(const double* __restrict__ Q, double* __restrict__ Gr, const double* __restrict__ dxinv,
-                                 DevGeom G, int order) {
-  int ng[3] = {G.dim[0] + 2 * G.g, G.dim[1] + 2 * G.g, G.dim[2] + 2 * G.g};
-  long long n = (long long)ng[0] * ng[1] * ng[2];
-  long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  int idx[3];
-  idx[0] = (int)(p % ng[0]) - G.g;
-  idx[1] = (int)((p / ng[0]) % ng[1]) - G.g;
-  idx[2] = (int)(p / ((long long)ng[0] * ng[1])) - G.g;
-  int off = 0;
-  for (int d = 0; d < 3; d++) {
-    bool line = true;
-    for (int e = 0; e < 3; e++)
-      if (e != d && (idx[e] < 0 || idx[e] >= G.dim[e])) line = false;
-    double* out = Gr + p * 12 + d * 4;
-    if (!line) {
-      out[0] = out[1] = out[2] = out[3] = 0.0;
-    } else {
-      long long sd = G.stride[d];
-      double di = dxinv[off + G.g + idx[d]];
-      for (int c = 0; c < 4; c++) {
-        const double* base = Q + p * 6 + 1 + c;
-        auto fk = [&](int k) { return base[(long long)k * sd * 6]; };
-        double v = order == 2 ? d1(idx[d], G.dim[d], G.g, 1, fk) : d4(idx[d], G.dim[d], G.g, fk);
-        out[c] = v * di;
+// The numbers the passes work in.
+__device__ __forceinline__ double vadd(double a, double b) { return a + b; }
+__device__ __forceinline__ double vsub(double a, double b) { return a - b; }
+__device__ __forceinline__ double vmul(double a, double b) { return a * b; }
+__device__ __forceinline__ double vtwo(double a) { return 2.0 * a; }
+__device__ __forceinline__ double veight(double a, double b) { return fma(8.0, a, b); }  // 8 a + b
+__device__ __forceinline__ double vdot(double a, double x, double b, double y, double c, double z, double q) {
+  return fma(a, x, fma(b, y, fma(c, z, q)));
+}
+__device__ __forceinline__ ff vadd(ff a, ff b) { return a + b; }
+__device__ __forceinline__ ff vsub(ff a, ff b) { return a - b; }
+__device__ __forceinline__ ff vmul(ff a, ff b) { return a * b; }
+__device__ __forceinline__ ff vtwo(ff a) { return mul2(a, 2.0f); }
+__device__ __forceinline__ ff veight(ff a, ff b) { return mul2(a, 8.0f) + b; }
+__device__ __forceinline__ ff vdot(ff a, ff x, ff b, ff y, ff c, ff z, ff q) {
+  FAcc s = acc_mul(a, x);
+  acc_fma(s, b, y);
+  acc_fma(s, c, z);
+  acc_add(s, q);
+  return acc_get(s);
+}
+template <class T> __device__ __forceinline__ T vnum(double x);
+template <> __device__ __forceinline__ double vnum<double>(double x) { return x; }
+template <> __device__ __forceinline__ ff vnum<ff>(double x) { return to_pair(x); }
+__device__ __forceinline__ double vout(double x) { return x; }
+__device__ __forceinline__ double vout(ff x) { return to_double(x); }
+
+// The stress tensor (xx, yy, zz, xy, xz, yz) and energy fluxes (x, y, z) at one point
+// (NavierStokes3DParabolicFunction.c:151-314) from the derivatives along the lines whose
+// other indices are interior (on[e]; the rest are zero).
+template <class T>
+__device__ __forceinline__ void visc_flux_at(const double* __restrict__ Q, double* __restrict__ F, const DevGeom& G,
+                                             const ViscParams& vp, const double* di, long long n, long long p,
+                                             const int* idx, const bool* on) {
+  const T* V = (const T*)(sizeof(T) == sizeof(double) && __is_same(T, double) ? Q : Q + VQ_PAIR * n);
+  const T* MU = __is_same(T, double) ? (const T*)(Q + VQ_MU * n) : V + 3 * n;
+  const double* TT = Q + VQ_T * n;
+  T D[3][3], H[3];  // D[e][c] = d v_c / dx_e, H[e] = dT/dx_e
+#pragma unroll
+  for (int e = 0; e < 3; e++) {
+    const long long sd = G.stride[e];
+    const int i = idx[e], N = G.dim[e];
+    if (!on[e]) {
+#pragma unroll
+      for (int c = 0; c < 3; c++) D[e][c] = vnum<T>(0.0);
+      H[e] = vnum<T>(0.0);
+      continue;
+    }
+    const bool central = vp.order != 2 && i > -G.g + 1 && i < N + G.g - 2;
+    const double d12 = di[e] * (1.0 / 12.0);
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const T* f = V + c * n + p;
+      if (central) {
+        D[e][c] = vmul(veight(vsub(f[sd], f[-sd]), vsub(f[-2 * sd], f[2 * sd])), vnum<T>(d12));
+      } else {  // the ends of the ghost-extended line (and the first-order scheme): FP64
+        const double* b = Q + c * n + p;
+        auto fk = [&](int k) { return b[k * sd]; };
+        D[e][c] = vnum<T>((vp.order == 2 ? d1(i, N, G.g, 1, fk) : d4(i, N, G.g, fk)) * di[e]);
       }
     }
-    off += ng[d];
+    const double* b = TT + p;
+    auto fk = [&](int k) { return b[k * sd]; };
+    if (central) H[e] = vnum<T>(fma(8.0, b[sd] - b[-sd], b[-2 * sd] - b[2 * sd]) * d12);
+    else H[e] = vnum<T>((vp.order == 2 ? d1(i, N, G.g, 1, fk) : d4(i, N, G.g, fk)) * di[e]);
   }
+  const T mr = vmul(MU[p], vnum<T>(vp.inv_Re)), kq = vmul(mr, vnum<T>(vp.inv_gm1 * vp.inv_Pr));
+  const T third = vmul(vadd(vadd(D[0][0], D[1][1]), D[2][2]), vnum<T>(2.0 / 3.0));
+  T s[6];
+#pragma unroll
+  for (int d = 0; d < 3; d++) s[d] = vmul(mr, vsub(vtwo(D[d][d]), third));
+  s[3] = vmul(mr, vadd(D[1][0], D[0][1]));
+  s[4] = vmul(mr, vadd(D[2][0], D[0][2]));
+  s[5] = vmul(mr, vadd(D[2][1], D[1][2]));
+  const T a = V[p], b = V[n + p], c = V[2 * n + p];
+  T* out = (T*)F + p;
+#pragma unroll
+  for (int k = 0; k < 6; k++) out[k * n] = s[k];
+  out[6 * n] = vdot(a, s[0], b, s[3], c, s[4], vmul(kq, H[0]));
+  out[7 * n] = vdot(a, s[3], b, s[1], c, s[5], vmul(kq, H[1]));
+  out[8 * n] = vdot(a, s[4], b, s[5], c, s[2], vmul(kq, H[2]));
 }
 
-// Viscous flux along DIR at one point (NavierStokes3DParabolicFunction.c:151-314).
-template <int DIR>
-__device__ __forceinline__ void visc_flux(const double* Qp, const double* Gp, const ViscParams& vp, double* F) {
-  const double two_third = 2.0 / 3.0;
-  double uvel = Qp[1], vvel = Qp[2], wvel = Qp[3], mu = Qp[5];
-  double mr = mu * vp.inv_Re;
-  double kq = mr * vp.inv_gm1 * vp.inv_Pr;
-  const double* X = Gp;      // d/dx of (u, v, w, T)
-  const double* Y = Gp + 4;  // d/dy
-  const double* Z = Gp + 8;  // d/dz
-  double t1, t2, t3, q;
-  if (DIR == 0) {
-    t1 = two_third * mr * (2.0 * X[0] - Y[1] - Z[2]);
-    t2 = mr * (Y[0] + X[1]);
-    t3 = mr * (Z[0] + X[2]);
-    q = kq * X[3];
-  } else if (DIR == 1) {
-    t1 = mr * (Y[0] + X[1]);
-    t2 = two_third * mr * (-X[0] + 2.0 * Y[1] - Z[2]);
-    t3 = mr * (Z[1] + Y[2]);
-    q = kq * Y[3];
-  } else {
-    t1 = mr * (Z[0] + X[2]);
-    t2 = mr * (Z[1] + Y[2]);
-    t3 = two_third * mr * (-X[0] - Y[1] + 2.0 * Z[2]);
-    q = kq * Z[3];
-  }
-  F[0] = t1;
-  F[1] = t2;
-  F[2] = t3;
-  F[3] = uvel * t1 + vvel * t2 + wvel * t3 + q;
-}
-
-// One thread per (interior line along DIR, segment of `seg` interior points).
-template <int DIR>
-__global__ void visc_dir_kernel(const double* __restrict__ Q, const double* __restrict__ Gr,
-                                const double* __restrict__ dxinv_dir, double* __restrict__ par, DevGeom G,
-                                ViscParams vp, int seg, int nseg, int first) {
-  long long ntrans = 1;
-  for (int e = 0; e < 3; e++)
-    if (e != DIR) ntrans *= G.dim[e];
-  long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (tid >= ntrans * nseg) return;
-  long long tr = tid % ntrans;
-  int sg = (int)(tid / ntrans);
-  long long pb = (long long)G.g * G.stride[DIR];
+// Points off the interior in one direction carry the flux along it only, two deep.
+__global__ void __launch_bounds__(256)
+visc_flux_kernel(const double* __restrict__ Q, double* __restrict__ F, const double* __restrict__ dxinv, DevGeom G,
+                 ViscParams vp, const int* __restrict__ flag, int id) {
+  const int ng[3] = {G.dim[0] + 2 * G.g, G.dim[1] + 2 * G.g, G.dim[2] + 2 * G.g};
+  const long long n = (long long)ng[0] * ng[1] * ng[2];
+  const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= n) return;
+  const int idx[3] = {(int)(p % ng[0]) - G.g, (int)((p / ng[0]) % ng[1]) - G.g,
+                      (int)(p / ((long long)ng[0] * ng[1])) - G.g};
+  int outside = 0;
+  bool reach = true, in[3];
+#pragma unroll
   for (int e = 0; e < 3; e++) {
-    if (e == DIR) continue;
-    int ie = (int)(tr % G.dim[e]);
-    tr /= G.dim[e];
-    pb += (long long)(ie + G.g) * G.stride[e];
+    in[e] = idx[e] >= 0 && idx[e] < G.dim[e];
+    outside += !in[e];
+    reach = reach && idx[e] >= -2 && idx[e] < G.dim[e] + 2;
   }
-  const long long sd = G.stride[DIR];
-  const int N = G.dim[DIR];
-  const int c0 = sg * seg, c1 = min(c0 + seg, N);
-  const double one_twelve = 1.0 / 12.0;
-  double W[5][4];
-  auto flux_at = [&](int i, double* F) {
-    long long p = pb + (long long)i * sd;
-    visc_flux<DIR>(Q + p * 6, Gr + p * 12, vp, F);
-  };
+  if (outside > 1 || !reach) return;
+  const bool on[3] = {in[1] && in[2], in[0] && in[2], in[0] && in[1]};
+  const double di[3] = {dxinv[G.g + idx[0]], dxinv[ng[0] + G.g + idx[1]], dxinv[ng[0] + ng[1] + G.g + idx[2]]};
+  if (flag && *flag != id) visc_flux_at<ff>(Q, F, G, vp, di, n, p, idx, on);
+  else visc_flux_at<double>(Q, F, G, vp, di, n, p, idx, on);
+}
+
+template <class T>
+__device__ __forceinline__ void visc_div_at(const double* __restrict__ F0, double* out, const DevGeom& G,
+                                            const ViscParams& vp, const double* di, long long n, long long p) {
+  const T* F = (const T*)F0 + p;
+  const int comp[3][4] = {{0, 3, 4, 6}, {3, 1, 5, 7}, {4, 5, 2, 8}};
 #pragma unroll
-  for (int k = 0; k < 4; k++) flux_at(c0 - 2 + k, W[k + 1]);
-  for (int c = c0; c < c1; c++) {
+  for (int v = 0; v < 4; v++) {
+    T sum = vnum<T>(0.0);
 #pragma unroll
-    for (int k = 0; k < 4; k++)
-#pragma unroll
-      for (int v = 0; v < 4; v++) W[k][v] = W[k + 1][v];
-    flux_at(c + 2, W[4]);
-    long long p = pb + (long long)c * sd;
-    double di = dxinv_dir[G.g + c];
-    double* out = par + p * 5;
-    if (first) out[0] = 0.0;
-#pragma unroll
-    for (int v = 0; v < 4; v++) {
+    for (int d = 0; d < 3; d++) {
+      const T* f = F + comp[d][v] * n;
+      const long long sd = G.stride[d];
+      T term;
       // interior points: the central fourth-order difference, or the backward
       // first-order one of the second-order scheme
-      double fd = vp.order == 2 ? __dsub_rn(__dadd_rn(__dmul_rn(0.0, W[3][v]), W[2][v]), W[1][v])
-                                : (W[0][v] - 8.0 * W[1][v] + 8.0 * W[3][v] - W[4][v]) * one_twelve;
-      double val = di * fd;
-      out[1 + v] = first ? val : out[1 + v] + val;
+      if (__is_same(T, double) && vp.order == 2) {
+        const double* b = (const double*)f;
+        term = vnum<T>(di[d] * __dsub_rn(__dadd_rn(__dmul_rn(0.0, b[sd]), b[0]), b[-sd]));
+      } else {
+        term = vmul(veight(vsub(f[sd], f[-sd]), vsub(f[-2 * sd], f[2 * sd])), vnum<T>(di[d] * (1.0 / 12.0)));
+      }
+      sum = d == 0 ? term : vadd(sum, term);
     }
+    out[1 + v] = vout(sum);
   }
 }
 
-cudaError_t launch_visc(const double* u, double* Q, double* Gr, double* par, const double* dxinv, const DevGeom& G,
-                        const ViscParams& vp, int seg, cudaStream_t s) {
-  long long n = (long long)(G.dim[0] + 2 * G.g) * (G.dim[1] + 2 * G.g) * (G.dim[2] + 2 * G.g);
-  int blk = 256;
-  visc_q_kernel<<<(unsigned)((n + blk - 1) / blk), blk, 0, s>>>(u, Q, G, vp);
-  visc_grad_kernel<<<(unsigned)((n + blk - 1) / blk), blk, 0, s>>>(Q, Gr, dxinv, G, vp.order);
-  int off = 0;
-  for (int d = 0; d < 3; d++) {
-    long long ntrans = 1;
-    for (int e = 0; e < 3; e++)
-      if (e != d) ntrans *= G.dim[e];
-    int nseg = (G.dim[d] + seg - 1) / seg;
-    long long nthr = ntrans * nseg;
-    unsigned grid = (unsigned)((nthr + 127) / 128);
-    const double* dxd = dxinv + off;
-    if (d == 0) visc_dir_kernel<0><<<grid, 128, 0, s>>>(Q, Gr, dxd, par, G, vp, seg, nseg, 1);
-    if (d == 1) visc_dir_kernel<1><<<grid, 128, 0, s>>>(Q, Gr, dxd, par, G, vp, seg, nseg, 0);
-    if (d == 2) visc_dir_kernel<2><<<grid, 128, 0, s>>>(Q, Gr, dxd, par, G, vp, seg, nseg, 0);
-    off += G.dim[d] + 2 * G.g;
-  }
+__global__ void __launch_bounds__(256)
+visc_div_kernel(const double* __restrict__ F, double* __restrict__ par, const double* __restrict__ dxinv, DevGeom G,
+                ViscParams vp, const int* __restrict__ flag, int id) {
+  const long long m = (long long)G.dim[0] * G.dim[1] * G.dim[2];
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= m) return;
+  const int i = (int)(t % G.dim[0]), j = (int)((t / G.dim[0]) % G.dim[1]), k = (int)(t / ((long long)G.dim[0] * G.dim[1]));
+  const int ng0 = G.dim[0] + 2 * G.g, ng1 = G.dim[1] + 2 * G.g, ng2 = G.dim[2] + 2 * G.g;
+  const long long n = (long long)ng0 * ng1 * ng2;
+  const long long p = (long long)(i + G.g) * G.stride[0] + (long long)(j + G.g) * G.stride[1] +
+                      (long long)(k + G.g) * G.stride[2];
+  const double di[3] = {dxinv[G.g + i], dxinv[ng0 + G.g + j], dxinv[ng0 + ng1 + G.g + k]};
+  double out[5];
+  out[0] = 0.0;
+  if (flag && *flag != id) visc_div_at<ff>(F, out, G, vp, di, n, p);
+  else visc_div_at<double>(F, out, G, vp, di, n, p);
+#pragma unroll
+  for (int v = 0; v < 5; v++) par[p * 5 + v] = out[v];
+}
+
+// flag, id: where the pairs may be used, a device integer and a value it does not hold
+// yet (visc_q stores it there to refuse them); nullptr: FP64 throughout.
+cudaError_t launch_visc(const double* u, double* Q, double* F, double* par, const double* dxinv, const DevGeom& G,
+                        const ViscParams& vp, int* flag, int id, cudaStream_t s) {
+  const long long n = (long long)(G.dim[0] + 2 * G.g) * (G.dim[1] + 2 * G.g) * (G.dim[2] + 2 * G.g);
+  const long long m = (long long)G.dim[0] * G.dim[1] * G.dim[2];
+  if (vp.order == 2) flag = nullptr;
+  visc_q_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(u, Q, dxinv, G, vp, flag, id);
+  visc_flux_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(Q, F, dxinv, G, vp, flag, id);
+  visc_div_kernel<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(F, par, dxinv, G, vp, flag, id);
   return cudaGetLastError();
 }
 

@@ -89,3 +89,11 @@ def test_weights_with_jumps(built_lib, oracle_lib, tmp_path, interp, weights):
 def test_units(built_lib, oracle_lib, tmp_path, model, unit):
     """Densities and pressures far from 1: the pairs' range check hands over to FP64."""
     check(build_case(model, "components", "roe", jump=True, unit=unit), tmp_path)
+
+
+@pytest.mark.parametrize("Re", [0.5, 20.0, 1600.0])
+def test_viscous_regimes(built_lib, oracle_lib, tmp_path, Re):
+    """Viscous fluxes from dominant (FP64 throughout) to small (pairs) against the convective ones."""
+    case = C.tgv(12, n_iter=1, dt=1e-3, perturb=0.05)
+    case.Re = Re
+    check(case, tmp_path)
