@@ -199,6 +199,49 @@ GBH_HD ff addu(ff a, ff b) {
   return s;
 }
 
+// Products and squares not normalised (|l| up to some 2^-22 of h), for sums of positive
+// terms, reciprocals and sums of products; l l is kept where an operand may be unnormalised.
+GBH_HD ff mulu(ff a, ff b) {
+  ff r;
+  r.h = fmul(a.h, b.h);
+  r.l = ffma(a.l, b.h, ffma(a.h, b.l, ffma(a.h, b.h, -r.h)));
+  return r;
+}
+// (both operands unnormalised)
+GBH_HD ff muluu(ff a, ff b) {
+  ff r;
+  r.h = fmul(a.h, b.h);
+  r.l = ffma(a.l, b.l, ffma(a.l, b.h, ffma(a.h, b.l, ffma(a.h, b.h, -r.h))));
+  return r;
+}
+GBH_HD ff mulfu(ff a, float b) {
+  ff r;
+  r.h = fmul(a.h, b);
+  r.l = ffma(a.l, b, ffma(a.h, b, -r.h));
+  return r;
+}
+GBH_HD ff sqru(ff a) {
+  ff r;
+  r.h = fmul(a.h, a.h);
+  r.l = ffma(fadd(a.h, a.h), a.l, ffma(a.h, a.h, -r.h));
+  return r;
+}
+// 1 / x not normalised, and 1 / x^2.
+GBH_HD ff rcpu(ff x) {
+  ff r;
+  r.h = rcp32(x.h);
+  const float e = ffma(-x.l, r.h, ffma(-x.h, r.h, 1.0f));
+  r.l = fmul(r.h, ffma(e, e, e));
+  return r;
+}
+GBH_HD ff inv_sq(ff x) {
+  const ff y = rcpu(x);
+  ff r;
+  r.h = fmul(y.h, y.h);
+  r.l = ffma(y.l, y.l, ffma(fadd(y.h, y.h), y.l, ffma(y.h, y.h, -r.h)));
+  return r;
+}
+
 // A sum of products of pairs: the leading products are added without error, the rest
 // collects in the second word.
 struct FAcc {
@@ -243,8 +286,6 @@ GBH_HD ff acc_get(FAcc c) { return fast2(c.h, c.l); }
 struct PRow {
   ff d, l, c, r, bl, br;
 };
-GBH_HD ff inv_sq(ff B) { return sqr(rcp(B)); }
-
 // SIX: with the factor 6 (the optimal weights' ratio) in c.
 template <bool ALTW, bool SIX = true>
 GBH_HD PRow weno_row(ff dm, ff dp, ff eps4, bool none) {
@@ -255,11 +296,12 @@ GBH_HD PRow weno_row(ff dm, ff dp, ff eps4, bool none) {
     o.c = ff{SIX ? 6.0f : 1.0f, 0.0f};
     return o;
   }
-  const ff s = dp + dm, d2 = mul2(o.d, 2.0f);
-  const ff base = addu(ffc(13.0 / 3.0) * sqr(o.d), eps4);
-  const ff Bl = addu(base, sqr(s + d2)), Bc = addu(base, sqr(s)), Br = addu(base, sqr(s - d2));
+  // 3 dp - dm, dp + dm and 3 dm - dp: the first differences of weno5_cell_q
+  const ff base = addu(mulu(ffc(13.0 / 3.0), sqr(o.d)), eps4);
+  const ff Bl = addu(base, sqru(o.d + mul2(dp, 2.0f))), Bc = addu(base, sqru(dp + dm)),
+           Br = addu(base, sqru(mul2(dm, 2.0f) - o.d));
   o.l = inv_sq(Bl);
-  o.c = SIX ? mulf(inv_sq(Bc), 6.0f) : inv_sq(Bc);
+  o.c = SIX ? mulfu(inv_sq(Bc), 6.0f) : inv_sq(Bc);
   o.r = inv_sq(Br);
   if (ALTW) {
     o.bl = Bl;
@@ -274,9 +316,9 @@ enum { PW_JS = 0, PW_MAPPED = 1, PW_BORGES = 2, PW_YC = 3, PW_NONE = 4 };  // WE
 // w (c + c^2 - 3 c w + w^2) / (c^2 + w (1 - 2c)) of the Jiang-Shu weight w, a quotient of
 // positive terms, so that a small weight keeps its relative precision.
 GBH_HD ff mapped_weight(ff w, double c) {
-  const ff num = (w - ffc(3.0 * c)) * w + ffc(c + c * c);
-  const ff den = addu(w * ffc(1.0 - 2.0 * c), ffc(c * c));
-  return (w * num) * rcp(den);
+  const ff num = muluu(w - ffc(3.0 * c), w) + ffc(c + c * c);
+  const ff den = addu(mulu(w, ffc(1.0 - 2.0 * c)), ffc(c * c));
+  return muluu(muluu(w, num), rcpu(den));
 }
 
 // The weights (w1, w3) of one side from the terms i1, i2, i3 (1/q of the three
@@ -292,14 +334,14 @@ GBH_HD bool side_weights(ff i1, ff i2, ff i3, ff tau, int wtype, ff& w1, ff& w3)
     i3 = T * i3 + ff{3.0f, 0.0f};
   }
   const ff S = addu(addu(i1, i2), i3);
-  const ff R = rcp(S);
-  w1 = i1 * R;
-  w3 = i3 * R;
+  const ff R = rcpu(S);
+  w1 = muluu(i1, R);
+  w3 = muluu(i3, R);
   if (ALTW && wtype == PW_MAPPED) {
-    const ff m1 = mapped_weight(w1, 0.1), m2 = mapped_weight(i2 * R, 0.6), m3 = mapped_weight(w3, 0.3);
-    const ff n = rcp(addu(addu(m1, m2), m3));
-    w1 = m1 * n;
-    w3 = m3 * n;
+    const ff m1 = mapped_weight(w1, 0.1), m2 = mapped_weight(muluu(i2, R), 0.6), m3 = mapped_weight(w3, 0.3);
+    const ff n = rcpu(addu(addu(m1, m2), m3));
+    w1 = muluu(m1, n);
+    w3 = muluu(m3, n);
   }
   return (S.h >= 7.888609e-31f) & (S.h <= 1.0e36f);  // 2^-100; false for NaN
 }
@@ -322,8 +364,8 @@ GBH_HD bool weno_pair_weights(ff t1, ff t2, ff t3, ff l1, ff c2, ff r3, ff r4, f
     tauL = mul2(sqr(t2 - t1), 4.0f);
     tauR = mul2(sqr(t3 - t2), 4.0f);
   }
-  bool ok = side_weights<ALTW>(l1, c2, mulf(r3, 3.0f), tauL, wtype, W.l1, W.l3);
-  ok = side_weights<ALTW>(r4, c3, mulf(l2, 3.0f), tauR, wtype, W.r1, W.r3) & ok;
+  bool ok = side_weights<ALTW>(l1, c2, mulfu(r3, 3.0f), tauL, wtype, W.l1, W.l3);
+  ok = side_weights<ALTW>(r4, c3, mulfu(l2, 3.0f), tauR, wtype, W.r1, W.r3) & ok;
   W.l1 = mul2(W.l1, 2.0f);
   W.r1 = mul2(W.r1, 2.0f);
   return ok;
@@ -375,16 +417,15 @@ GBH_HD bool weno_window_weights(const ff* dl, ff eps4, int wtype, PWeights& W, f
   if (!(ALTW && wtype == PW_NONE)) {
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-      const ff s = dl[k + 1] + dl[k], d2 = mul2(d[k], 2.0f);
-      const ff base = addu(ffc(13.0 / 3.0) * sqr(d[k]), eps4);
+      const ff base = addu(mulu(ffc(13.0 / 3.0), sqr(d[k])), eps4);
       if (k < 2) {
-        const ff B = addu(base, sqr(s + d2));
+        const ff B = addu(base, sqru(d[k] + mul2(dl[k + 1], 2.0f)));
         (k == 0 ? l1 : l2) = inv_sq(B);
         (k == 0 ? bl1 : bl2) = B;
       }
-      if (k == 1 || k == 2) (k == 1 ? c2 : c3) = mulf(inv_sq(addu(base, sqr(s))), 6.0f);
+      if (k == 1 || k == 2) (k == 1 ? c2 : c3) = mulfu(inv_sq(addu(base, sqru(dl[k + 1] + dl[k]))), 6.0f);
       if (k > 1) {
-        const ff B = addu(base, sqr(s - d2));
+        const ff B = addu(base, sqru(mul2(dl[k], 2.0f) - d[k]));
         (k == 2 ? r3 : r4) = inv_sq(B);
         (k == 2 ? br3 : br4) = B;
       }

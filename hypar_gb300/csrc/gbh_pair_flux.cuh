@@ -486,8 +486,8 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
     double uu[NV], fv[NV];
 #pragma unroll
     for (int v = 0; v < NV; v++) uu[v] = su[v * S + w];
-    const Prim<M> pr = to_prim<M>(uu, pp);
-    cell_flux<M, DIR>(pr, fv);
+    const Prim<M> pr = to_prim_mom<M>(uu, pp);
+    cell_flux_mom<M, DIR>(pr, uu[1 + DIR], fv);
 #pragma unroll
     for (int v = 0; v < NV; v++) sf[v * S + w] = fv[v];
     if (GRAV) {
@@ -692,15 +692,15 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
         for (int e = 0; e < ND; e++) acc_fma(acc, neg(Ecc.vel[e]), y[(1 + e) * S]);
         acc_add(acc, y[(NV - 1) * S]);
         a = acc_get(acc);
-        b = ah * (Ecc.un * y[0] - y[(1 + DIR) * S]);
+        b = mulu(ah, mulu(Ecc.un, y[0]) - y[(1 + DIR) * S]);
       };
       // field v of the difference at one face, from its common parts
       auto field = [&](const ff* y, int v, ff a, ff b) {
-        if (v == 0) return gh * a + b;
-        if (v == 1) return gh * a - b;
-        if (v == 2) return y[0] - Ecc.gi * a;
+        if (v < 2) return mulu(gh, a) + (v == 0 ? b : neg(b));
+        if (v == 2) return y[0] - mulu(Ecc.gi, a);
         const int e = (v - 3) + ((v - 3) >= DIR ? 1 : 0);  // the shear fields: transverse directions ascending
-        return Ecc.vel[e < ND ? e : 0] * y[0] - y[(1 + e) * S];
+        return mulu(e == 0 ? Ecc.vel[0] : (e == 1 || ND < 3 ? Ecc.vel[ND > 1 ? 1 : 0] : Ecc.vel[ND - 1]), y[0]) -
+               y[(1 + e) * S];
       };
 #pragma unroll
       for (int k = 0; k < 5; k++) {
@@ -709,7 +709,9 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
           if (h) parts(xc + k, gc[GRAV ? k : 0], tc[GRAV ? k : 0]);
         }
       }
-#pragma unroll
+      // one field at a time (unrolled only with gravity, which keeps values per field): the
+      // unrolled loop's code does not fit the instruction cache
+#pragma unroll(GRAV ? NV : 1)
       for (int v = 0; v < NV; v++) {
         const ff dl[5] = {field(x, v, gs[0], th[0]), field(x + 1, v, gs[1], th[1]), field(x + 2, v, gs[2], th[2]),
                           field(x + 3, v, gs[3], th[3]), field(x + 4, v, gs[4], th[4])};
@@ -826,7 +828,7 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
     const int i = a0 - 3 + q;  // the own cell
     if (ok) {
 #pragma unroll
-      for (int v = 0; v < NV; v++) sg[v * S + w] = to_double(ffc(1.0 / 12.0) * g12[v]);
+      for (int v = 0; v < NV; v++) sg[v * S + w] = to_double(mulu(ffc(1.0 / 12.0), g12[v]));
       if (GRAV && src_dir) {
         ss[w] = to_double(ffc(1.0 / 12.0) * gsm);
         ss[S + w] = to_double(ffc(1.0 / 12.0) * gse);
@@ -848,12 +850,12 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
   }
   __syncthreads();
   if (own) {
-    const double dxi = dxinv[G.g + a0 - 3 + q];
+    const double dxi = dxinv[G.g + a0 - 3 + q], c1 = dxi * (2.0 / 3.0), c2 = dxi * (-1.0 / 12.0);
 #pragma unroll
     for (int v = 0; v < NV; v++) {
       const double* f = sf + v * S + w;
-      const double c4 = fma(2.0 / 3.0, f[1] - f[-1], (f[2] - f[-2]) * (-1.0 / 12.0));
-      double h = dxi * (c4 + (sg[v * S + w] - sg[v * S + w - 1]));
+      const double c4 = fma(c1, f[1] - f[-1], (f[2] - f[-2]) * c2);
+      double h = fma(dxi, sg[v * S + w] - sg[v * S + w - 1], c4);
       if (GRAV && src_dir && (v == 1 + DIR || v == NV - 1)) {
         const int k = v == 1 + DIR ? 0 : 1;
         const double* g = sgg + w;
