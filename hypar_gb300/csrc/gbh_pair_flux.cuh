@@ -94,6 +94,36 @@ __device__ __forceinline__ PCell<M> pcell(const ff* u, const PParams& q, bool wa
   return s;
 }
 
+// Roe average of two conserved states in one pass, with neither 1/rho nor the velocities
+// of the states (roe_eig_cons in gbh_device.cuh).
+template <int M, int DIR>
+__device__ __forceinline__ PEig peig_cons(const ff* a, const ff* b, const PParams& q) {
+  constexpr int ND = ModelTraits<M>::ND, NV = ModelTraits<M>::NV;
+  const ff ra = rsqrt(a[0]), rb = rsqrt(b[0]);
+  const ff ta = a[0] * ra, tb = b[0] * rb;
+  const ff inv = rcp(addu(ta, tb));
+  FAcc qa, qb;
+  PEig E;
+#pragma unroll
+  for (int k = 0; k < ND; k++) {
+    const ff wa = a[1 + k] * ra, wb = b[1 + k] * rb;
+    if (k == 0) {
+      qa = acc_mul(wa, wa);
+      qb = acc_mul(wb, wb);
+    } else {
+      acc_fma(qa, wa, wa);
+      acc_fma(qb, wb, wb);
+    }
+    E.vel[k] = (wa + wb) * inv;
+  }
+  // e + P = e + (gamma-1) (e - |m|^2/(2 rho))
+  const ff Ha = a[NV - 1] + mulu(q.gm1, a[NV - 1] - mul2(acc_get(qa), 0.5f));
+  const ff Hb = b[NV - 1] + mulu(q.gm1, b[NV - 1] - mul2(acc_get(qb), 0.5f));
+  E.H = (mulu(Ha, ra) + mulu(Hb, rb)) * inv;
+  peig_finish<M, DIR>(E, E.H, q);  // (the density serves Euler1D only, which averages cells)
+  return E;
+}
+
 // R diag(c0, c1, c2, ..., c2) L x in the eigen-system E, fields as in projL (0: u_n - a,
 // 1: u_n + a, the rest u_n): since R L = I this is c2 x + (c0 - c2) w0 r0 + (c1 - c2) w1 r1.
 template <int M, int DIR>
@@ -186,7 +216,7 @@ __device__ __forceinline__ ff pharten(ff lam) {
 // value, its right difference and the second differences of the two cells.
 __device__ __forceinline__ ff pmean(ff u2, ff dr, ff d2, ff d3, ff us6) {
   const ff tw = ffc(1.0 / 12.0);
-  return u2 + (mul2(dr, 0.5f) + tw * (us6 - (d2 + d3)));
+  return u2 + (mul2(dr, 0.5f) + mulu(tw, us6 - (d2 + d3)));
 }
 
 // Coefficients of one field for LLF / RF: dissipation alpha, or the side taken (sg).
@@ -220,13 +250,17 @@ __device__ __forceinline__ void pupwind(const ff* fs6, const ff* fd6, const ff* 
     ff a[NV], b[NV];
 #pragma unroll
     for (int v = 0; v < NV; v++) {
-      const ff h = tw * ud6[v];
+      const ff h = mulu(tw, ud6[v]);
       a[v] = um[v] - h;
       b[v] = um[v] + h;
     }
-    sL = pcell<M>(a, q, UPW != UPW_ROE);
-    sR = pcell<M>(b, q, UPW != UPW_ROE);
-    E = peig<M, DIR>(sL, sR, q);
+    if (UPW == UPW_ROE) {
+      E = peig_cons<M, DIR>(a, b, q);
+    } else {
+      sL = pcell<M>(a, q, true);
+      sR = pcell<M>(b, q, true);
+      E = peig<M, DIR>(sL, sR, q);
+    }
     rho = um[0].h;
   } else {
     E = Ecc;
@@ -342,6 +376,120 @@ __device__ __forceinline__ void iface_fp64(const double* __restrict__ U, long lo
   }
 }
 
+// The FP64 evaluation of a block's flagged interfaces by all its threads, for the 1-D and
+// 2-D models: few interfaces lie side by side at a shock, and one thread's chain of some 700
+// dependent FP64 operations takes 20 microseconds, which launches of one or two waves of
+// blocks wait for (shock-entropy line of 20001: 591 -> 437 us for 15 launches; Riemann
+// problem 601x403: 2030 -> 1680 us for 12).  In 3-D the other blocks hide that chain, and
+// this form's registers cost the Taylor-Green 256^3 directions 3 %; there, and with
+// gravity, each thread evaluates its own interface (iface_fp64).  A task is one side of one reconstruction (component-wise) or one field's
+// pair of sides (characteristic); its values go to scr, 4 NV per interface: the pair of
+// quantity 2 v + (0: f, 1: u) at 2 (2 v + h).  Then one thread per interface upwinds.
+// Everything is relative to the interface's left cell, as in iface_flux.
+template <int M, bool CHAR>
+struct Fp64Tasks {
+  static constexpr int NV = ModelTraits<M>::NV, N = CHAR ? 2 * NV : 4 * NV;
+};
+
+// State of cell i of the line with base point pb.
+template <int M, int DIR>
+__device__ __forceinline__ void line_state(const double* __restrict__ U, long long pb, int i, const DevGeom& geo,
+                                           double* u) {
+  constexpr int NV = ModelTraits<M>::NV;
+  const double* src =
+      U + (pb + (long long)fold_index(i, geo.dim[DIR], geo.bclo[DIR], geo.bchi[DIR]) * geo.stride[DIR]) * NV;
+#pragma unroll
+  for (int v = 0; v < NV; v++) u[v] = src[v];
+}
+
+template <int M, int UPW, int DIR>
+__device__ __forceinline__ CellAux<M> cell_aux(const double* u, const PhysParams& pp) {
+  const Prim<M> q = to_prim<M>(u, pp);
+  CellAux<M> a;
+  a.rs = roe_side<M>(q);
+  a.c = 0.0;
+  if (UPW == UPW_RUS) a.c = rusanov_speed<M, DIR>(q, pp);
+  else if (M == MODEL_EULER1D && UPW != UPW_ROE) a.c = sound_speed<M>(q, pp);
+  return a;
+}
+
+template <int M, bool CHAR, int UPW, int DIR, bool ALTW>
+__device__ __forceinline__ void fp64_task(const double* __restrict__ U, long long pb, int i, const DevGeom& geo,
+                                          const double* sf, int S, int w, int task, const PhysParams& pp,
+                                          double* scr) {
+  constexpr int NV = ModelTraits<M>::NV;
+  const double eps4 = 4.0 * pp.eps;
+  if (!CHAR) {
+    const int v = task >> 2, isu = (task >> 1) & 1, right = task & 1;
+    double x[6], m[5];
+#pragma unroll
+    for (int p = 0; p < 6; p++) {
+      const int c = i - 2 + p;
+      const double uv = U[(pb + (long long)fold_index(c, geo.dim[DIR], geo.bclo[DIR], geo.bchi[DIR]) * geo.stride[DIR]) *
+                              NV + v];
+      x[p] = isu ? uv : sf[v * S + w - 2 + p];
+    }
+#pragma unroll
+    for (int p = 0; p < 5; p++) m[p] = (right ? x[5 - p] : x[p]) - x[2];
+    scr[task] = weno5_one_side<ALTW>(m, eps4, pp.wtype);
+  } else {
+    const int v = task >> 1, isu = task & 1;
+    double u[NV], u2[NV];
+    line_state<M, DIR>(U, pb, i, geo, u2);
+    line_state<M, DIR>(U, pb, i + 1, geo, u);
+    const Eig E = roe_eig<M, DIR>(roe_side<M>(to_prim<M>(u2, pp)), roe_side<M>(to_prim<M>(u, pp)), pp);
+    double x[6];
+#pragma unroll
+    for (int p = 0; p < 6; p++) {
+      if (p == 2) {
+        x[p] = 0.0;
+        continue;
+      }
+      double d[NV], y[NV];
+      line_state<M, DIR>(U, pb, i - 2 + p, geo, u);
+#pragma unroll
+      for (int e = 0; e < NV; e++) d[e] = isu ? u[e] - u2[e] : sf[e * S + w - 2 + p] - sf[e * S + w];
+      projL<M, DIR>(E, pp, d, y);
+      x[p] = y[0];
+#pragma unroll
+      for (int e = 1; e < NV; e++) x[p] = v == e ? y[e] : x[p];
+    }
+    double oL, oR;
+    wpair<ALTW, true>(x, x, eps4, pp.wtype, oL, oR);
+    scr[2 * task] = oL;
+    scr[2 * task + 1] = oR;
+  }
+}
+
+template <int M, bool CHAR, int UPW, int DIR>
+__device__ __forceinline__ void fp64_upwind(const double* __restrict__ U, long long pb, int i, const DevGeom& geo,
+                                            const double* sf, int S, int w, const PhysParams& pp, const double* scr,
+                                            double* G) {
+  constexpr int NV = ModelTraits<M>::NV;
+  double fL[NV], fR[NV], uL[NV], uR[NV], u2[NV], u3[NV], f2[NV], fI[NV];
+#pragma unroll
+  for (int v = 0; v < NV; v++) {
+    fL[v] = scr[4 * v];
+    fR[v] = scr[4 * v + 1];
+    uL[v] = scr[4 * v + 2];
+    uR[v] = scr[4 * v + 3];
+    f2[v] = sf[v * S + w];
+  }
+  line_state<M, DIR>(U, pb, i, geo, u2);
+  line_state<M, DIR>(U, pb, i + 1, geo, u3);
+  const CellAux<M> cl = cell_aux<M, UPW, DIR>(u2, pp), cr = cell_aux<M, UPW, DIR>(u3, pp);
+  Eig E;
+  if (NeedCC<M, CHAR, UPW>::value) E = roe_eig<M, DIR>(cl.rs, cr.rs, pp);
+  if (CHAR) upwind_char<M, UPW, DIR>(fL, fR, uL, uR, E, cl, cr, pp, fI, 1.0, u2, f2);
+  else upwind_iface<M, false, UPW, DIR>(fL, fR, uL, uR, E, cl, cr, pp, fI, 1.0, u2, f2);
+#pragma unroll
+  for (int v = 0; v < NV; v++) {
+    const double* f = sf + v * S + w;
+    const double d1 = f[0] - f[-1], d2 = f[1] - f[0], d3 = f[2] - f[1];
+    G[v * S] = fI[v] - fma(6.0, d2, d1 - d3) * (1.0 / 12.0);
+  }
+}
+
 // stage_epilogue of NB values at once: all reads are issued before the first write, so
 // that their latencies overlap.
 template <int NB>
@@ -452,6 +600,8 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
     }
     return pb;
   };
+  int* cnt = (int*)(sf + T + 3);  // interfaces that leave the pairs' bound (a padding slot)
+  if (t == 0) *cnt = 0;
   // Cells a0-3 .. a0+Lc+2 of the lines, consecutive threads on consecutive doubles: along a
   // line for DIR 0, else across the lines.
   if (DIR == 0) {
@@ -820,23 +970,48 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
          (sE <= 1.2e30f) & (ffma(lam, ua, ma) <= 0.09375f * s0) & (ffma(lam, us, ms) <= 0.09375f * sm1);
     if (GRAV && src_dir) ok = ok & (magg * (float)term[0] <= 0.09375f * s0);
   }
-  __syncthreads();  // the differences are read no more: their place takes G and the cells' sums
+  // The differences are read no more: their place takes G and the cells' sums.
+  const int pos = (!GRAV && M != MODEL_NS3D && iface && !ok) ? atomicAdd(cnt, 1) : 0;
+  __syncthreads();
   double* sg = sf + NV * S;
   double* sh = sg + NV * S;
   double* ss = sh + NV * S;  // gravity: the source function's corrections, momentum and energy
+  if (iface && ok) {
+#pragma unroll
+    for (int v = 0; v < NV; v++) sg[v * S + w] = to_double(mulu(ffc(1.0 / 12.0), g12[v]));
+    if (GRAV && src_dir) {
+      ss[w] = to_double(ffc(1.0 / 12.0) * gsm);
+      ss[S + w] = to_double(ffc(1.0 / 12.0) * gse);
+    }
+  }
+  if (GRAV || M == MODEL_NS3D) {
+    if (iface && !ok)
+      iface_fp64<M, CHAR, UPW, DIR, ALTW, GRAV>(U, line_base(l0 + line), a0 - 3 + q, G, sf, sgf, sgg, S, w, pp, src_dir,
+                                                sg + w, ss + w);
+  } else if (const int nbad = *cnt) {
+    int* list = CHAR ? (int*)sx : (int*)sr;  // their slots (in a free place)
+    if (iface && !ok) list[pos] = w;
+    __syncthreads();
+    constexpr int NT = Fp64Tasks<M, CHAR>::N;
+    const int batch = S / 4;  // NV S values of scratch
+    for (int base = 0; base < nbad; base += batch) {
+      const int m = nbad - base < batch ? nbad - base : batch;
+      for (int k = t; k < m * NT; k += T) {
+        const int it = k / NT, x = list[base + it], l = x / LL;
+        fp64_task<M, CHAR, UPW, DIR, ALTW>(U, line_base(l0 + l), a0 - 3 + x - l * LL, G, sf, S, x, k - it * NT, pp,
+                                           sh + it * 4 * NV);
+      }
+      __syncthreads();
+      for (int it = t; it < m; it += T) {
+        const int x = list[base + it], l = x / LL;
+        fp64_upwind<M, CHAR, UPW, DIR>(U, line_base(l0 + l), a0 - 3 + x - l * LL, G, sf, S, x, pp, sh + it * 4 * NV,
+                                       sg + x);
+      }
+      __syncthreads();
+    }
+  }
   if (iface) {
     const int i = a0 - 3 + q;  // the own cell
-    if (ok) {
-#pragma unroll
-      for (int v = 0; v < NV; v++) sg[v * S + w] = to_double(mulu(ffc(1.0 / 12.0), g12[v]));
-      if (GRAV && src_dir) {
-        ss[w] = to_double(ffc(1.0 / 12.0) * gsm);
-        ss[S + w] = to_double(ffc(1.0 / 12.0) * gse);
-      }
-    } else {
-      iface_fp64<M, CHAR, UPW, DIR, ALTW, GRAV>(U, line_base(l0 + line), i, G, sf, sgf, sgg, S, w, pp, src_dir, sg + w,
-                                                ss + w);
-    }
     const int I = i + 1;  // the interface to its right
     if (ep.bnd && (I == 0 || I == N)) {
       double Fb[NV];
