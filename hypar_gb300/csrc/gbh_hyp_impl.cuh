@@ -913,6 +913,7 @@ hyp_lane_kernel(const double* __restrict__ U, double* __restrict__ H, const doub
   __shared__ double srec[TI][2 * NV][2];
   __shared__ double sfI[TI][NV];
   __shared__ Eig secc[TI];
+  pdl_wait();
   const int I0 = (int)blockIdx.x * TC;
   const int N = G.dim[0];
   const long long sd = G.stride[0];
@@ -1103,9 +1104,8 @@ cudaError_t launch_dir(const double* U, double* H, const double* dxinv_dir, cons
       // lane groups: TI interfaces of the one line per block, 16 lanes per interface
       const int ti = -L.seg;
       const unsigned nblk = (unsigned)((N + ti - 2) / (ti - 1));
-      if (ti == 8) hyp_lane_kernel<M, UPW, ALTW, 8><<<nblk, 128, 0, s>>>(U, H, dxinv_dir, G, pp, ep);
-      else hyp_lane_kernel<M, UPW, ALTW, 16><<<nblk, 256, 0, s>>>(U, H, dxinv_dir, G, pp, ep);
-      return cudaGetLastError();
+      if (ti == 8) return launch_pdl(hyp_lane_kernel<M, UPW, ALTW, 8>, nblk, 128, 0, s, U, H, dxinv_dir, G, pp, ep);
+      return launch_pdl(hyp_lane_kernel<M, UPW, ALTW, 16>, nblk, 256, 0, s, U, H, dxinv_dir, G, pp, ep);
     }
   }
   // Steger-Warming and the adjoint's tapes: the FP64 kernels.

@@ -12,6 +12,30 @@
 
 namespace gbh {
 
+// Programmatic dependent launch: the blocks of the next kernel of the stream are placed
+// (and wait in pdl_wait) while this one's last blocks still run, which hides most of the
+// few microseconds between the short launches of a stage.  A kernel launched by
+// launch_pdl calls pdl_wait before it touches memory: it returns when the kernel before
+// it has finished and its writes are visible.
+__device__ __forceinline__ void pdl_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <typename... P, typename... A>
+cudaError_t launch_pdl(void (*k)(P...), unsigned grid, int block, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3((unsigned)block);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, k, P(args)...);
+}
+
 // Ghost-cell source along one face, folded into every halo load:
 // memory = read the ghost point stored in the array (filled by the boundary
 // kernel), periodic = wrap to the opposite interior cell, mirror = HyPar's

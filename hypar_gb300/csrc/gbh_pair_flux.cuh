@@ -1090,6 +1090,7 @@ __global__ void __launch_bounds__(256, PAIR_MINB)
 hyp_pair_kernel(const double* __restrict__ U, double* __restrict__ H, const double* __restrict__ dxinv, DevGeom G,
                 PhysParams pp, StageEpi ep, long long ntrans, int L, int XL) {
   extern __shared__ double pair_smem[];
+  pdl_wait();
   pair_body<M, CHAR, UPW, DIR, ALTW, GRAV>(U, H, dxinv, G, pp, ep, ntrans, L, XL, blockIdx.x, pair_smem);
 }
 
@@ -1104,8 +1105,7 @@ cudaError_t launch_pair(const double* U, double* H, const double* dxinv_dir, con
   const size_t sm = PairLayout<M, CHAR, UPW, ALTW, GRAV>::bytes(p.T);
   if (sm > 48 * 1024)
     if (cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) return e;
-  k<<<(unsigned)nblk, p.T, sm, s>>>(U, H, dxinv_dir, G, pp, ep, ntrans, p.L, p.XL);
-  return cudaGetLastError();
+  return launch_pdl(k, (unsigned)nblk, p.T, sm, s, U, H, dxinv_dir, G, pp, ep, ntrans, p.L, p.XL);
 }
 
 // Ensemble: the blocks of all members in one launch.
@@ -1114,6 +1114,7 @@ __global__ void __launch_bounds__(256, PAIR_MINB)
 hyp_batched_pair_kernel(const MemberDev* __restrict__ mem, int nmem, const double* __restrict__ U,
                         double* __restrict__ H, const double* __restrict__ dxinv, PhysParams pp, StageEpi ep) {
   extern __shared__ double pair_smem[];
+  pdl_wait();
   StageEpi e = ep;
   const long long b = blockIdx.x;
   const MemberDev& m = batched_member<DIR>(mem, nmem, b, e);
@@ -1131,8 +1132,7 @@ cudaError_t launch_batched_dir(const MemberDev* mem, int nmem, long long nblk, i
   const size_t sm = PairLayout<M, CHAR, UPW, false, false>::bytes(T);
   if (sm > 48 * 1024)
     if (cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) return e;
-  k<<<(unsigned)nblk, T, sm, s>>>(mem, nmem, U, H, dxinv, pp, ep);
-  return cudaGetLastError();
+  return launch_pdl(k, (unsigned)nblk, T, sm, s, mem, nmem, U, H, dxinv, pp, ep);
 }
 
 }  // namespace gbh
