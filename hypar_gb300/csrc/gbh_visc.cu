@@ -59,6 +59,7 @@ enum { VQ_T = 3, VQ_MU = 4, VQ_PAIR = 5 };
 __global__ void __launch_bounds__(256)
 visc_q_kernel(const double* __restrict__ u, double* __restrict__ Q, const double* __restrict__ dxinv, DevGeom G,
               ViscParams vp, int* __restrict__ flag, int id) {
+  pdl_wait();
   const int ng0 = G.dim[0] + 2 * G.g, ng1 = G.dim[1] + 2 * G.g, ng2 = G.dim[2] + 2 * G.g;
   const long long n = (long long)ng0 * ng1 * ng2;
   long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -214,6 +215,7 @@ __device__ __forceinline__ void visc_flux_at(const double* __restrict__ Q, doubl
 __global__ void __launch_bounds__(256)
 visc_flux_kernel(const double* __restrict__ Q, double* __restrict__ F, const double* __restrict__ dxinv, DevGeom G,
                  ViscParams vp, const int* __restrict__ flag, int id) {
+  pdl_wait();
   const int ng[3] = {G.dim[0] + 2 * G.g, G.dim[1] + 2 * G.g, G.dim[2] + 2 * G.g};
   const long long n = (long long)ng[0] * ng[1] * ng[2];
   const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -265,6 +267,7 @@ __device__ __forceinline__ void visc_div_at(const double* __restrict__ F0, doubl
 __global__ void __launch_bounds__(256)
 visc_div_kernel(const double* __restrict__ F, double* __restrict__ par, const double* __restrict__ dxinv, DevGeom G,
                 ViscParams vp, const int* __restrict__ flag, int id) {
+  pdl_wait();
   const long long m = (long long)G.dim[0] * G.dim[1] * G.dim[2];
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= m) return;
@@ -289,10 +292,10 @@ cudaError_t launch_visc(const double* u, double* Q, double* F, double* par, cons
   const long long n = (long long)(G.dim[0] + 2 * G.g) * (G.dim[1] + 2 * G.g) * (G.dim[2] + 2 * G.g);
   const long long m = (long long)G.dim[0] * G.dim[1] * G.dim[2];
   if (vp.order == 2) flag = nullptr;
-  visc_q_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(u, Q, dxinv, G, vp, flag, id);
-  visc_flux_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(Q, F, dxinv, G, vp, flag, id);
-  visc_div_kernel<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(F, par, dxinv, G, vp, flag, id);
-  return cudaGetLastError();
+  const unsigned gn = (unsigned)((n + 255) / 256), gm = (unsigned)((m + 255) / 256);
+  if (cudaError_t e = launch_pdl(visc_q_kernel, gn, 256, 0, s, u, Q, dxinv, G, vp, flag, id)) return e;
+  if (cudaError_t e = launch_pdl(visc_flux_kernel, gn, 256, 0, s, Q, F, dxinv, G, vp, flag, id)) return e;
+  return launch_pdl(visc_div_kernel, gm, 256, 0, s, F, par, dxinv, G, vp, flag, id);
 }
 
 // ---------------------------------------------------------------------------
@@ -382,6 +385,7 @@ __device__ __forceinline__ void bc_ghost(const ZoneDev& z, const double* w, doub
 }
 
 __global__ void bc_zone_kernel(double* u, DevGeom G, int nv, ZoneDev z) {
+  pdl_wait();
   int b[3] = {1, 1, 1};
   for (int d = 0; d < G.nd; d++) b[d] = z.ie[d] - z.is[d];
   long long n = (long long)b[0] * b[1] * b[2];
@@ -505,8 +509,7 @@ cudaError_t launch_bc_zone_t(double* u, const DevGeom& G, int nv, const int* zon
     if (d < G.nd) n *= (z.ie[d] - z.is[d] > 0 ? z.ie[d] - z.is[d] : 0);
   }
   if (n <= 0) return cudaSuccess;
-  bc_zone_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(u, G, nv, z);
-  return cudaGetLastError();
+  return launch_pdl(bc_zone_kernel, (unsigned)((n + 255) / 256), 256, 0, s, u, G, nv, z);
 }
 
 // The sponge zone's source (BCSponge.c:34-61): src -= sigma_i (u - u_ref) at every
