@@ -1,4 +1,4 @@
-// gbh_hyp_impl.cuh -- the fused hyperbolic kernel, one launch per direction.
+// gbh_hyp_impl.cuh -- the hyperbolic term, one launch per direction.
 //
 // Replaces, for one direction d, HyPar's FFunction -> SetInterpLimiterVar ->
 // UFunction -> 4x InterpolateInterfacesHyp -> Upwind -> flux difference chain
@@ -7,12 +7,16 @@
 // right-hand-side assembly (TimeRHSFunctionExplicit.c:89-92) and the stage
 // update of TimeRK (TimeRK.c:126-195).
 //
-// Each thread walks `seg` consecutive interfaces of one grid line along d,
-// keeping a six-cell window (cells j-3..j+2 of interface j-1/2) in registers:
-// a cell's flux, Roe-average ingredients and modified state are computed once,
-// when the cell enters the window, and the flux difference of cell j-1 is
-// formed from the previous interface's flux held in registers, so no interface
-// array ever reaches memory.  Ghost cells outside the domain are read through
+// Here: the FP64 evaluation of one interface (iface_flux), the kernels built on it for
+// Steger-Warming splitting and the adjoint's tapes, the lane groups of short 1-D lines,
+// and the launchers.  Everything else runs in gbh_pair_flux.cuh, which takes iface_flux
+// where its bound fails.
+//
+// The segment walker: a thread walks `seg` consecutive interfaces of one grid line along
+// d, keeping a six-cell window (cells j-3..j+2 of interface j-1/2) in registers: a cell's
+// flux, Roe-average ingredients and modified state are computed once, when the cell
+// enters the window, and the flux difference of cell j-1 is formed from the previous
+// interface's flux held in registers.  Ghost cells outside the domain are read through
 // the boundary fold (periodic wrap / mirror) or from memory.
 #pragma once
 
@@ -566,23 +570,16 @@ __device__ __forceinline__ void iface_flux(const double (&wu)[6][ModelTraits<M>:
 // One thread's share of a launch: interfaces [sg*seg, min((sg+1)*seg, N)] of
 // the grid line with transverse index `tr` (other dimensions ascending, first
 // fastest), and the flux difference / epilogue of the cells in between.
-// GRAV (NavierStokes3D with Rusanov): the well-balanced gravity treatment --
-// the modified solution uC = [f u_{0..3}, P/(gamma-1)/g + f rho|v|^2/2]
-// (NavierStokes3DModifiedSolution.c:52-66), the dissipation factor
-// max(g_L, g_R) (NavierStokes3DUpwind.c:407) and, along a direction with
-// gravity, the source term of NavierStokes3DSource.c:38-112 subtracted from
-// the hyperbolic term of this direction (except when only that term is asked for).
 // WT (Euler2D, component-wise, Jiang-Shu: the adjoint's configuration): the wide
 // tape -- per interface uL, uR and, per component, the smoothness terms and
 // normalisation reciprocals of the f and u pairs (TAPE_WIDE doubles).
-template <int M, bool CHAR, int UPW, int DIR, bool ALTW = false, bool GRAV = false, bool WT = false>
+template <int M, bool CHAR, int UPW, int DIR, bool ALTW = false, bool WT = false>
 __device__ __forceinline__ void hyp_segment(const double* __restrict__ U, double* __restrict__ H,
                                             const double* __restrict__ dxinv, const DevGeom& G,
                                             const PhysParams& pp, const StageEpi& ep, int seg, long long tr,
                                             int sg) {
   constexpr int NV = ModelTraits<M>::NV, ND = ModelTraits<M>::ND;
   constexpr bool CC = NeedCC<M, CHAR, UPW>::value;
-  constexpr bool REL = RelFlux<GRAV>::value;
   const long long line = tr;
 
   long long pbase = (long long)G.g * G.stride[DIR];
@@ -601,9 +598,8 @@ __device__ __forceinline__ void hyp_segment(const double* __restrict__ U, double
   const double eps4 = 4.0 * pp.eps;
 
   double wu[6][NV], wf[6][NV], wuc[6];
-  double wgf[6], wgg[6];  // gravity fields f, g (GRAV)
+  double wgf[6], wgg[6];  // (gravity fields: not used here)
   CellAux<M> ax[6];
-  const bool src_dir = GRAV && pp.grav[DIR] != 0.0 && (ep.mode != EPI_HYP || ep.with_source);
 
   auto load = [&](int i) {
     const long long pt = pbase + (long long)fold_index(i, N, lo, hi) * sd;
@@ -612,18 +608,7 @@ __device__ __forceinline__ void hyp_segment(const double* __restrict__ U, double
     for (int v = 0; v < NV; v++) wu[5][v] = src[v];
     Prim<M> q = to_prim<M>(wu[5], pp);
     cell_flux<M, DIR>(q, wf[5]);
-    if (GRAV) {
-      wgf[5] = pp.gf[pt];
-      wgg[5] = pp.gg[pt];
-      if (M == MODEL_EULER1D) {
-        wuc[5] = wu[5][NV - 1] * wgf[5];  // u* = u / S (gf holds 1 / S)
-      } else {
-        double vsq = q.vel[0] * q.vel[0] + q.vel[1] * q.vel[1] + q.vel[2] * q.vel[2];
-        wuc[5] = fma(q.P * pp.inv_gm1, nr_rcp(wgg[5]), (0.5 * q.rho * vsq) * wgf[5]);
-      }
-    } else {
-      wuc[5] = ufunc_energy<M>(q, pp, wu[5][NV - 1]);
-    }
+    wuc[5] = ufunc_energy<M>(q, pp, wu[5][NV - 1]);
     if (CC) ax[5].rs = roe_side<M>(q);
     if (UPW == UPW_RUS) ax[5].c = rusanov_speed<M, DIR>(q, pp);
     else if (M == MODEL_EULER1D && UPW != UPW_ROE) ax[5].c = sound_speed<M>(q, pp);
@@ -637,10 +622,6 @@ __device__ __forceinline__ void hyp_segment(const double* __restrict__ U, double
         wf[p][v] = wf[p + 1][v];
       }
       wuc[p] = wuc[p + 1];
-      if (GRAV) {
-        wgf[p] = wgf[p + 1];
-        wgg[p] = wgg[p + 1];
-      }
       ax[p] = ax[p + 1];
     }
   };
@@ -650,14 +631,14 @@ __device__ __forceinline__ void hyp_segment(const double* __restrict__ U, double
     shift();
   }
 
-  double fIp[NV], SI[NV], SIp[NV];
+  double fIp[NV], SI[NV];
 #pragma unroll
-  for (int v = 0; v < NV; v++) fIp[v] = SI[v] = SIp[v] = 0.0;
+  for (int v = 0; v < NV; v++) fIp[v] = SI[v] = 0.0;
 
   for (int I = I0; I <= I1; I++) {
     load(I + 2);
     double fI[NV];
-    iface_flux<M, CHAR, UPW, DIR, ALTW, GRAV, WT>(wu, wf, wuc, wgf, wgg, ax, pp, ep, eps4, src_dir,
+    iface_flux<M, CHAR, UPW, DIR, ALTW, false, WT>(wu, wf, wuc, wgf, wgg, ax, pp, ep, eps4, false,
                                                    line * (N + 1) + I, fI, SI);
     if (ep.bnd && (I == 0 || I == N)) {
       long long ntr = 1;
@@ -666,7 +647,7 @@ __device__ __forceinline__ void hyp_segment(const double* __restrict__ U, double
         if (e != DIR) ntr *= G.dim[e];
       double Fb[NV];
 #pragma unroll
-      for (int v = 0; v < NV; v++) Fb[v] = REL ? fI[v] + wf[2][v] : fI[v];
+      for (int v = 0; v < NV; v++) Fb[v] = fI[v] + wf[2][v];
       boundary_flux<NV>(ep, I, N, line, ntr, Fb);
     }
 
@@ -676,21 +657,11 @@ __device__ __forceinline__ void hyp_segment(const double* __restrict__ U, double
       const long long off = (pbase + (long long)c * sd) * NV;
       const double dxi = dxinv[G.g + c];
       const bool finish = ep.last && ep.mode != EPI_HYP;
-      double kv[NV], term[NV];
-      if (src_dir) {
-        // [0, rho RT e_DIR, rho RT v_DIR] f of the cell (NavierStokes3DSource.c:92-97)
-        const double rho = wu[2][0], rRT = rho * pp.RT, f = wgf[2];
-        const double vd = rho == 0.0 ? 0.0 : wu[2][1 + DIR] * nr_rcp(rho);
-#pragma unroll
-        for (int v = 0; v < NV; v++) term[v] = 0.0;
-        term[1 + DIR] = rRT * f;
-        term[NV - 1] = (rRT * vd) * f;
-      }
+      double kv[NV];
 #pragma unroll
       for (int v = 0; v < NV; v++) {
         // centre-relative fluxes: F_I - F_{I-1} = (f_c - f_{c-1}) + (fI_I - fI_{I-1})
-        double h = REL ? dxi * ((wf[2][v] - wf[1][v]) + (fI[v] - fIp[v])) : dxi * (fI[v] - fIp[v]);
-        if (src_dir) h = fma(-term[v] * (SI[v] - SIp[v]), dxi, h);  // rhs = -hyp + source
+        const double h = dxi * ((wf[2][v] - wf[1][v]) + (fI[v] - fIp[v]));
         double hyp = ep.first ? h : H[off + v] + h;
         if (!finish) {
           H[off + v] = hyp;
@@ -721,10 +692,7 @@ __device__ __forceinline__ void hyp_segment(const double* __restrict__ U, double
       }
     }
 #pragma unroll
-    for (int v = 0; v < NV; v++) {
-      fIp[v] = fI[v];
-      SIp[v] = SI[v];
-    }
+    for (int v = 0; v < NV; v++) fIp[v] = fI[v];
     shift();
   }
 }
@@ -1013,18 +981,17 @@ hyp_tile_kernel(const double* __restrict__ U, double* __restrict__ H, const doub
   hyp_tile_body<M, CHAR, UPW, DIR, ALTW, TI, WT>(U, H, dxinv, G, pp, ep, ntrans, blockIdx.x);
 }
 
-template <int M, bool CHAR, int UPW, int DIR, bool ALTW, bool GRAV = false, bool WT = false>
+template <int M, bool CHAR, int UPW, int DIR, bool ALTW, bool WT = false>
 __global__ void __launch_bounds__(128)
 hyp_dir_kernel(const double* __restrict__ U, double* __restrict__ H, const double* __restrict__ dxinv,
                DevGeom G, PhysParams pp, StageEpi ep, int seg, int nseg, long long ntrans) {
   long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (tid >= ntrans * (long long)nseg) return;
-  hyp_segment<M, CHAR, UPW, DIR, ALTW, GRAV, WT>(U, H, dxinv, G, pp, ep, seg, tid % ntrans, (int)(tid / ntrans));
+  hyp_segment<M, CHAR, UPW, DIR, ALTW, WT>(U, H, dxinv, G, pp, ep, seg, tid % ntrans, (int)(tid / ntrans));
 }
 
-// All members of an ensemble advanced by one launch per direction: a thread
-// finds its member by binary search over the start offsets, then walks its
-// segment exactly as in the single-grid kernel.
+// All members of an ensemble advanced by one launch per direction: a block finds its
+// member by binary search over the start offsets, then works as in the single-grid kernel.
 // The member that owns work item `w` of direction DIR (members' first items
 // ascending), with the stage pointers moved to its arrays.
 template <int DIR>
@@ -1116,36 +1083,29 @@ cudaError_t launch_dir(const double* U, double* H, const double* dxinv_dir, cons
       return launch_pair<M, CHAR, UPW, DIR, ALTW, GRAV>(U, H, dxinv_dir, G, pp, ep, ntrans, pair_cap_of(L.seg, L.block), s);
   }
   if constexpr (!PAIR || TAPE) {
-  if (L.seg < 0 && !GRAV) {
-    // tiles of -seg interfaces (32, 64 or 128), one block each
-    const int ti = -L.seg;
-    const long long nblk = ntrans * ((N + ti - 2) / (ti - 1));
-    if (ti == 32)
-      hyp_tile_kernel<M, CHAR, UPW, DIR, ALTW, 32, WT><<<(unsigned)nblk, 32, 0, s>>>(U, H, dxinv_dir, G, pp, ep,
-                                                                                   ntrans);
-    else if (ti == 64)
-      hyp_tile_kernel<M, CHAR, UPW, DIR, ALTW, 64, WT><<<(unsigned)nblk, 64, 0, s>>>(U, H, dxinv_dir, G, pp, ep,
-                                                                                   ntrans);
-    else
-      hyp_tile_kernel<M, CHAR, UPW, DIR, ALTW, 128, WT><<<(unsigned)nblk, 128, 0, s>>>(U, H, dxinv_dir, G, pp, ep,
-                                                                                     ntrans);
+    if (L.seg < 0) {
+      // tiles of -seg interfaces (32, 64 or 128), one block each
+      const int ti = -L.seg;
+      const long long nblk = ntrans * ((N + ti - 2) / (ti - 1));
+      if (ti == 32)
+        hyp_tile_kernel<M, CHAR, UPW, DIR, ALTW, 32, WT><<<(unsigned)nblk, 32, 0, s>>>(U, H, dxinv_dir, G, pp, ep,
+                                                                                       ntrans);
+      else if (ti == 64)
+        hyp_tile_kernel<M, CHAR, UPW, DIR, ALTW, 64, WT><<<(unsigned)nblk, 64, 0, s>>>(U, H, dxinv_dir, G, pp, ep,
+                                                                                       ntrans);
+      else
+        hyp_tile_kernel<M, CHAR, UPW, DIR, ALTW, 128, WT><<<(unsigned)nblk, 128, 0, s>>>(U, H, dxinv_dir, G, pp, ep,
+                                                                                         ntrans);
+      return cudaGetLastError();
+    }
+    const int seg = L.seg > 0 ? L.seg : 32;
+    const int nseg = (N + seg - 1) / seg;
+    const long long nthr = ntrans * nseg;
+    const int block = L.block > 0 ? L.block : 128;
+    const long long grid = (nthr + block - 1) / block;
+    hyp_dir_kernel<M, CHAR, UPW, DIR, ALTW, WT><<<(unsigned)grid, block, 0, s>>>(U, H, dxinv_dir, G, pp, ep, seg, nseg,
+                                                                                 ntrans);
     return cudaGetLastError();
-  }
-  // a tile shape asked of a kernel without the tile form (gravity): segments that
-  // spread the line over about four warps per SM
-  int seg = L.seg > 0 ? L.seg : 32;
-  if (L.seg < 0) {
-    const long long want = 152LL * 4 * 32;
-    seg = (int)((ntrans * N + want - 1) / want);
-    seg = seg < 1 ? 1 : (seg > 64 ? 64 : seg);
-  }
-  int nseg = (N + seg - 1) / seg;
-  long long nthr = ntrans * nseg;
-  int block = L.block > 0 ? L.block : 128;
-  long long grid = (nthr + block - 1) / block;
-  hyp_dir_kernel<M, CHAR, UPW, DIR, ALTW, GRAV, WT><<<(unsigned)grid, block, 0, s>>>(U, H, dxinv_dir, G, pp, ep,
-                                                                                  seg, nseg, ntrans);
-  return cudaGetLastError();
   }
 }
 

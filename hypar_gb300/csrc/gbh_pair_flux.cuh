@@ -325,7 +325,8 @@ __device__ __forceinline__ void pupwind(const ff* fs6, const ff* fd6, const ff* 
   (void)ND;
 }
 
-// The FP64 evaluation of one interface as the correction G, written to G[v S]; with
+// The FP64 evaluation of one interface by its own thread (3-D, gravity) as the correction
+// G, written to G[v S]; with
 // gravity (sgf, sgg: the hydrostatic fields) also the source function's interface values
 // as corrections of its central value, to Gs.  Window: cells i-2 .. i+3 of the line with
 // base point pb (states from memory), own cell = slot w (fluxes in shared memory).
