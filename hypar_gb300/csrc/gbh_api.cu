@@ -537,7 +537,7 @@ extern "C" int gb_solver_create(const gb_config* cfg, const double* dxinv, int d
     if (c.zones[z][0] == GB_BC_SPONGE && !zone_empty(c, z)) s->sponge = true;
   if (s->viscous || s->sponge) A(&s->d_par, bytes);
   if (s->viscous) {
-    A(&s->d_Q, (size_t)st * 9 * sizeof(double));
+    A(&s->d_Q, (size_t)st * 7 * sizeof(double));
     A(&s->d_Gr, (size_t)st * 9 * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc((void**)&s->d_vflag, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(s->d_vflag, 0, sizeof(int));

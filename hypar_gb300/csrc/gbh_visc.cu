@@ -8,14 +8,14 @@
 // lines whose other indices are interior, so at a ghost point the derivatives
 // across the ghost direction are zero.  Three passes over arrays of one component each
 // (consecutive threads, consecutive addresses):
-//   visc_q    : velocity, T = gamma P / rho and mu = T^0.76 at every point
+//   visc_q    : velocity and T = gamma P / rho at every point
 //   visc_flux : the scaled derivatives of velocity and temperature, with the rule above,
-//               and from them the stress tensor (6) and the energy fluxes (3)
+//               and from them and mu = T^0.76 the stress tensor (6) and the energy fluxes (3)
 //   visc_div  : par = sum over d of dxinv_d d/dx_d (flux along d) at interior points.
 //
 // All three are bound by arithmetic, the FP64 pipe above all (2 operations per clock and
-// SM), so the passes share what the three directions have in common (162 FP64 operations
-// per point against the 310 of one flux pass per direction) and, where the viscous flux is
+// SM), so the passes share what the three directions have in common (some 150 FP64
+// operations per point against the 310 of one flux pass per direction) and, where the viscous flux is
 // small against the convective one, work in pairs of FP32 numbers (gbh_pair.cuh): the
 // derivatives of the velocity, the stresses, the energy flux and their divergence.
 // Velocities hold 48 bits as pairs, so their derivatives are off by 2^-50 |v| / h and the
@@ -23,7 +23,7 @@
 // that is below a quarter of the rounding of the convective flux (rho a^2) it is added to.
 // visc_q checks this, and any point that fails (or leaves the pairs' range, or is not
 // finite) turns the whole evaluation to FP64.  Temperature derivatives stay in FP64.
-// 256^3: 8.30 -> 1.65 ms per evaluation.
+// 256^3: 8.30 -> 2.5 ms per evaluation.
 #include "gbh_internal.h"
 #include "gbh_pair.cuh"
 
@@ -37,22 +37,33 @@ __device__ __forceinline__ int fold1(int i, int N, int lo, int hi) {
 
 
 // T^0.76 (raiseto, include/math_ops.h:37).  y = T^(19/25) from an FP32 estimate y0 and
-// z = y0^25 / T^19: y = y0 z^(-1/25) = y0 (1 + e/25 + 13 e^2/625 + ...), e = 1 - z.  The
-// estimate's error of some 1e-6 leaves 1e-17 after these terms, and the rounding of z
-// (some ten units) counts a 25th: 20 FP64 operations against about 90 of exp(0.76 log T),
-// at its accuracy.
+// z = y0^25 / T^19 = (y0 / T)^19 y0^6: y = y0 z^(-1/25) = y0 (1 + e/25 + 13 e^2/625 + ...),
+// e = 1 - z.  The estimate's error of some 1e-6 leaves 1e-17 after these terms, and the
+// rounding of z (some ten units) counts a 25th: 18 FP64 operations against about 90 of
+// exp(0.76 log T), at its accuracy.
 __device__ __forceinline__ double pow076(double T) {
   const float t = d2f_mag(T);
   if (!(T > 0.0) || !(t > 1e-8f) || !(t < 1e8f)) return exp(0.76 * log(T));
-  const double y = (double)exp2f(0.76f * log2f(t)), r = nr_rcp(T);
-  const double y2 = y * y, y4 = y2 * y2, y8 = y4 * y4, y16 = y8 * y8;
-  const double r2 = r * r, r4 = r2 * r2, r8 = r4 * r4, r16 = r8 * r8;
-  const double e = fma(-((y16 * y8) * y), (r16 * r2) * r, 1.0);
+  const double y = (double)exp2f(0.76f * log2f(t)), k = y * nr_rcp(T);
+  const double k2 = k * k, k4 = k2 * k2, k8 = k4 * k4, k16 = k8 * k8, y2 = y * y;
+  const double e = fma(-((k16 * k2) * k), (y2 * y2) * y2, 1.0);
   return fma(y * e, fma(13.0 / 625.0, e, 0.04), y);
 }
+// The same as a pair: z in pairs, to 2^-44 or so, whose 25th is the pair's own precision.
+// (Beyond 1e-4 .. 1e4 the powers' second words leave the FP32 range: FP64.)
+__device__ __forceinline__ ff pow076_pair(double T) {
+  const float t = d2f_mag(T);
+  if (!(T > 0.0) || !(t > 1e-4f) || !(t < 1e4f)) return to_pair(pow076(T));
+  const float y = exp2f(0.76f * log2f(t));
+  const ff k = mulf(rcp(to_pair(T)), y), k2 = sqr(k), k16 = sqr(sqr(sqr(k2)));
+  const ff y2 = {fmul(y, y), ffma(y, y, -fmul(y, y))};
+  const ff z = ((k16 * k2) * k) * (sqr(y2) * y2);
+  const ff e = ff{1.0f, 0.0f} - z;
+  return ff{y, 0.0f} + mulf(e * (ffc(0.04) + ff{fmul(0.0208f, e.h), 0.0f}), y);
+}
 
-// Arrays of one component each, n points: doubles u, v, w, T, mu, then pairs u, v, w, mu.
-enum { VQ_T = 3, VQ_MU = 4, VQ_PAIR = 5 };
+// Arrays of one component each, n points: doubles u, v, w, T, then pairs u, v, w.
+enum { VQ_T = 3, VQ_PAIR = 4 };
 
 // At all points including ghosts; ghost points read through the fold.  *flag takes `id`
 // where the pairs' bound fails.
@@ -78,17 +89,13 @@ visc_q_kernel(const double* __restrict__ u, double* __restrict__ Q, const double
   double v[3];
 #pragma unroll
   for (int d = 0; d < 3; d++) v[d] = rho == 0.0 ? 0.0 : uu[1 + d] * ri;
-  double vsq = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
-  double P = (uu[4] - 0.5 * rho * vsq) * vp.gm1;
-  double T = vp.gamma * P * ri;
-  const double mu = pow076(T);
+  const double mv = fma(uu[1], v[0], fma(uu[2], v[1], uu[3] * v[2]));  // rho |v|^2
+  const double T = vp.gamma * (fma(-0.5, mv, uu[4]) * vp.gm1) * ri;
 #pragma unroll
   for (int d = 0; d < 3; d++) Q[d * n + p] = v[d];
   Q[VQ_T * n + p] = T;
-  Q[VQ_MU * n + p] = mu;
   if (!flag) return;
   ff* R = (ff*)(Q + VQ_PAIR * n);
-  const ff pm = to_pair(mu);
   float vm = 0.0f;
 #pragma unroll
   for (int d = 0; d < 3; d++) {
@@ -96,10 +103,9 @@ visc_q_kernel(const double* __restrict__ u, double* __restrict__ Q, const double
     R[d * n + p] = pv;
     vm = fadd(vm, fabsf(pv.h));
   }
-  R[3 * n + p] = pm;
   const float h = fmaxf(d2f_mag(dxinv[G.g + i]), fmaxf(d2f_mag(dxinv[ng0 + G.g + j]), d2f_mag(dxinv[ng0 + ng1 + G.g + k])));
-  const float t = d2f_mag(T), r = d2f_mag(rho);
-  const bool ok = (T > 0.0) & (pm.h * (float)vp.inv_Re * h <= 0.03125f * r * sqrtf(t)) & (t >= 1e-18f) & (t <= 1e18f) &
+  const float t = d2f_mag(T), r = d2f_mag(rho), mu = exp2f(0.76f * log2f(t));
+  const bool ok = (T > 0.0) & (mu * d2f_mag(vp.inv_Re) * h <= 0.03125f * r * sqrtf(t)) & (t >= 1e-18f) & (t <= 1e18f) &
                   (r >= 1e-18f) & (vm <= 1e18f) & (h <= 1e18f);
   if (!ok) *flag = id;
 }
@@ -155,6 +161,10 @@ template <> __device__ __forceinline__ ff vnum<ff>(double x) { return to_pair(x)
 __device__ __forceinline__ double vout(double x) { return x; }
 __device__ __forceinline__ double vout(ff x) { return to_double(x); }
 
+template <class T> __device__ __forceinline__ T vmu(double t);
+template <> __device__ __forceinline__ double vmu<double>(double t) { return pow076(t); }
+template <> __device__ __forceinline__ ff vmu<ff>(double t) { return pow076_pair(t); }
+
 // The stress tensor (xx, yy, zz, xy, xz, yz) and energy fluxes (x, y, z) at one point
 // (NavierStokes3DParabolicFunction.c:151-314) from the derivatives along the lines whose
 // other indices are interior (on[e]; the rest are zero).
@@ -163,7 +173,6 @@ __device__ __forceinline__ void visc_flux_at(const double* __restrict__ Q, doubl
                                              const ViscParams& vp, const double* di, long long n, long long p,
                                              const int* idx, const bool* on) {
   const T* V = (const T*)(sizeof(T) == sizeof(double) && __is_same(T, double) ? Q : Q + VQ_PAIR * n);
-  const T* MU = __is_same(T, double) ? (const T*)(Q + VQ_MU * n) : V + 3 * n;
   const double* TT = Q + VQ_T * n;
   T D[3][3], H[3];  // D[e][c] = d v_c / dx_e, H[e] = dT/dx_e
 #pragma unroll
@@ -194,7 +203,7 @@ __device__ __forceinline__ void visc_flux_at(const double* __restrict__ Q, doubl
     if (central) H[e] = vnum<T>(fma(8.0, b[sd] - b[-sd], b[-2 * sd] - b[2 * sd]) * d12);
     else H[e] = vnum<T>((vp.order == 2 ? d1(i, N, G.g, 1, fk) : d4(i, N, G.g, fk)) * di[e]);
   }
-  const T mr = vmul(MU[p], vnum<T>(vp.inv_Re)), kq = vmul(mr, vnum<T>(vp.inv_gm1 * vp.inv_Pr));
+  const T mr = vmul(vmu<T>(TT[p]), vnum<T>(vp.inv_Re)), kq = vmul(mr, vnum<T>(vp.inv_gm1 * vp.inv_Pr));
   const T third = vmul(vadd(vadd(D[0][0], D[1][1]), D[2][2]), vnum<T>(2.0 / 3.0));
   T s[6];
 #pragma unroll
