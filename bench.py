@@ -51,25 +51,18 @@ UNIT = "cell-component updates/s"
 # with the launch shapes the autotuner picks at full size, whose per-cell work is
 # that of the full grid to within the segment-boundary share).
 FP64_PER_CELL_STEP = {
-    "vortex": {"tile": {"flops": 8454.6, "instr": 5494.4, "captured": "512^2, tiles of 128 interfaces"},
-               "walker": {"flops": 8585.4, "instr": 5575.5, "captured": "512^2, segments 54/27"}},
+    "vortex": {"pairs": {"flops": 492.7, "instr": 447.5, "captured": "1024^2 (the full grid)"}},
     "sod": {"lanes": {"flops": 3654.7, "instr": 2455.2, "captured": "1024 (the full grid), lane groups of 16"}},
-    "tgv": {"walker": {"flops": 18445.5, "instr": 12291.2,
-                       "captured": "128^3, segments 48/32/32 (the earlier 256^3 shape)"},
-            "tile": {"flops": 16107.9, "instr": 10815.0, "captured": "128^3, tiles of 64 (the 256^3 shape)"}},
-    "rtb": {"walker": {"flops": 16583.3, "instr": 11627.6, "captured": "128^3, segments 32/32/32 (the 201^3 shape)"}},
-    "rtb64": {"walker": {"flops": 25265.3, "instr": 17712.2, "captured": "64^3 (the full grid), segments 7/7/7"}},
-    "dns": {"walker": {"flops": 20731.2, "instr": 14874.6, "captured": "128^3, segments 48/48/48 (the 256^3 shape)"}},
-    "dns64cr": {"walker": {"flops": 34332.9, "instr": 23470.2, "captured": "64^3 (the full grid), segments 5/5/4"}},
+    "tgv": {"pairs": {"flops": 1395.0, "instr": 1238.3, "captured": "128^3"}},
+    "rtb": {"pairs": {"flops": 1360.7, "instr": 1188.4, "captured": "128^3"}},
+    "rtb64": {"pairs": {"flops": 1864.3, "instr": 1618.3, "captured": "64^3 (the full grid)"}},
+    "dns": {"pairs": {"flops": 1053.8, "instr": 932.5, "captured": "128^3"}},
+    "dns64cr": {"pairs": {"flops": 11671.3, "instr": 7694.7, "captured": "64^3 (the full grid)"}},
 }
 # DRAM bytes (read + write) per cell of one launch (x launch / y launch with the RK
-# update), per kernel form: the segment walker from a 2048^2 capture of the
-# centre-relative kernels (traffic proportional to cells at these sizes), the tile form
-# from a capture of the default 1024^2 run (the 34 MB state partly stays in L2 there).
-DRAM_BYTES_PER_CELL = {"vortex": {("hyp_x", "walker"): 57.32, ("hyp_y", "walker"): 153.39,
-                                  ("hyp_x", "tile"): 32.35, ("hyp_y", "tile"): 110.18}}
-TRAFFIC_SOURCE = {"walker": "a 2048^2 capture of the segment-walker form, scaled by cells",
-                  "tile": "a 1024^2 capture of the tile form"}
+# update), from a capture of the default 1024^2 run (the 34 MB state partly stays in L2).
+DRAM_BYTES_PER_CELL = {"vortex": {("hyp_x", "pairs"): 32.68, ("hyp_y", "pairs"): 128.78}}
+TRAFFIC_SOURCE = {"pairs": "a 1024^2 capture"}
 
 
 # The reference's published GPU numbers for the same decks (cell-component updates/s):
@@ -335,7 +328,7 @@ def run_ours(args, case, desc, ws, rank, local):
     achieved_gbs = bytes_per_launch / avg_launch_s / 1e9
     cls_dir = "xyz".index(cls[-1]) if cls.startswith("hyp_") else 0
     seg0 = tuned[cls_dir][0] if tuned else 0
-    form = "lanes" if seg0 in (-8, -16) else ("tile" if seg0 < 0 else "walker")
+    form = "lanes" if seg0 in (-8, -16) else "pairs"
     traffic = DRAM_BYTES_PER_CELL.get(args.workload, {}).get((cls, form))
     roofline = {"bound": "hbm", "achieved": achieved_gbs, "peak": hbm_peak, "unit": "GB/s",
                 "frac": achieved_gbs / hbm_peak, "traffic": traffic * cells if traffic else None,
@@ -346,7 +339,7 @@ def run_ours(args, case, desc, ws, rank, local):
                 "algorithmic_bytes_per_launch": bytes_per_launch}
     step_bytes = cells * sum(stage_bytes(cfg, st) + (8.0 * nv * 2) * (cfg.ndims - 1)
                              for st in range(cfg.rk_nstages))
-    forms = ["lanes" if sg in (-8, -16) else ("tile" if sg < 0 else "walker") for sg, _ in tuned]
+    forms = ["lanes" if sg in (-8, -16) else "pairs" for sg, _ in tuned]
     known = FP64_PER_CELL_STEP.get(args.workload, {}) if not args.size else {}
     fw = None
     if known and all(f in known for f in forms):
@@ -367,8 +360,9 @@ def run_ours(args, case, desc, ws, rank, local):
                               "flops_source": "ncu instruction counters of one step, " + fw["captured"]})
     launches_per_step = 0
     for k, (ms_k, n_k) in prof.items():
-        # the viscous group is 5 kernels; a CRWENO5 direction is a solve and a flux kernel
-        per = 5 if k == "viscous" else (2 if k.startswith("hyp") and cfg.hyp_scheme == 1 else 1)
+        # the viscous group is 3 kernels; a CRWENO5 direction the cell fluxes, a solve and
+        # a flux kernel
+        per = 3 if k == "viscous" else (3 if k.startswith("hyp") and cfg.hyp_scheme == 1 else 1)
         launches_per_step += per * n_k
     gpu_launches = launches_per_step  # counted over a pass of as many steps as the timed region
     clocks = clk.summary()

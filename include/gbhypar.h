@@ -251,17 +251,17 @@ int gb_solver_error(gb_solver *s, const double *uex, int layout, int mem, double
  * areas (BoundaryIntegral.c, CalculateConservationError.c). */
 int gb_solver_conservation_begin(gb_solver *s);
 int gb_solver_conservation_error(gb_solver *s, double *err);
-/* Launch shape of the fused kernels: interfaces walked per thread (seg) and
- * threads per block, per direction (values <= 0 keep the current ones); seg = -32,
- * -64 or -128 selects shared-memory tiles of that many interfaces per block (one
- * interface per thread, for small grids; block is then the tile); seg = -8 or -16
- * (Euler1D, component-wise WENO5, no gravity) tiles of that many interfaces with 8
- * lanes per interface, one per reconstruction (for short 1-D lines). */
+/* Launch shape of the fused kernels, per direction (values <= 0 keep the current
+ * ones).  The WENO5 kernels choose the lines and cells of a block by the grid's size;
+ * seg = -32, -64 or -128, or a block below 128, is the most threads a block may take.
+ * Steger-Warming splitting and CRWENO5's flux pass walk seg interfaces per thread in
+ * blocks of `block` threads (Steger-Warming with seg = -32, -64 or -128: tiles of that
+ * many interfaces).  seg = -8 or -16 (Euler1D, component-wise WENO5, no gravity): tiles
+ * of that many interfaces with 16 lanes per interface (for short 1-D lines). */
 int gb_solver_set_launch(gb_solver *s, int dir, int seg, int block);
 int gb_solver_get_launch(gb_solver *s, int dir, int *seg, int *block);
 /* Choose seg/block per direction by timing candidates on `reps` steps of the
- * resident solution (restored afterwards): segment lengths that spread the
- * walk evenly over the SMs in 1..4 waves, and fixed lengths 8..64. */
+ * resident solution (restored afterwards). */
 int gb_solver_autotune(gb_solver *s, int reps);
 /* 1 if every value of the resident interior solution is finite, else 0. */
 int gb_solver_check_finite(gb_solver *s, int *finite);
@@ -292,17 +292,13 @@ int gb_ensemble_set_state(gb_ensemble *e, int member, const double *u, int layou
 int gb_ensemble_get_state(gb_ensemble *e, int member, double *u, int layout, int mem);
 int gb_ensemble_step(gb_ensemble *e, int nsteps);
 double gb_ensemble_time(const gb_ensemble *e);
-/* Launch shape per direction, as gb_solver_set_launch: seg > 0 interfaces walked per
- * thread, seg = -32, -64 or -128 one block per tile of that many interfaces of a
- * member's grid line; 0 keeps the current value.  With a tile form, block = -1
- * selects the persistent work-list kernel (HyPar's ensemble mode,
- * src/TimeIntegration/TimeRK.c:164-170, as one launch per stage and direction of as
- * many blocks as the SMs hold, taking the members' tiles from an atomic counter),
- * block > 0 the grid launch of one block per tile; get_launch reports -1 for the
- * persistent form. */
+/* Launch shape per direction, as gb_solver_set_launch (seg 0 keeps the current value):
+ * one launch per stage and direction over all members (HyPar's ensemble mode,
+ * src/TimeIntegration/TimeRK.c:164-170).  block = -1 with seg = -32, -64 or -128 asked
+ * for a persistent launch; it is accepted and reported, and runs the same blocks. */
 int gb_ensemble_set_launch(gb_ensemble *e, int dir, int seg, int block);
 int gb_ensemble_get_launch(gb_ensemble *e, int dir, int *seg, int *block);
-/* Choose seg/block (walker or tiles) per direction by timing graph-replayed steps
+/* Choose the most threads per block per direction by timing graph-replayed steps
  * (state restored). */
 int gb_ensemble_autotune(gb_ensemble *e, int reps);
 /* CalculateError of one member against its exact solution (as gb_solver_error). */
