@@ -100,6 +100,8 @@ static void rebuild_table(gb_ensemble* e) {
       md.ntrans[d] = ntr;
       int cap = pair_cap_of(e->seg[d], e->block[d]);
       if (cap <= 0) cap = pair_cap(cells);
+      const int most = pair_threads(e->base.model == GB_MODEL_NS3D, e->base.interp == GB_INTERP_CHARACTERISTIC);
+      if (cap > most) cap = most;
       const PairPlan p = pair_plan(md.G.dim[d], ntr, d, cap, true);
       md.L[d] = p.L;
       md.XL[d] = p.XL;

@@ -377,14 +377,13 @@ __device__ __forceinline__ void iface_fp64(const double* __restrict__ U, long lo
   }
 }
 
-// The FP64 evaluation of a block's flagged interfaces by all its threads, for the 1-D and
-// 2-D models: few interfaces lie side by side at a shock, and one thread's chain of some 700
-// dependent FP64 operations takes 20 microseconds, which launches of one or two waves of
-// blocks wait for (shock-entropy line of 20001: 591 -> 437 us for 15 launches; Riemann
-// problem 601x403: 2030 -> 1680 us for 12).  In 3-D the other blocks hide that chain, and
-// this form's registers cost the Taylor-Green 256^3 directions 3 %; there, and with
-// gravity, each thread evaluates its own interface (iface_fp64).  A task is one side of one reconstruction (component-wise) or one field's
-// pair of sides (characteristic); its values go to scr, 4 NV per interface: the pair of
+// The FP64 evaluation of a block's flagged interfaces by all its threads (COOP): few
+// interfaces lie side by side at a shock, and one thread's chain of some 700 dependent FP64
+// operations takes 20 microseconds, which launches of one or two waves of blocks wait for
+// (shock-entropy line of 20001: 591 -> 437 us for 15 launches; Riemann problem 601x403:
+// 2030 -> 1680 us for 12).  With gravity and in the 3-D characteristic form each thread
+// evaluates its own interface (iface_fp64).  A task is one side of one reconstruction
+// (component-wise) or one field's pair of sides (characteristic); its values go to scr, 4 NV per interface: the pair of
 // quantity 2 v + (0: f, 1: u) at 2 (2 v + h).  Then one thread per interface upwinds.
 // Everything is relative to the interface's left cell, as in iface_flux.
 template <int M, bool CHAR>
@@ -571,6 +570,8 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
   using LY = PairLayout<M, CHAR, UPW, ALTW, GRAV>;
   constexpr int NV = LY::NV, ND = LY::ND, NR = LY::NR;
   constexpr bool CC = LY::CC, NEEDC = LY::NEEDC, STATES = LY::STATES;
+  // a block evaluates its flagged interfaces together, else each thread its own
+  constexpr bool COOP = !GRAV && !(M == MODEL_NS3D && CHAR);
   const int T = blockDim.x, S = T + 4, t = threadIdx.x;
   double* sf = sm;
   ff* sd = (ff*)(sf + NV * S);  // rows 0..NV-1: f, NV..2NV-1: u, then the modified solution and g
@@ -972,7 +973,7 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
     if (GRAV && src_dir) ok = ok & (magg * (float)term[0] <= 0.09375f * s0);
   }
   // The differences are read no more: their place takes G and the cells' sums.
-  const int pos = (!GRAV && M != MODEL_NS3D && iface && !ok) ? atomicAdd(cnt, 1) : 0;
+  const int pos = (COOP && iface && !ok) ? atomicAdd(cnt, 1) : 0;
   __syncthreads();
   double* sg = sf + NV * S;
   double* sh = sg + NV * S;
@@ -985,7 +986,7 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
       ss[S + w] = to_double(ffc(1.0 / 12.0) * gse);
     }
   }
-  if (GRAV || M == MODEL_NS3D) {
+  if (!COOP) {
     if (iface && !ok)
       iface_fp64<M, CHAR, UPW, DIR, ALTW, GRAV>(U, line_base(l0 + line), a0 - 3 + q, G, sf, sgf, sgg, S, w, pp, src_dir,
                                                 sg + w, ss + w);
@@ -1087,7 +1088,7 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
 // faster (61.7 and 2.54 ms; shared memory allows three).
 constexpr int PAIR_MINB = 3;
 template <int M, bool CHAR, int UPW, int DIR, bool ALTW, bool GRAV>
-__global__ void __launch_bounds__(256, PAIR_MINB)
+__global__ void __launch_bounds__((M == MODEL_NS3D && !CHAR ? 224 : 256), PAIR_MINB)
 hyp_pair_kernel(const double* __restrict__ U, double* __restrict__ H, const double* __restrict__ dxinv, DevGeom G,
                 PhysParams pp, StageEpi ep, long long ntrans, int L, int XL) {
   extern __shared__ double pair_smem[];
@@ -1099,7 +1100,9 @@ template <int M, bool CHAR, int UPW, int DIR, bool ALTW, bool GRAV>
 cudaError_t launch_pair(const double* U, double* H, const double* dxinv_dir, const DevGeom& G, const PhysParams& pp,
                         const StageEpi& ep, long long ntrans, int cap, cudaStream_t s) {
   const int N = G.dim[DIR];
-  const PairPlan p = pair_plan(N, ntrans, DIR, cap > 0 ? cap : pair_cap(ntrans * N));
+  const int most = pair_threads(M == MODEL_NS3D, CHAR);
+  cap = cap > 0 ? cap : pair_cap(ntrans * N);
+  const PairPlan p = pair_plan(N, ntrans, DIR, cap < most ? cap : most);
   const long long nblk = (ntrans + p.XL - 1) / p.XL * ((N + p.L - 1) / p.L);
   if (nblk > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
   auto k = hyp_pair_kernel<M, CHAR, UPW, DIR, ALTW, GRAV>;
@@ -1111,7 +1114,7 @@ cudaError_t launch_pair(const double* U, double* H, const double* dxinv_dir, con
 
 // Ensemble: the blocks of all members in one launch.
 template <int M, bool CHAR, int UPW, int DIR>
-__global__ void __launch_bounds__(256, PAIR_MINB)
+__global__ void __launch_bounds__((M == MODEL_NS3D && !CHAR ? 224 : 256), PAIR_MINB)
 hyp_batched_pair_kernel(const MemberDev* __restrict__ mem, int nmem, const double* __restrict__ U,
                         double* __restrict__ H, const double* __restrict__ dxinv, PhysParams pp, StageEpi ep) {
   extern __shared__ double pair_smem[];

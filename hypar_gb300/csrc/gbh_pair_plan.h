@@ -35,10 +35,15 @@ inline PairPlan pair_plan(int N, long long nlines, int dir, int cap, bool fixed 
   return best;
 }
 
-// Threads per block: large blocks lose fewer slots, small ones spread a small grid over
-// the 152 SMs.
+// Threads per block: large blocks lose fewer slots, small ones spread a small grid over the
+// 152 SMs.  Euler2D steps with blocks of 64 / 128 / 256: 128^2 121 / 123 / 165 us, 192^2 158 /
+// 157 / 181, 320^2 343 / 331 / 346, 384^2 432 / 419 / 406, 640^2 1096 / 1058 / 989.
 inline int pair_cap(long long cells) { return cells >= 150000 ? 256 : (cells >= 30000 ? 128 : 64); }
 
+// Most threads of a block.  The 3-D component-wise kernels take 224: three such blocks per
+// SM leave 96 registers per thread, which their evaluation of flagged interfaces needs; the
+// others are the faster with 256 and 80 registers (vortex 1024^2 2.25 ms against 2.45).
+inline int pair_threads(bool ns3d, bool chr) { return ns3d && !chr ? 224 : 256; }
 // Threads per block asked for by a launch shape: a tile of t interfaces (seg = -t) or a
 // block below 128 threads is taken as the cap, anything else leaves it to pair_cap (0).
 inline int pair_cap_of(int seg, int block) { return seg <= -32 ? -seg : (block > 0 && block < 128 ? block : 0); }
