@@ -325,7 +325,7 @@ __device__ __forceinline__ void pupwind(const ff* fs6, const ff* fd6, const ff* 
   (void)ND;
 }
 
-// The FP64 evaluation of one interface by its own thread (3-D, gravity) as the correction
+// The FP64 evaluation of one interface by its own thread (gravity, 3-D characteristic) as the correction
 // G, written to G[v S]; with
 // gravity (sgf, sgg: the hydrostatic fields) also the source function's interface values
 // as corrections of its central value, to Gs.  Window: cells i-2 .. i+3 of the line with
@@ -1080,7 +1080,8 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
   }
 }
 
-// Blocks of 256 threads per SM the kernels are held to.  Bound by issue slots and latency
+// Blocks of 256 threads (3-D component-wise: 224, pair_threads) per SM the kernels are held
+// to.  Bound by issue slots and latency
 // (some 6000 mostly FP32 instructions per thread against 75 FP64 ones): two blocks (128
 // registers) left the schedulers idle half of the time; three (80 registers; spills in the
 // FP64 evaluation only) take the Taylor-Green 256^3 directions from 75.9 to 61.4 ms per RK4
