@@ -149,7 +149,7 @@ __device__ __forceinline__ bool cr_weights_pair(ff i1, ff i2, ff i3, ff tau, int
     w2 = m2 * n;
     w3 = m3 * n;
   }
-  return (S.h >= 7.888609e-31f) & (S.h <= 1.0e36f);
+  return sum_in_range(S);
 }
 
 // Grid line `tr` along DIR: offset (in points) of its cell 0.
@@ -715,7 +715,8 @@ cr_flux_kernel(const double* __restrict__ U, double* __restrict__ H, const doubl
       ok = (s0 >= 8.7e-19f) & (s0 <= 1.2e30f) & (sm >= 8.7e-19f) & (sm <= 1.2e30f) & (sE >= 8.7e-19f) & (sE <= 1.2e30f);
 #pragma unroll
       for (int v = 0; v < NV; v++) {
-        ok = ok & (ffma(lam, fabsf(ud6[v].h), fabsf(fd6[v].h)) <= 0.09375f * (v == 0 ? s0 : (v == NV - 1 ? sE : sm)));
+        ok = ok & (ffma(lam, fabsf(ud6[v].h), fabsf(fd6[v].h)) <= 0.09375f * (v == 0 ? s0 : (v == NV - 1 ? sE : sm))) &
+             is_finite(g12[v]);
         fI[v] = fma(0.5, fL[v] + fR[v], to_double(ffc(1.0 / 12.0) * g12[v]));
       }
     }

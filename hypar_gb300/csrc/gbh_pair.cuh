@@ -173,10 +173,11 @@ GBH_HD float d2f_mag(double x) {
   const uint32_t m = shl64hi(H, dlo(x), 3) & 0x7fffffu;
   return e <= 0 ? 0.0f : (e >= (255 << 20) ? u2f(0x7f800000u) : u2f(((uint32_t)e << 3) | m));
 }
+// (Denormals become 0; infinities and NaN stay what they are.)
 GBH_HD double f2d(float a) {
-  const uint32_t b = f2u(a);
-  const uint32_t hi = (((b >> 3) & 0x0fffffffu) + 0x38000000u) | (b & 0x80000000u);
-  return (b & 0x7f800000u) ? mkd(hi, b << 29) : 0.0;
+  const uint32_t b = f2u(a), e = b & 0x7f800000u;
+  const uint32_t hi = (((b >> 3) & 0x0fffffffu) + (e == 0x7f800000u ? 0x70000000u : 0x38000000u)) | (b & 0x80000000u);
+  return e ? mkd(hi, b << 29) : 0.0;
 }
 GBH_HD double to_double(ff a) { return f2d(a.h) + f2d(a.l); }
 
@@ -188,6 +189,8 @@ GBH_HD ff ffc(double c) {
   r.l = (float)(c - (double)r.h);
   return r;
 }
+// (A normalised pair: a NaN of the second word is in the first one too.)
+GBH_HD bool is_finite(ff a) { return fabsf(a.h) <= 3.0e38f; }
 GBH_HD ff ffabs(ff a) { return a.h < 0.0f ? neg(a) : a; }
 GBH_HD ff ffmax(ff a, ff b) { return (a.h > b.h || (a.h == b.h && a.l > b.l)) ? a : b; }
 GBH_HD ff ffsqrt(ff x) { return x * rsqrt(x); }
@@ -321,9 +324,16 @@ GBH_HD ff mapped_weight(ff w, double c) {
   return muluu(muluu(w, num), rcpu(den));
 }
 
+// Whether a sum of sub-stencils' terms is in the range in which pairs keep their precision.
+// The second word is tested too: a smoothness term that overflows leaves 1/B^2 = (0, NaN),
+// which the first word of the sum does not show where another sub-stencil is smooth.
+GBH_HD bool sum_in_range(ff S) {
+  return (S.h >= 7.888609e-31f) & (S.h <= 1.0e36f) & (fabsf(S.l) <= S.h);  // 2^-100; false for NaN
+}
+
 // The weights (w1, w3) of one side from the terms i1, i2, i3 (1/q of the three
 // sub-stencils times 1, 6, 3), tau (4 tau of the side; Borges and Yamaleev-Carpenter).
-// Returns false where the sum leaves the range in which pairs keep their precision.
+// Returns false where the sum leaves its range.
 template <bool ALTW>
 GBH_HD bool side_weights(ff i1, ff i2, ff i3, ff tau, int wtype, ff& w1, ff& w3) {
   if (ALTW && (wtype == PW_BORGES || wtype == PW_YC)) {
@@ -343,7 +353,7 @@ GBH_HD bool side_weights(ff i1, ff i2, ff i3, ff tau, int wtype, ff& w1, ff& w3)
     w1 = muluu(m1, n);
     w3 = muluu(m3, n);
   }
-  return (S.h >= 7.888609e-31f) & (S.h <= 1.0e36f);  // 2^-100; false for NaN
+  return sum_in_range(S);
 }
 
 // The weights of a pair: the farthest upwind sub-stencils' doubled, the downwind ones'.

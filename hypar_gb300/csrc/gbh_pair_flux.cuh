@@ -760,6 +760,7 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
         float mag;
         if (h == 0) {
           mag = weno_mag6(W, t1, t2, t3);
+          ok = ok & (mag <= 3.0e38f);  // (the maxima below drop a NaN)
           if (UPW == UPW_RF) sfd[v * S + w] = weno_dif6(W, t1, t2, t3);
           if (GRAV && (v == 1 + DIR || v == NV - 1)) {
             const ff g = weno_sum6(W, tg1, tg2, tg3);
@@ -774,7 +775,7 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
           }
           *res = weno_sum6(W, t1, t2, t3);
           m0 = v == 0 ? mag : m0;
-          mm = (v > 0 && v < NV - 1 && !(mag <= mm)) ? mag : mm;  // a NaN stays
+          mm = (v > 0 && v < NV - 1) ? fmaxf(mm, mag) : mm;
           mE = v == NV - 1 ? mag : mE;
         } else {
           if (STATES) sum[v * S + w] = pmean(to_pair(su[v * S + w]), *res, d2, d3, weno_sum6(W, t1, t2, t3));
@@ -784,9 +785,10 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
             third_differences(dl, t1, t2, t3);
           }
           mag = weno_mag6(W, t1, t2, t3);
+          ok = ok & (mag <= 3.0e38f);
           *res = weno_dif6(W, t1, t2, t3);
           u0 = v == 0 ? mag : u0;
-          um = (v > 0 && v < NV - 1 && !(mag <= um)) ? mag : um;
+          um = (v > 0 && v < NV - 1) ? fmaxf(um, mag) : um;
           uE = v == NV - 1 ? mag : uE;
         }
       }
@@ -880,21 +882,23 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
           } else {
             sch[v] = weno_sum6(W, tg1, tg2, tg3) * lcol[v];
             const float mg = weno_mag6(W, tg1, tg2, tg3) * fabsf(lcol[v].h) * (v < 2 ? sc01 : 1.0f);
-            magg = !(mg <= magg) ? mg : magg;
+            ok = ok & (mg <= 3.0e38f);
+            magg = fmaxf(magg, mg);
           }
         }
         float mag = weno_mag6(W, t1, t2, t3);
         if (v < 2) mag = mag * sc01;
+        ok = ok & (mag <= 3.0e38f);  // (the maxima below drop a NaN)
         if (h == 0) {
           sx[v * S + w] = weno_sum6(W, t1, t2, t3);
           if (UPW == UPW_RF) sfd[v * S + w] = weno_dif6(W, t1, t2, t3);
-          if (v < 3) ma = !(mag <= ma) ? mag : ma;
-          else ms = !(mag <= ms) ? mag : ms;
+          if (v < 3) ma = fmaxf(ma, mag);
+          else ms = fmaxf(ms, mag);
         } else {
           sx[(NV + v) * S + w] = weno_dif6(W, t1, t2, t3);
           if (STATES) sum[v * S + w] = weno_sum6(W, t1, t2, t3);
-          if (v < 3) ua = !(mag <= ua) ? mag : ua;
-          else us = !(mag <= us) ? mag : us;
+          if (v < 3) ua = fmaxf(ua, mag);
+          else us = fmaxf(us, mag);
         }
       }
     }
@@ -972,6 +976,11 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
          (sE <= 1.2e30f) & (ffma(lam, ua, ma) <= 0.09375f * s0) & (ffma(lam, us, ms) <= 0.09375f * sm1);
     if (GRAV && src_dir) ok = ok & (magg * (float)term[0] <= 0.09375f * s0);
   }
+  // What entered from a term that overflowed or was not finite is NaN here (every result is a
+  // normalised pair).
+#pragma unroll
+  for (int v = 0; v < NV; v++) ok = ok & is_finite(g12[v]);
+  if (GRAV && src_dir) ok = ok & is_finite(gsm) & is_finite(gse);
   // The differences are read no more: their place takes G and the cells' sums.
   const int pos = (COOP && iface && !ok) ? atomicAdd(cnt, 1) : 0;
   __syncthreads();
