@@ -128,7 +128,9 @@ __device__ __forceinline__ bool cr_weights_pair(ff i1, ff i2, ff i3, ff tau, int
     w3 = ffc(0.3);
     return true;
   }
+  bool ok = true;
   if (ALT && (wtype == WENO_W_BORGES || wtype == WENO_W_YC)) {
+    ok = sum_in_range(addu(addu(i1, i2), i3));
     const ff T = sqr(tau), one = {1.0f, 0.0f};
     i1 = T * i1 + one;
     i2 = T * i2 + one;
@@ -149,7 +151,7 @@ __device__ __forceinline__ bool cr_weights_pair(ff i1, ff i2, ff i3, ff tau, int
     w2 = m2 * n;
     w3 = m3 * n;
   }
-  return sum_in_range(S);
+  return ok & sum_in_range(S);
 }
 
 // Grid line `tr` along DIR: offset (in points) of its cell 0.
@@ -712,7 +714,7 @@ cr_flux_kernel(const double* __restrict__ U, double* __restrict__ H, const doubl
       const ff kap = GRAV ? to_pair(fmax(gL, gR)) : zero;
       pupwind<M, UPW, DIR>(fs6, fd6, ud6, um, E, cl, cr, P, g12, lam, rho, Hs, GRAV ? &kap : nullptr);
       const float s0 = rho * lam, sm = s0 * lam, sE = s0 * Hs;
-      ok = (s0 >= 8.7e-19f) & (s0 <= 1.2e30f) & (sm >= 8.7e-19f) & (sm <= 1.2e30f) & (sE >= 8.7e-19f) & (sE <= 1.2e30f);
+      ok = scales_in_range(rho, lam, Hs, GRAV ? kap.h : 1.0f);
 #pragma unroll
       for (int v = 0; v < NV; v++) {
         ok = ok & (ffma(lam, fabsf(ud6[v].h), fabsf(fd6[v].h)) <= 0.09375f * (v == 0 ? s0 : (v == NV - 1 ? sE : sm))) &

@@ -324,11 +324,13 @@ GBH_HD ff mapped_weight(ff w, double c) {
   return muluu(muluu(w, num), rcpu(den));
 }
 
-// Whether a sum of sub-stencils' terms is in the range in which pairs keep their precision.
-// The second word is tested too: a smoothness term that overflows leaves 1/B^2 = (0, NaN),
-// which the first word of the sum does not show where another sub-stencil is smooth.
+// Whether a sum of sub-stencils' terms is in the range in which pairs keep their precision:
+// below 2^-100 its second word has none left, above 2^100 the smoothness terms are so small
+// that eps, or their second words, may lie below what pairs hold.  The second word of the sum
+// is tested too: a smoothness term that overflows leaves 1/B^2 = (0, NaN), which the first
+// word does not show where another sub-stencil is smooth.
 GBH_HD bool sum_in_range(ff S) {
-  return (S.h >= 7.888609e-31f) & (S.h <= 1.0e36f) & (fabsf(S.l) <= S.h);  // 2^-100; false for NaN
+  return (S.h >= 7.888609e-31f) & (S.h <= 1.2676506e30f) & (fabsf(S.l) <= S.h);  // 2^-100, 2^100; false for NaN
 }
 
 // The weights (w1, w3) of one side from the terms i1, i2, i3 (1/q of the three
@@ -336,8 +338,11 @@ GBH_HD bool sum_in_range(ff S) {
 // Returns false where the sum leaves its range.
 template <bool ALTW>
 GBH_HD bool side_weights(ff i1, ff i2, ff i3, ff tau, int wtype, ff& w1, ff& w3) {
+  bool ok = true;
   if (ALTW && (wtype == PW_BORGES || wtype == PW_YC)) {
-    // c_k (1 + T / q_k) with T = (4 tau)^2
+    // c_k (1 + T / q_k) with T = (4 tau)^2; T is off by up to 2^-149, so 1/q_k has to be in
+    // range by itself
+    ok = sum_in_range(addu(addu(i1, i2), i3));
     const ff T = sqr(tau);
     i1 = T * i1 + ff{1.0f, 0.0f};
     i2 = T * i2 + ff{6.0f, 0.0f};
@@ -353,7 +358,7 @@ GBH_HD bool side_weights(ff i1, ff i2, ff i3, ff tau, int wtype, ff& w1, ff& w3)
     w1 = muluu(m1, n);
     w3 = muluu(m3, n);
   }
-  return sum_in_range(S);
+  return ok & sum_in_range(S);
 }
 
 // The weights of a pair: the farthest upwind sub-stencils' doubled, the downwind ones'.

@@ -12,11 +12,11 @@
 // What bounds the error: a pair carries 48 bits, the chain from the differences to G loses
 // two or three of them, so G is off by some 2^-46 of the magnitude of its terms.  Where
 // those terms exceed 2^-7 of the interface's flux scale (rho lam, rho lam^2, rho lam H
-// with lam = |u_n| + a), the scale leaves the range 2^-60 .. 2^100, a weight's sum leaves
-// its own, or anything is not finite, the interface takes the FP64 evaluation
-// (iface_flux) instead: shocks, contacts, under-resolved fields, odd units.  The decision
-// uses the interface's own window only, so every kernel that evaluates an interface takes
-// the same one and neighbouring blocks agree on the flux between them.
+// with lam = |u_n| + a), a scale of the states or the fluxes leaves the range 2^-44 .. 2^100
+// (scales_in_range), a weight's sum leaves its own, or anything is not finite, the interface
+// takes the FP64 evaluation (iface_flux) instead: shocks, contacts, under-resolved fields, odd
+// units.  The decision uses the interface's own window only, so every kernel that evaluates an
+// interface takes the same one and neighbouring blocks agree on the flux between them.
 #pragma once
 
 #include "gbh_pair.cuh"
@@ -27,6 +27,23 @@ namespace gbh {
 struct PEig {
   ff vel[3], un, a, ek, H, hac, rs, gi, lamn;  // gi = (gamma-1)/a^2
 };
+
+// Whether an interface's scales (density, speed, enthalpy) are such that pairs hold its terms:
+// to_pair drops what lies below 2^-103, which has to be below 2^-53 of the states and the
+// fluxes by a margin (2^-44 leaves 2^-6 of it; kap: gravity's factor of the dissipation, on
+// the differences of the modified solution), products of the largest must not overflow, and
+// the eigenvectors' 1/(2a), 1/a^2 need second words above 2^-149.  False for NaN.
+__device__ __forceinline__ bool scales_in_range(float rho, float lam, float H, float kap = 1.0f) {
+  constexpr float LO = 5.684342e-14f, HI = 1.2676506e30f;  // 2^-44, 2^100
+  const float lo = LO * fmaxf(kap, 1.0f), s0 = rho * lam, uE = rho * H, sm = s0 * lam, sE = s0 * H;
+  return (rho >= lo) & (s0 >= lo) & (uE >= lo) & (sm >= LO) & (sE >= LO) & (rho <= HI) & (s0 <= HI) & (uE <= HI) &
+         (sm <= HI) & (sE <= HI) & (lam >= 9.094947e-13f) & (lam <= 1.0995116e12f);  // 2^-40, 2^40
+}
+
+// The same for gravity's source, rt per unit difference of the hydrostatic pressure field.
+__device__ __forceinline__ bool source_in_range(float rt, float lam, float sm, float sE) {
+  return (rt * 5.684342e-14f <= sm) & (rt * lam * 5.684342e-14f <= sE);
+}
 
 // Per-cell ingredients in pairs: sqrt(rho), velocity, enthalpy, wave speed.
 template <int M>
@@ -813,11 +830,10 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
     const float s0 = rho * lam, sm1 = s0 * lam, sE = s0 * Hs;
     ok = ok & (ffma(lam, u0, m0) <= 0.09375f * s0) & (ffma(lam, um, mm) <= 0.09375f * sm1) &
          (ffma(lam, uE, mE) <= 0.09375f * sE);
-    ok = ok & (s0 >= 8.7e-19f) & (s0 <= 1.2e30f) & (sm1 >= 8.7e-19f) & (sm1 <= 1.2e30f) & (sE >= 8.7e-19f) &
-         (sE <= 1.2e30f);
+    ok = ok & scales_in_range(rho, lam, Hs, GRAV ? kap.h : 1.0f);
     if (GRAV && src_dir) {
       const float rt = (float)term[0];
-      ok = ok & (magsm * rt <= 0.09375f * sm1) & (magse * rt * lam <= 0.09375f * sE);
+      ok = ok & (magsm * rt <= 0.09375f * sm1) & (magse * rt * lam <= 0.09375f * sE) & source_in_range(rt, lam, sm1, sE);
     }
   } else {
     PCell<M> cl = cell_of(w), cr = cell_of(w + 1);
@@ -971,10 +987,12 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
     }
     // the fields' strengths are densities (shear: momenta) times a speed for f
     const float s0 = rho * lam, sm1 = s0 * lam;
-    const float sE = s0 * Hs;
-    ok = ok & (s0 >= 8.7e-19f) & (s0 <= 1.2e30f) & (sm1 >= 8.7e-19f) & (sm1 <= 1.2e30f) & (sE >= 8.7e-19f) &
-         (sE <= 1.2e30f) & (ffma(lam, ua, ma) <= 0.09375f * s0) & (ffma(lam, us, ms) <= 0.09375f * sm1);
-    if (GRAV && src_dir) ok = ok & (magg * (float)term[0] <= 0.09375f * s0);
+    ok = ok & scales_in_range(rho, lam, Hs, GRAV ? kap.h : 1.0f) & (ffma(lam, ua, ma) <= 0.09375f * s0) &
+         (ffma(lam, us, ms) <= 0.09375f * sm1);
+    if (GRAV && src_dir) {
+      const float rt = (float)term[0];
+      ok = ok & (magg * rt <= 0.09375f * s0) & source_in_range(rt, lam, sm1, s0 * Hs);
+    }
   }
   // What entered from a term that overflowed or was not finite is NaN here (every result is a
   // normalised pair).
