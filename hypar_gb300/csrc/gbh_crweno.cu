@@ -700,7 +700,7 @@ cr_flux_kernel(const double* __restrict__ U, double* __restrict__ H, const doubl
     if constexpr (UPW != UPW_SWFS) {
       const ff six = {6.0f, 0.0f}, zero = {0.0f, 0.0f};
       ff fs6[NV], fd6[NV], ud6[NV], um[NV], g12[NV];
-      float lam, rho, Hs;
+      float lam, rho, Hs, alm;
 #pragma unroll
       for (int v = 0; v < NV; v++) {
         fs6[v] = zero;
@@ -712,12 +712,12 @@ cr_flux_kernel(const double* __restrict__ U, double* __restrict__ H, const doubl
       PEig E;
       if (CC) E = peig<M, DIR>(cl, cr, P);
       const ff kap = GRAV ? to_pair(fmax(gL, gR)) : zero;
-      pupwind<M, UPW, DIR>(fs6, fd6, ud6, um, E, cl, cr, P, g12, lam, rho, Hs, GRAV ? &kap : nullptr);
+      pupwind<M, UPW, DIR>(fs6, fd6, ud6, um, E, cl, cr, P, g12, lam, rho, Hs, alm, GRAV ? &kap : nullptr);
       const float s0 = rho * lam, sm = s0 * lam, sE = s0 * Hs;
       ok = scales_in_range(rho, lam, Hs, GRAV ? kap.h : 1.0f);
 #pragma unroll
       for (int v = 0; v < NV; v++) {
-        ok = ok & (ffma(lam, fabsf(ud6[v].h), fabsf(fd6[v].h)) <= 0.09375f * (v == 0 ? s0 : (v == NV - 1 ? sE : sm))) &
+        ok = ok & (ffma(alm, fabsf(ud6[v].h), fabsf(fd6[v].h)) <= 0.09375f * (v == 0 ? s0 : (v == NV - 1 ? sE : sm))) &
              is_finite(g12[v]);
         fI[v] = fma(0.5, fL[v] + fR[v], to_double(ffc(1.0 / 12.0) * g12[v]));
       }

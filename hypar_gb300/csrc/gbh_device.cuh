@@ -124,37 +124,6 @@ __device__ __forceinline__ void cell_flux(const Prim<M>& q, double* f) {
   f[NV - 1] = (q.e + q.P) * vn;
 }
 
-// The same with the momenta in the place of density times velocity (rho |v|^2 = m . v, the
-// mass flux m_DIR): seven FP64 operations per cell fewer in 3-D, equal up to rounding.
-template <int M>
-__device__ __forceinline__ Prim<M> to_prim_mom(const double* u, const PhysParams& pp) {
-  constexpr int ND = ModelTraits<M>::ND, NV = ModelTraits<M>::NV;
-  Prim<M> q;
-  q.rho = u[0];
-  q.rinv = nr_rcp(q.rho);
-  q.e = u[NV - 1];
-  double mv = 0.0;
-#pragma unroll
-  for (int k = 0; k < 3; k++) q.vel[k] = 0.0;
-#pragma unroll
-  for (int k = 0; k < ND; k++) {
-    double v = u[1 + k] * q.rinv;
-    if (M == MODEL_NS3D) v = (q.rho == 0.0) ? 0.0 : v;
-    q.vel[k] = v;
-    mv = k == 0 ? u[1] * v : fma(u[1 + k], v, mv);
-  }
-  q.P = fma(-0.5, mv, q.e) * pp.gm1;
-  return q;
-}
-template <int M, int DIR>
-__device__ __forceinline__ void cell_flux_mom(const Prim<M>& q, double mn, double* f) {
-  constexpr int ND = ModelTraits<M>::ND, NV = ModelTraits<M>::NV;
-  f[0] = mn;
-#pragma unroll
-  for (int k = 0; k < ND; k++) f[1 + k] = k == DIR ? fma(mn, q.vel[k], q.P) : mn * q.vel[k];
-  f[NV - 1] = (q.e + q.P) * q.vel[DIR];
-}
-
 // UFunction value of the energy component: NavierStokes3D recomputes it
 // (NavierStokes3DModifiedSolution.c:56-65, gravity fields = 1); Euler1D
 // (gravity field exp(0) = 1) and Euler2D (no UFunction) leave u unchanged.

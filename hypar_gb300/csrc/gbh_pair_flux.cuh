@@ -10,13 +10,17 @@
 // numbers, whose arithmetic has 64 times the FP64 pipe's throughput on GB300.
 //
 // What bounds the error: a pair carries 48 bits, the chain from the differences to G loses
-// two or three of them, so G is off by some 2^-46 of the magnitude of its terms.  Where
-// those terms exceed 2^-7 of the interface's flux scale (rho lam, rho lam^2, rho lam H
-// with lam = |u_n| + a), a scale of the states or the fluxes leaves the range 2^-44 .. 2^100
-// (scales_in_range), a weight's sum leaves its own, or anything is not finite, the interface
-// takes the FP64 evaluation (iface_flux) instead: shocks, contacts, under-resolved fields, odd
-// units.  The decision uses the interface's own window only, so every kernel that evaluates an
-// interface takes the same one and neighbouring blocks agree on the flux between them.
+// two or three of them, so G is off by some 2^-46 of the magnitude of its terms.  The
+// interface takes the FP64 evaluation (iface_flux) instead where
+//   - its terms exceed a bound times its flux scale (rho lam, rho lam^2, rho lam H with
+//     lam = |u_n| + a; pair_bound, dissipation terms at the dissipation's own speed),
+//   - what the characteristic projections add up exceeds one (proj_bound): a field may cancel
+//     out of large differences, their rounding does not,
+//   - a scale of the states or the fluxes leaves the range 2^-44 .. 2^100 (scales_in_range), a
+//     weight's sum leaves its own, or anything is not finite:
+// shocks, contacts, under-resolved fields, odd units.  The decision uses the interface's own
+// window only, so every kernel that evaluates an interface takes the same one and neighbouring
+// blocks agree on the flux between them.
 #pragma once
 
 #include "gbh_pair.cuh"
@@ -27,6 +31,19 @@ namespace gbh {
 struct PEig {
   ff vel[3], un, a, ek, H, hac, rs, gi, lamn;  // gi = (gamma-1)/a^2
 };
+
+// Bounds of an interface's terms (12 x their share of its flux scale) and of its projections'.
+// Set so that a right-hand side is no further from one in extended precision than that of
+// the FP64 kernels: over waves of 6 to 100 cells and noise of 0.1 to 8 %, root mean square in
+// units of 2^-53 of the flux scale over the spacing, 1-D 0.22-0.63 (FP64 kernels 0.27-0.63),
+// 2-D 0.20-0.51 (0.21-0.51), 3-D component-wise 0.23-0.40 (0.44-0.57; there 2^-7 is enough),
+// 3-D characteristic 0.31-0.60 (0.45-0.73).  With 2^-7 and without the projections' bound a
+// wave of 6 cells was 0.67 off for 0.37.  Time: Euler2D ensemble 16.9 -> 20.2 ms, the other
+// workloads within 3 %.
+__host__ __device__ constexpr float pair_bound(int model, bool chr) {
+  return 12.0f * (model == MODEL_NS3D ? (chr ? 0.001953125f : 0.0078125f) : 0.0009765625f);  // 2^-9, 2^-7, 2^-10
+}
+__host__ __device__ constexpr float proj_bound(int model) { return model == MODEL_NS3D ? 3.0e38f : 0.5f; }
 
 // Whether an interface's scales (density, speed, enthalpy) are such that pairs hold its terms:
 // to_pair drops what lies below 2^-103, which has to be below 2^-53 of the states and the
@@ -251,12 +268,13 @@ __device__ __forceinline__ void pfield(ff l, ff c, ff r, ff& al, float& sg) {
 // G of one interface times 12 from the conserved sums and differences of the
 // reconstructions (fs6 = 6 (fL + fR - 2 central), fd6 = 6 (fR - fL), ud6 = 6 (uR - uL)),
 // mean states um where the scheme averages the reconstructed states, and the cells'
-// ingredients.  lam, rho, H: the interface's scales.  kappa: gravity's factor of the
-// dissipation.
+// ingredients.  lam, rho, H: the interface's scales; alm: the largest dissipation speed, which
+// may exceed lam by far (the entropy fix, Euler1D's Rusanov speed, gravity).  kappa: gravity's
+// factor of the dissipation.
 template <int M, int UPW, int DIR>
 __device__ __forceinline__ void pupwind(const ff* fs6, const ff* fd6, const ff* ud6, const ff* um, const PEig& Ecc,
                                         const PCell<M>& cl, const PCell<M>& cr, const PParams& q, ff* g12, float& lam,
-                                        float& rho, float& Hs, const ff* kappa = nullptr) {
+                                        float& rho, float& Hs, float& alm, const ff* kappa = nullptr) {
   constexpr int NV = ModelTraits<M>::NV, ND = ModelTraits<M>::ND;
   constexpr bool STATES = (UPW == UPW_ROE && M == MODEL_EULER2D) ||
                           ((UPW == UPW_LLF || UPW == UPW_RF) && M != MODEL_EULER1D);
@@ -291,7 +309,7 @@ __device__ __forceinline__ void pupwind(const ff* fs6, const ff* fd6, const ff* 
     const ff avg = (M == MODEL_EULER1D ? sqr(E.a) : E.a) + ffabs(E.un);
     ff al = ffmax(ffmax(cl.c, cr.c), avg);
     if (kappa) al = al * *kappa;
-    lam = fmaxf(lam, al.h);
+    alm = al.h;
 #pragma unroll
     for (int v = 0; v < NV; v++) g12[v] = fs6[v] - al * ud6[v];
     return;
@@ -313,8 +331,8 @@ __device__ __forceinline__ void pupwind(const ff* fs6, const ff* fd6, const ff* 
       c0 = c0 * *kappa;
       c1 = c1 * *kappa;
       c2 = c2 * *kappa;
-      lam = fmul(lam, kappa->h);
     }
+    alm = fmaxf(c0.h, c1.h);
     pdissip<M, DIR>(E, q, ud6, c0, c1, c2, y);
 #pragma unroll
     for (int v = 0; v < NV; v++) g12[v] = fs6[v] - y[v];
@@ -329,7 +347,8 @@ __device__ __forceinline__ void pupwind(const ff* fs6, const ff* fd6, const ff* 
 #pragma unroll
     for (int k = 0; k < 3; k++) al[k] = al[k] * *kappa;
   }
-  lam = fmaxf(lam, fmaxf(al[0].h, al[1].h));
+  alm = fmaxf(al[0].h, fmaxf(al[1].h, al[2].h));
+  if (UPW == UPW_RF) alm = fmaxf(alm, lam);  // fields taken from one side count f's terms twice
   pdissip<M, DIR>(E, q, ud6, al[0], al[1], al[2], y);
 #pragma unroll
   for (int v = 0; v < NV; v++) g12[v] = fs6[v] - y[v];
@@ -342,10 +361,10 @@ __device__ __forceinline__ void pupwind(const ff* fs6, const ff* fd6, const ff* 
   (void)ND;
 }
 
-// The FP64 evaluation of one interface by its own thread (gravity, 3-D characteristic) as the correction
-// G, written to G[v S]; with
-// gravity (sgf, sgg: the hydrostatic fields) also the source function's interface values
-// as corrections of its central value, to Gs.  Window: cells i-2 .. i+3 of the line with
+// The FP64 evaluation of one interface by its own thread (gravity, 3-D characteristic): its
+// flux less the left cell's, written to G[v S]; with gravity (sgf, sgg: the hydrostatic
+// fields) also the source function's interface values as corrections of its central value,
+// to Gs.  Window: cells i-2 .. i+3 of the line with
 // base point pb (states from memory), own cell = slot w (fluxes in shared memory).
 template <int M, bool CHAR, int UPW, int DIR, bool ALTW, bool GRAV>
 __device__ __forceinline__ void iface_fp64(const double* __restrict__ U, long long pb, int i, const DevGeom& geo,
@@ -381,11 +400,7 @@ __device__ __forceinline__ void iface_fp64(const double* __restrict__ U, long lo
   ep.tape = nullptr;
   iface_flux<M, CHAR, UPW, DIR, ALTW, GRAV, false>(wu, wf, wuc, wgf, wgg, ax, pp, ep, 4.0 * pp.eps, src_dir, 0, fI, SI);
 #pragma unroll
-  for (int v = 0; v < NV; v++) {
-    const double d1 = wf[2][v] - wf[1][v], d2 = wf[3][v] - wf[2][v], d3 = wf[4][v] - wf[3][v];
-    // without gravity fI is relative to the left cell's flux
-    G[v * S] = (GRAV ? fI[v] - wf[2][v] : fI[v]) - fma(6.0, d2, d1 - d3) * (1.0 / 12.0);
-  }
+  for (int v = 0; v < NV; v++) G[v * S] = GRAV ? fI[v] - wf[2][v] : fI[v];
   if (GRAV && src_dir) {
     const double d1 = wgg[2] - wgg[1], d2 = wgg[3] - wgg[2], d3 = wgg[4] - wgg[3];
     const double c = fma(6.0, d2, d1 - d3) * (1.0 / 12.0);
@@ -500,11 +515,13 @@ __device__ __forceinline__ void fp64_upwind(const double* __restrict__ U, long l
   if (CHAR) upwind_char<M, UPW, DIR>(fL, fR, uL, uR, E, cl, cr, pp, fI, 1.0, u2, f2);
   else upwind_iface<M, false, UPW, DIR>(fL, fR, uL, uR, E, cl, cr, pp, fI, 1.0, u2, f2);
 #pragma unroll
-  for (int v = 0; v < NV; v++) {
-    const double* f = sf + v * S + w;
-    const double d1 = f[0] - f[-1], d2 = f[1] - f[0], d3 = f[2] - f[1];
-    G[v * S] = fI[v] - fma(6.0, d2, d1 - d3) * (1.0 / 12.0);
-  }
+  for (int v = 0; v < NV; v++) G[v * S] = fI[v];
+}
+
+// The fourth-order central value of the interface to the right of slot f[0], less f[0].
+__device__ __forceinline__ double central_rel(const double* f) {
+  const double d1 = f[0] - f[-1], d2 = f[1] - f[0], d3 = f[2] - f[1];
+  return fma(6.0, d2, d1 - d3) * (1.0 / 12.0);
 }
 
 // stage_epilogue of NB values at once: all reads are issued before the first write, so
@@ -589,6 +606,7 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
   constexpr bool CC = LY::CC, NEEDC = LY::NEEDC, STATES = LY::STATES;
   // a block evaluates its flagged interfaces together, else each thread its own
   constexpr bool COOP = !GRAV && !(M == MODEL_NS3D && CHAR);
+  constexpr float BOUND = pair_bound(M, CHAR), PROJ_BOUND = proj_bound(M);
   const int T = blockDim.x, S = T + 4, t = threadIdx.x;
   double* sf = sm;
   ff* sd = (ff*)(sf + NV * S);  // rows 0..NV-1: f, NV..2NV-1: u, then the modified solution and g
@@ -655,8 +673,9 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
     double uu[NV], fv[NV];
 #pragma unroll
     for (int v = 0; v < NV; v++) uu[v] = su[v * S + w];
-    const Prim<M> pr = to_prim_mom<M>(uu, pp);
-    cell_flux_mom<M, DIR>(pr, uu[1 + DIR], fv);
+    const Prim<M> pr = to_prim<M>(uu, pp);
+    cell_flux<M, DIR>(pr, fv);
+    fv[0] = uu[1 + DIR];
 #pragma unroll
     for (int v = 0; v < NV; v++) sf[v * S + w] = fv[v];
     if (GRAV) {
@@ -714,7 +733,7 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
   const bool own = line < nl && q >= 3 && q <= Lc + 2;
   bool ok = true;
   ff g12[NV];
-  float lam, rho, Hs;
+  float lam, rho, Hs, alm;
   auto cell_of = [&](int x) {
     PCell<M> c;
     c.t = c.H = c.c = ff{1.0f, 0.0f};
@@ -826,14 +845,14 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
       cr = cell_of(w + 1);
     }
     if (CC) Ecc = peig<M, DIR>(cl, cr, P);
-    pupwind<M, UPW, DIR>(fs6, fd6, ud6, us, Ecc, cl, cr, P, g12, lam, rho, Hs, GRAV ? &kap : nullptr);
+    pupwind<M, UPW, DIR>(fs6, fd6, ud6, us, Ecc, cl, cr, P, g12, lam, rho, Hs, alm, GRAV ? &kap : nullptr);
     const float s0 = rho * lam, sm1 = s0 * lam, sE = s0 * Hs;
-    ok = ok & (ffma(lam, u0, m0) <= 0.09375f * s0) & (ffma(lam, um, mm) <= 0.09375f * sm1) &
-         (ffma(lam, uE, mE) <= 0.09375f * sE);
+    ok = ok & (ffma(alm, u0, m0) <= BOUND * s0) & (ffma(alm, um, mm) <= BOUND * sm1) &
+         (ffma(alm, uE, mE) <= BOUND * sE);
     ok = ok & scales_in_range(rho, lam, Hs, GRAV ? kap.h : 1.0f);
     if (GRAV && src_dir) {
       const float rt = (float)term[0];
-      ok = ok & (magsm * rt <= 0.09375f * sm1) & (magse * rt * lam <= 0.09375f * sE) & source_in_range(rt, lam, sm1, sE);
+      ok = ok & (magsm * rt <= BOUND * sm1) & (magse * rt * lam <= BOUND * sE) & source_in_range(rt, lam, sm1, sE);
     }
   } else {
     PCell<M> cl = cell_of(w), cr = cell_of(w + 1);
@@ -847,9 +866,22 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
     }
     // Per unit of g, the source function's terms; 6 x the terms of fields 0-2, of the shear
     // fields, of f, of u (the largest of each).
-    float ma = 0.0f, ms = 0.0f, ua = 0.0f, us = 0.0f, magg = 0.0f;
+    float ma = 0.0f, ms = 0.0f, ua = 0.0f, us = 0.0f, magg = 0.0f, pf = 0.0f, pu = 0.0f;
     const float sc01 = M == MODEL_EULER1D ? Ecc.rs.h : 1.0f;
     const ff gh = P.gm1 * Ecc.hac, ah = Ecc.a * Ecc.hac;
+    // The magnitude of what a face's projections add up, in densities: a field may cancel out of
+    // it (an entropy jump leaves no sound), its rounding does not.
+    const float i2a = ah.h * sc01;
+    auto terms = [&](const ff* y) {
+      float s = ffma(Ecc.ek.h, fabsf(y[0].h), fabsf(y[(NV - 1) * S].h)), m = 0.0f;
+#pragma unroll
+      for (int e = 0; e < ND; e++) {
+        const float ve = fabsf(Ecc.vel[e].h), ye = fabsf(y[(1 + e) * S].h);
+        s = ffma(ve, ye, s);
+        m = fadd(ffma(ve, fabsf(y[0].h), ye), m);
+      }
+      return ffma(i2a, m, ffma(Ecc.gi.h, s, fabsf(y[0].h)));
+    };
 #pragma unroll 1
     for (int h = 0; h < 2; h++) {
       // the projections' common parts at the five faces: s/(gamma-1) times (gamma-1) hac, t hac
@@ -879,6 +911,14 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
           if (h) parts(xc + k, gc[GRAV ? k : 0], tc[GRAV ? k : 0]);
         }
       }
+      float p1, p2, p3;  // of the third differences
+      {
+        const ff* y = GRAV && h ? xc : x;
+        const float q0 = terms(y), q1 = terms(y + 1), q2 = terms(y + 2), q3 = terms(y + 3), q4 = terms(y + 4);
+        p1 = q0 + 2.0f * q1 + q2;
+        p2 = q1 + 2.0f * q2 + q3;
+        p3 = q2 + 2.0f * q3 + q4;
+      }
       // one field at a time (unrolled only with gravity, which keeps values per field): the
       // unrolled loop's code does not fit the instruction cache
 #pragma unroll(GRAV ? NV : 1)
@@ -905,12 +945,16 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
         float mag = weno_mag6(W, t1, t2, t3);
         if (v < 2) mag = mag * sc01;
         ok = ok & (mag <= 3.0e38f);  // (the maxima below drop a NaN)
+        const float w2 = h == 0 ? W.r3.h - W.l3.h : W.r3.h + W.l3.h - 1.0f;
+        const float proj = ffma(W.r1.h, p3, ffma(W.l1.h, p1, fabsf(w2) * p2));
         if (h == 0) {
+          pf = fmaxf(pf, proj);
           sx[v * S + w] = weno_sum6(W, t1, t2, t3);
           if (UPW == UPW_RF) sfd[v * S + w] = weno_dif6(W, t1, t2, t3);
           if (v < 3) ma = fmaxf(ma, mag);
           else ms = fmaxf(ms, mag);
         } else {
+          pu = fmaxf(pu, proj);
           sx[(NV + v) * S + w] = weno_dif6(W, t1, t2, t3);
           if (STATES) sum[v * S + w] = weno_sum6(W, t1, t2, t3);
           if (v < 3) ua = fmaxf(ua, mag);
@@ -936,14 +980,12 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
         const ff avg = (M == MODEL_EULER1D ? sqr(Ecc.a) : Ecc.a) + ffabs(Ecc.un);
         lm[0] = lm[1] = lm[2] = ffmax(ffmax(cl.c, cr.c), avg);
         if (GRAV) lm[0] = lm[1] = lm[2] = lm[0] * kap;
-        lam = fmaxf(lam, lm[0].h);
       } else if (UPW == UPW_ROE) {
 #pragma unroll
         for (int k = 0; k < 3; k++) {
           lm[k] = M == MODEL_EULER1D ? ffabs(lm[k]) : pharten(lm[k]);
           if (GRAV) lm[k] = lm[k] * kap;
         }
-        if (GRAV) lam = fmul(lam, kap.h);
       } else {
         const ff cv = cl.vel[DIR], rv = cr.vel[DIR];
         pfield<UPW>(cv - cl.c, lm[0], rv - cr.c, lm[0], sg[0]);
@@ -953,8 +995,9 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
 #pragma unroll
           for (int k = 0; k < 3; k++) lm[k] = lm[k] * kap;
         }
-        lam = fmaxf(lam, fmaxf(lm[0].h, lm[1].h));
       }
+      alm = fmaxf(lm[0].h, fmaxf(lm[1].h, lm[2].h));
+      if (UPW == UPW_RF) alm = fmaxf(alm, lam);  // fields taken from one side count f's terms twice
 #pragma unroll
       for (int k = 0; k < NV; k++) {
         const int m = k < 2 ? k : 2;
@@ -983,15 +1026,15 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
         const ff* dd = sd + (NV + v) * S + w;
         um[v] = pmean(to_pair(su[v * S + w]), dd[0], dd[0] - dd[-1], dd[1] - dd[0], us6[v]);
       }
-      pupwind<M, UPW, DIR>(fs6, fd6, ud6, um, Ecc, cl, cr, P, g12, lam, rho, Hs);
+      pupwind<M, UPW, DIR>(fs6, fd6, ud6, um, Ecc, cl, cr, P, g12, lam, rho, Hs, alm);
     }
     // the fields' strengths are densities (shear: momenta) times a speed for f
     const float s0 = rho * lam, sm1 = s0 * lam;
-    ok = ok & scales_in_range(rho, lam, Hs, GRAV ? kap.h : 1.0f) & (ffma(lam, ua, ma) <= 0.09375f * s0) &
-         (ffma(lam, us, ms) <= 0.09375f * sm1);
+    ok = ok & scales_in_range(rho, lam, Hs, GRAV ? kap.h : 1.0f) & (ffma(alm, ua, ma) <= BOUND * s0) &
+         (ffma(alm, us, ms) <= BOUND * sm1) & (ffma(alm, pu, pf) <= PROJ_BOUND * s0);
     if (GRAV && src_dir) {
       const float rt = (float)term[0];
-      ok = ok & (magg * rt <= 0.09375f * s0) & source_in_range(rt, lam, sm1, s0 * Hs);
+      ok = ok & (magg * rt <= BOUND * s0) & source_in_range(rt, lam, sm1, s0 * Hs);
     }
   }
   // What entered from a term that overflowed or was not finite is NaN here (every result is a
@@ -1005,6 +1048,9 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
   double* sg = sf + NV * S;
   double* sh = sg + NV * S;
   double* ss = sh + NV * S;  // gravity: the source function's corrections, momentum and energy
+  int* list = CHAR ? (int*)sx : (int*)sr;  // the slots evaluated in FP64 (in a free place)
+  int* fp64 = list + 2 * S;                // per slot: whether its interface is
+  fp64[w] = iface && !ok;
   if (iface && ok) {
 #pragma unroll
     for (int v = 0; v < NV; v++) sg[v * S + w] = to_double(mulu(ffc(1.0 / 12.0), g12[v]));
@@ -1018,7 +1064,6 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
       iface_fp64<M, CHAR, UPW, DIR, ALTW, GRAV>(U, line_base(l0 + line), a0 - 3 + q, G, sf, sgf, sgg, S, w, pp, src_dir,
                                                 sg + w, ss + w);
   } else if (const int nbad = *cnt) {
-    int* list = CHAR ? (int*)sx : (int*)sr;  // their slots (in a free place)
     if (iface && !ok) list[pos] = w;
     __syncthreads();
     constexpr int NT = Fp64Tasks<M, CHAR>::N;
@@ -1047,7 +1092,7 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
 #pragma unroll
       for (int v = 0; v < NV; v++) {
         const double* f = sf + v * S + w;
-        Fb[v] = fma(7.0, f[0] + f[1], -(f[-1] + f[2])) * (1.0 / 12.0) + sg[v * S + w];
+        Fb[v] = (ok ? fma(7.0, f[0] + f[1], -(f[-1] + f[2])) * (1.0 / 12.0) : f[0]) + sg[v * S + w];
       }
       boundary_flux<NV>(ep, I, N, l0 + line, ntrans, Fb);
     }
@@ -1055,11 +1100,21 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
   __syncthreads();
   if (own) {
     const double dxi = dxinv[G.g + a0 - 3 + q], c1 = dxi * (2.0 / 3.0), c2 = dxi * (-1.0 / 12.0);
+    const bool fr = fp64[w], fl = fp64[w - 1];
 #pragma unroll
     for (int v = 0; v < NV; v++) {
       const double* f = sf + v * S + w;
-      const double c4 = fma(c1, f[1] - f[-1], (f[2] - f[-2]) * c2);
-      double h = fma(dxi, sg[v * S + w] - sg[v * S + w - 1], c4);
+      const double g1 = sg[v * S + w], g0 = sg[v * S + w - 1];
+      double h;
+      if (fr | fl) {
+        // beside an interface evaluated in FP64 the fluxes may jump: both relative to their left
+        // cells, as in the FP64 kernels, where the central difference would round the jump
+        const double D1 = fr ? g1 : central_rel(f) + g1, D0 = fl ? g0 : central_rel(f - 1) + g0;
+        h = dxi * ((f[0] - f[-1]) + (D1 - D0));
+      } else {
+        const double c4 = fma(c1, f[1] - f[-1], (f[2] - f[-2]) * c2);
+        h = fma(dxi, g1 - g0, c4);
+      }
       if (GRAV && src_dir && (v == 1 + DIR || v == NV - 1)) {
         const int k = v == 1 + DIR ? 0 : 1;
         const double* g = sgg + w;
