@@ -618,7 +618,8 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
   ff* sfd = sum + (STATES ? NV * S : 0);
   double* sgf = (double*)(sx + LY::NRES * S);
   double* sgg = sgf + S;
-  const bool src_dir = GRAV && pp.grav[DIR] != 0.0 && (ep.mode != EPI_HYP || ep.with_source);
+  const bool grav_dir = GRAV && pp.grav[DIR] != 0.0;
+  const bool src_dir = grav_dir && (ep.mode != EPI_HYP || ep.with_source);
   const int N = G.dim[DIR], LL = L + 6;
   const long long sdir = G.stride[DIR];
   const int lo = G.bclo[DIR], hi = G.bchi[DIR];
@@ -850,7 +851,7 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
     ok = ok & (ffma(alm, u0, m0) <= BOUND * s0) & (ffma(alm, um, mm) <= BOUND * sm1) &
          (ffma(alm, uE, mE) <= BOUND * sE);
     ok = ok & scales_in_range(rho, lam, Hs, GRAV ? kap.h : 1.0f);
-    if (GRAV && src_dir) {
+    if (grav_dir) {  // asked for or not, so that both evaluations take the same form
       const float rt = (float)term[0];
       ok = ok & (magsm * rt <= BOUND * sm1) & (magse * rt * lam <= BOUND * sE) & source_in_range(rt, lam, sm1, sE);
     }
@@ -1032,7 +1033,7 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
     const float s0 = rho * lam, sm1 = s0 * lam;
     ok = ok & scales_in_range(rho, lam, Hs, GRAV ? kap.h : 1.0f) & (ffma(alm, ua, ma) <= BOUND * s0) &
          (ffma(alm, us, ms) <= BOUND * sm1) & (ffma(alm, pu, pf) <= PROJ_BOUND * s0);
-    if (GRAV && src_dir) {
+    if (grav_dir) {
       const float rt = (float)term[0];
       ok = ok & (magg * rt <= BOUND * s0) & source_in_range(rt, lam, sm1, s0 * Hs);
     }
@@ -1041,7 +1042,7 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
   // normalised pair).
 #pragma unroll
   for (int v = 0; v < NV; v++) ok = ok & is_finite(g12[v]);
-  if (GRAV && src_dir) ok = ok & is_finite(gsm) & is_finite(gse);
+  if (grav_dir) ok = ok & is_finite(gsm) & is_finite(gse);
   // The differences are read no more: their place takes G and the cells' sums.
   const int pos = (COOP && iface && !ok) ? atomicAdd(cnt, 1) : 0;
   __syncthreads();
