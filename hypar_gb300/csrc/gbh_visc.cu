@@ -103,10 +103,15 @@ visc_q_kernel(const double* __restrict__ u, double* __restrict__ Q, const double
     R[d * n + p] = pv;
     vm = fadd(vm, fabsf(pv.h));
   }
-  const float h = fmaxf(d2f_mag(dxinv[G.g + i]), fmaxf(d2f_mag(dxinv[ng0 + G.g + j]), d2f_mag(dxinv[ng0 + ng1 + G.g + k])));
-  const float t = d2f_mag(T), r = d2f_mag(rho), mu = exp2f(0.76f * log2f(t));
-  const bool ok = (T > 0.0) & (mu * d2f_mag(vp.inv_Re) * h <= 0.03125f * r * sqrtf(t)) & (t >= 1e-18f) & (t <= 1e18f) &
-                  (r >= 1e-18f) & (vm <= 1e18f) & (h <= 1e18f);
+  const float h0 = d2f_mag(dxinv[G.g + i]), h1 = d2f_mag(dxinv[ng0 + G.g + j]), h2 = d2f_mag(dxinv[ng0 + ng1 + G.g + k]);
+  const float h = fmaxf(h0, fmaxf(h1, h2)), hmin = fminf(h0, fminf(h1, h2));
+  const float t = d2f_mag(T), r = d2f_mag(rho), ire = d2f_mag(vp.inv_Re), mu = exp2f(0.76f * log2f(t));
+  // rho and 1/h in 2^-24 .. 2^24, a^2 in 2^-20 .. 2^40, |v| up to 2^24: the divergence of the
+  // energy flux, up to rho a |v|^2 / h / 4, stays below 2^120, and 2^-59 of rho a^3 / h above
+  // 2^-149, where second words end
+  const bool ok = (T > 0.0) & (mu * ire * h <= 0.03125f * r * sqrtf(t)) & (t >= 9.5367432e-7f) &
+                  (t <= 1.0995116e12f) & (r >= 5.9604645e-8f) & (r <= 1.6777216e7f) & (vm <= 1.6777216e7f) &
+                  (hmin >= 5.9604645e-8f) & (h <= 1.6777216e7f) & (ire >= 8.6736174e-19f);
   if (!ok) *flag = id;
 }
 
