@@ -112,7 +112,10 @@ visc_q_kernel(const double* __restrict__ u, double* __restrict__ Q, const double
   const bool ok = (T > 0.0) & (mu * ire * h <= 0.03125f * r * sqrtf(t)) & (t >= 9.5367432e-7f) &
                   (t <= 1.0995116e12f) & (r >= 5.9604645e-8f) & (r <= 1.6777216e7f) & (vm <= 1.6777216e7f) &
                   (hmin >= 5.9604645e-8f) & (h <= 1.6777216e7f) & (ire >= 8.6736174e-19f);
-  if (!ok) *flag = id;
+  // points off the interior in two directions enter no derivative (visc_flux), and boundaries
+  // applied in memory leave them unset
+  const int outside = (i < 0 || i >= G.dim[0]) + (j < 0 || j >= G.dim[1]) + (k < 0 || k >= G.dim[2]);
+  if (!ok && outside < 2) *flag = id;
 }
 
 // Fourth-order first derivative of one Q component at position i of a line of

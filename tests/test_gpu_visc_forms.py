@@ -68,3 +68,17 @@ def test_forms_of_the_periodic_box(built_lib, tmp_path):
     case.Re = 0.5
     rhs, ref = terms(case, tmp_path / "b")
     assert np.array_equal(rhs, ref)  # FP64
+
+
+@pytest.mark.parametrize("wall", ["slip-wall", "noslip-wall"])
+@pytest.mark.parametrize("dims", [(0, 1), (1, 2), (0, 1, 2)], ids=["duct-z", "duct-x", "box"])
+def test_forms_between_walls(built_lib, tmp_path, dims, wall):
+    """Walls in two or three directions: the edges' ghost points, which no wall fills, do not
+    decide the form."""
+    case = C.tgv(12, n_iter=1, perturb=0.05)
+    case.bcs = {(d, f): (wall, [0.0, 0.0, 0.0]) for d in dims for f in (1, -1)}
+    rhs, ref = terms(case, tmp_path)
+    assert np.isfinite(rhs).all()
+    assert not np.array_equal(rhs, ref)  # pairs
+    tol = 2.0 * 2.0 ** -53 * flux_scale(case)
+    assert (np.abs(rhs - ref).max(0) <= tol).all(), np.abs(rhs - ref).max(0) / tol
