@@ -45,7 +45,7 @@ cudaError_t launch_interp_euler2d(int, int, int, int, double*, const double*, co
 cudaError_t launch_interp_ns3d(int, int, int, int, double*, const double*, const double*, const DevGeom&,
                                const PhysParams&, cudaStream_t);
 cudaError_t launch_visc(const double*, double*, double*, double*, const double*, const DevGeom&,
-                        const ViscParams&, int*, int, cudaStream_t);
+                        const ViscParams&, int*, cudaStream_t);
 cudaError_t launch_bc_zone(double*, const DevGeom&, int, const int*, const double*, double, cudaStream_t);
 cudaError_t launch_bc_zone_t(double*, const DevGeom&, int, const int*, const double*, double, const double*, int, int,
                              cudaStream_t);
@@ -309,7 +309,7 @@ static int rhs_launches(gb_solver* s, double* U, StageEpi ep, double t) {
   ep.par = nullptr;
   if (s->viscous) {
     int pr = prof_begin(s, GB_PROF_VISC);
-    CK(launch_visc(U, s->d_Q, s->d_Gr, s->d_par, s->d_dxinv, s->G, s->vp, s->d_vflag, ++s->visc_id, s->stream));
+    CK(launch_visc(U, s->d_Q, s->d_Gr, s->d_par, s->d_dxinv, s->G, s->vp, s->d_vflag, s->stream));
     prof_end(s, pr);
     ep.par = s->d_par;
   }
@@ -539,8 +539,8 @@ extern "C" int gb_solver_create(const gb_config* cfg, const double* dxinv, int d
   if (s->viscous) {
     A(&s->d_Q, (size_t)st * 7 * sizeof(double));
     A(&s->d_Gr, (size_t)st * 9 * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&s->d_vflag, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(s->d_vflag, 0, sizeof(int));
+    if (e == cudaSuccess) e = cudaMalloc((void**)&s->d_vflag, 2 * sizeof(int));
+    if (e == cudaSuccess) e = cudaMemset(s->d_vflag, 0, 2 * sizeof(int));
   }
   A(&s->d_dxinv, off * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc((void**)&s->d_flag, sizeof(int));
@@ -1006,7 +1006,7 @@ extern "C" int gb_ParabolicFunction(double* par, double* u, void* sv, void* m, d
   CK(cudaMemsetAsync(par, 0, s->nvals * sizeof(double), s->stream));
   if (!s->viscous) return GB_OK;
   // the term by itself: FP64 throughout (the pairs are for its sum with the convective one)
-  CK(launch_visc(u, s->d_Q, s->d_Gr, par, s->d_dxinv, s->G, s->vp, nullptr, 0, s->stream));
+  CK(launch_visc(u, s->d_Q, s->d_Gr, par, s->d_dxinv, s->G, s->vp, nullptr, s->stream));
   return GB_OK;
 }
 

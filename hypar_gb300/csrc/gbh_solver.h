@@ -42,7 +42,6 @@ struct gb_solver {
   std::vector<int> mem_zones;  // zone indices applied in memory before each RHS
   gbh::HypLaunch hl[3];
   int* d_vflag = nullptr;  // the viscous term's refusal of the float pairs (launch_visc)
-  int visc_id = 0;         // counts its evaluations
   double t = 0.0;
   // HyPar's stage / step hooks (include/hypar.h:334-341), installed with
   // gb_solver_set_hooks and called on the host by every fused step

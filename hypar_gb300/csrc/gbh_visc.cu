@@ -65,11 +65,13 @@ __device__ __forceinline__ ff pow076_pair(double T) {
 // Arrays of one component each, n points: doubles u, v, w, T, then pairs u, v, w.
 enum { VQ_T = 3, VQ_PAIR = 4 };
 
-// At all points including ghosts; ghost points read through the fold.  *flag takes `id`
-// where the pairs' bound fails.
+// At all points including ghosts; ghost points read through the fold.  flag[0] is set where the
+// pairs' bound fails; visc_flux copies it to flag[1], which visc_div reads while it clears
+// flag[0] for the next evaluation: no kernel reads what another thread of it writes, every
+// evaluation starts from its own points alone, and a captured one does so at each replay.
 __global__ void __launch_bounds__(256)
 visc_q_kernel(const double* __restrict__ u, double* __restrict__ Q, const double* __restrict__ dxinv, DevGeom G,
-              ViscParams vp, int* __restrict__ flag, int id) {
+              ViscParams vp, int* __restrict__ flag) {
   pdl_wait();
   const int ng0 = G.dim[0] + 2 * G.g, ng1 = G.dim[1] + 2 * G.g, ng2 = G.dim[2] + 2 * G.g;
   const long long n = (long long)ng0 * ng1 * ng2;
@@ -115,7 +117,7 @@ visc_q_kernel(const double* __restrict__ u, double* __restrict__ Q, const double
   // points off the interior in two directions enter no derivative (visc_flux), and boundaries
   // applied in memory leave them unset
   const int outside = (i < 0 || i >= G.dim[0]) + (j < 0 || j >= G.dim[1]) + (k < 0 || k >= G.dim[2]);
-  if (!ok && outside < 2) *flag = id;
+  if (!ok && outside < 2) flag[0] = 1;
 }
 
 // Fourth-order first derivative of one Q component at position i of a line of
@@ -231,8 +233,10 @@ __device__ __forceinline__ void visc_flux_at(const double* __restrict__ Q, doubl
 // Points off the interior in one direction carry the flux along it only, two deep.
 __global__ void __launch_bounds__(256)
 visc_flux_kernel(const double* __restrict__ Q, double* __restrict__ F, const double* __restrict__ dxinv, DevGeom G,
-                 ViscParams vp, const int* __restrict__ flag, int id) {
+                 ViscParams vp, int* flag) {
   pdl_wait();
+  const bool refused = !flag || flag[0];
+  if (flag && blockIdx.x == 0 && threadIdx.x == 0) flag[1] = refused;
   const int ng[3] = {G.dim[0] + 2 * G.g, G.dim[1] + 2 * G.g, G.dim[2] + 2 * G.g};
   const long long n = (long long)ng[0] * ng[1] * ng[2];
   const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -250,7 +254,7 @@ visc_flux_kernel(const double* __restrict__ Q, double* __restrict__ F, const dou
   if (outside > 1 || !reach) return;
   const bool on[3] = {in[1] && in[2], in[0] && in[2], in[0] && in[1]};
   const double di[3] = {dxinv[G.g + idx[0]], dxinv[ng[0] + G.g + idx[1]], dxinv[ng[0] + ng[1] + G.g + idx[2]]};
-  if (flag && *flag != id) visc_flux_at<ff>(Q, F, G, vp, di, n, p, idx, on);
+  if (!refused) visc_flux_at<ff>(Q, F, G, vp, di, n, p, idx, on);
   else visc_flux_at<double>(Q, F, G, vp, di, n, p, idx, on);
 }
 
@@ -283,8 +287,10 @@ __device__ __forceinline__ void visc_div_at(const double* __restrict__ F0, doubl
 
 __global__ void __launch_bounds__(256)
 visc_div_kernel(const double* __restrict__ F, double* __restrict__ par, const double* __restrict__ dxinv, DevGeom G,
-                ViscParams vp, const int* __restrict__ flag, int id) {
+                ViscParams vp, int* flag) {
   pdl_wait();
+  const bool refused = !flag || flag[1];
+  if (flag && blockIdx.x == 0 && threadIdx.x == 0) flag[0] = 0;
   const long long m = (long long)G.dim[0] * G.dim[1] * G.dim[2];
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= m) return;
@@ -296,23 +302,23 @@ visc_div_kernel(const double* __restrict__ F, double* __restrict__ par, const do
   const double di[3] = {dxinv[G.g + i], dxinv[ng0 + G.g + j], dxinv[ng0 + ng1 + G.g + k]};
   double out[5];
   out[0] = 0.0;
-  if (flag && *flag != id) visc_div_at<ff>(F, out, G, vp, di, n, p);
+  if (!refused) visc_div_at<ff>(F, out, G, vp, di, n, p);
   else visc_div_at<double>(F, out, G, vp, di, n, p);
 #pragma unroll
   for (int v = 0; v < 5; v++) par[p * 5 + v] = out[v];
 }
 
-// flag, id: where the pairs may be used, a device integer and a value it does not hold
-// yet (visc_q stores it there to refuse them); nullptr: FP64 throughout.
+// flag: where the pairs may be used, two device integers, the first one 0; nullptr: FP64
+// throughout.
 cudaError_t launch_visc(const double* u, double* Q, double* F, double* par, const double* dxinv, const DevGeom& G,
-                        const ViscParams& vp, int* flag, int id, cudaStream_t s) {
+                        const ViscParams& vp, int* flag, cudaStream_t s) {
   const long long n = (long long)(G.dim[0] + 2 * G.g) * (G.dim[1] + 2 * G.g) * (G.dim[2] + 2 * G.g);
   const long long m = (long long)G.dim[0] * G.dim[1] * G.dim[2];
   if (vp.order == 2) flag = nullptr;
   const unsigned gn = (unsigned)((n + 255) / 256), gm = (unsigned)((m + 255) / 256);
-  if (cudaError_t e = launch_pdl(visc_q_kernel, gn, 256, 0, s, u, Q, dxinv, G, vp, flag, id)) return e;
-  if (cudaError_t e = launch_pdl(visc_flux_kernel, gn, 256, 0, s, Q, F, dxinv, G, vp, flag, id)) return e;
-  return launch_pdl(visc_div_kernel, gm, 256, 0, s, F, par, dxinv, G, vp, flag, id);
+  if (cudaError_t e = launch_pdl(visc_q_kernel, gn, 256, 0, s, u, Q, dxinv, G, vp, flag)) return e;
+  if (cudaError_t e = launch_pdl(visc_flux_kernel, gn, 256, 0, s, Q, F, dxinv, G, vp, flag)) return e;
+  return launch_pdl(visc_div_kernel, gm, 256, 0, s, F, par, dxinv, G, vp, flag);
 }
 
 // ---------------------------------------------------------------------------
