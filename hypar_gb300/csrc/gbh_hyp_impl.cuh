@@ -882,6 +882,7 @@ hyp_lane_kernel(const double* __restrict__ U, double* __restrict__ H, const doub
   __shared__ double sfI[TI][NV];
   __shared__ Eig secc[TI];
   pdl_wait();
+  pdl_launch();
   const int I0 = (int)blockIdx.x * TC;
   const int N = G.dim[0];
   const long long sd = G.stride[0];

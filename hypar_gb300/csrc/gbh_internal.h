@@ -12,15 +12,16 @@
 
 namespace gbh {
 
-// Programmatic dependent launch: the blocks of the next kernel of the stream are placed
-// (and wait in pdl_wait) while this one's last blocks still run, which hides most of the
-// few microseconds between the short launches of a stage.  A kernel launched by
-// launch_pdl calls pdl_wait before it touches memory: it returns when the kernel before
-// it has finished and its writes are visible.
-__device__ __forceinline__ void pdl_wait() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
+// Programmatic dependent launch: the launch of the next kernel of the stream overlaps this
+// one.  A kernel launched by launch_pdl calls pdl_wait before it touches memory: it returns
+// when the kernel before it has finished and its writes are visible.  The next kernel's blocks
+// are placed (and wait) when every block of this one has called pdl_launch or ended.  Only the
+// short kernels of one wave call it (boundary zones, lane groups): blocks placed while others
+// still run share the SMs that were free first, two or three to an SM where others hold none.
+// Called at the start of the float-pair and viscous kernels it took turbulence of 32^3 from
+// 1.66 to 2.40 ms per step, of 24^3 from 0.93 to 1.30, the bubble 32^3 from 416 to 476 us.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <typename... P, typename... A>
 cudaError_t launch_pdl(void (*k)(P...), unsigned grid, int block, size_t smem, cudaStream_t s, A... args) {
   cudaLaunchConfig_t c = {};

@@ -409,6 +409,7 @@ __device__ __forceinline__ void bc_ghost(const ZoneDev& z, const double* w, doub
 
 __global__ void bc_zone_kernel(double* u, DevGeom G, int nv, ZoneDev z) {
   pdl_wait();
+  pdl_launch();
   int b[3] = {1, 1, 1};
   for (int d = 0; d < G.nd; d++) b[d] = z.ie[d] - z.is[d];
   long long n = (long long)b[0] * b[1] * b[2];
