@@ -43,7 +43,7 @@ struct PEig {
 __host__ __device__ constexpr float pair_bound(int model, bool chr) {
   return 12.0f * (model == MODEL_NS3D ? (chr ? 0.001953125f : 0.0078125f) : 0.0009765625f);  // 2^-9, 2^-7, 2^-10
 }
-__host__ __device__ constexpr float proj_bound(int model) { return model == MODEL_NS3D ? 3.0e38f : 0.5f; }
+__host__ __device__ constexpr float proj_bound(int model) { return model == MODEL_NS3D ? 3.0e38f : 1.0f; }
 
 // Whether an interface's scales (density, speed, enthalpy) are such that pairs hold its terms:
 // to_pair drops what lies below 2^-103, which has to be below 2^-53 of the states and the
@@ -490,6 +490,40 @@ __device__ __forceinline__ void fp64_task(const double* __restrict__ U, long lon
     wpair<ALTW, true>(x, x, eps4, pp.wtype, oL, oR);
     scr[2 * task] = oL;
     scr[2 * task + 1] = oR;
+  }
+}
+
+// The same for every field of one quantity (characteristic): a block with many flagged
+// interfaces takes these, which project a cell once instead of once per field (half the FP64
+// operations; noise of 20 % on 512^2, Euler2D: 7.1 -> 4.8 ms per step).  The operations on a
+// value are the same, and its bits.
+template <int M, int DIR, bool ALTW>
+__device__ __forceinline__ void fp64_fields(const double* su, const double* sf, int S, int w, int isu,
+                                            const PhysParams& pp, double* scr) {
+  constexpr int NV = ModelTraits<M>::NV;
+  double u2[NV], u3[NV], x[NV][6];
+#pragma unroll
+  for (int v = 0; v < NV; v++) {
+    u2[v] = su[v * S + w];
+    u3[v] = su[v * S + w + 1];
+  }
+  const Eig E = roe_eig<M, DIR>(roe_side<M>(to_prim<M>(u2, pp)), roe_side<M>(to_prim<M>(u3, pp)), pp);
+  const double* q = isu ? su : sf;
+#pragma unroll
+  for (int p = 0; p < 6; p++) {
+    double d[NV], y[NV];
+#pragma unroll
+    for (int e = 0; e < NV; e++) d[e] = q[e * S + w - 2 + p] - q[e * S + w];
+    if (p != 2) projL<M, DIR>(E, pp, d, y);
+#pragma unroll
+    for (int v = 0; v < NV; v++) x[v][p] = p == 2 ? 0.0 : y[v];
+  }
+#pragma unroll
+  for (int v = 0; v < NV; v++) {
+    double oL, oR;
+    wpair<ALTW, true>(x[v], x[v], 4.0 * pp.eps, pp.wtype, oL, oR);
+    scr[4 * v + 2 * isu] = oL;
+    scr[4 * v + 2 * isu + 1] = oR;
   }
 }
 
@@ -1071,7 +1105,13 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
     const int batch = S / 4;  // NV S values of scratch
     for (int base = 0; base < nbad; base += batch) {
       const int m = nbad - base < batch ? nbad - base : batch;
-      for (int k = t; k < m * NT; k += T) {
+      // characteristic: whole quantities where the single fields would take more than two rounds
+      const bool whole = CHAR && m * NT > 2 * T;
+      if constexpr (CHAR) {
+        for (int k = t; whole && k < m * 2; k += T)
+          fp64_fields<M, DIR, ALTW>(su, sf, S, list[base + (k >> 1)], k & 1, pp, sh + (k >> 1) * 4 * NV);
+      }
+      for (int k = t; !whole && k < m * NT; k += T) {
         const int it = k / NT, x = list[base + it], l = x / LL;
         fp64_task<M, CHAR, UPW, DIR, ALTW>(U, line_base(l0 + l), a0 - 3 + x - l * LL, G, sf, S, x, k - it * NT, pp,
                                            sh + it * 4 * NV);
