@@ -941,7 +941,7 @@ struct gb_adjoint {
   gb_config cfg;
   DevGeom G;
   PhysParams pp;
-  HypLaunch hl[2];
+  HypLaunch hl[2];  // of the taped steps; the others take the float pairs
   int vjp_seg[2] = {8, 8};
   int vjp_block = 128;
   int device = 0;
@@ -1099,8 +1099,8 @@ static int adj_step(gb_adjoint* a, cudaStream_t strm, const double* uin, double*
       if (e.tape && a->tape_w == TAPE_WIDE)
         AK(launch_hyp_euler2d_wide_tape(d, U, a->H, a->d_dxinv + a->dx_off[d], a->G, a->pp, e, a->hl[d], strm));
       else
-        AK(launch_hyp_euler2d(d, c.interp, c.upwind, U, a->H, a->d_dxinv + a->dx_off[d], a->G, a->pp, e, a->hl[d],
-                              strm));
+        AK(launch_hyp_euler2d(d, c.interp, c.upwind, U, a->H, a->d_dxinv + a->dx_off[d], a->G, a->pp, e,
+                              e.tape ? a->hl[d] : HypLaunch(), strm));
     }
     for (int t = st + 1; t < ns; t++)
       if (ep.ca[t] != 0.0) touched[t] = 1;
@@ -1337,7 +1337,8 @@ extern "C" int gb_adjoint_sync(gb_adjoint* a) {
 extern "C" int gb_adjoint_set_launch(gb_adjoint* a, int which, int seg, int block) {
   if (!a || which < 0 || which > 3) { gbh_set_error("gb_adjoint_set_launch: bad argument"); return GB_ERR_ARG; }
   if (which < 2) {
-    if (seg > 0 || seg == -32 || seg == -64 || seg == -128) a->hl[which].seg = seg;  // -t: tiles of t interfaces
+    // -t: tiles of t interfaces; the float-pair shapes of a solver leave the tapes' form alone
+    if ((seg > 0 && seg < GB_SEG_AUTO) || seg == -32 || seg == -64 || seg == -128) a->hl[which].seg = seg;
     if (block > 0) {
       if (block % 32 || block > 128) { gbh_set_error("block must be a multiple of 32, at most 128"); return GB_ERR_ARG; }
       a->hl[which].block = block;

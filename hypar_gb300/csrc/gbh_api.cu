@@ -497,10 +497,6 @@ extern "C" int gb_solver_create(const gb_config* cfg, const double* dxinv, int d
   s->vp.inv_Re = 1.0 / Re_eff;
   s->vp.inv_Pr = 1.0 / c.Pr;
   s->vp.order = c.par_scheme == 2 ? 2 : 4;
-  for (int d = 0; d < 3; d++) {
-    s->hl[d].seg = 32;
-    s->hl[d].block = 128;
-  }
   long long off = 0;
   for (int d = 0; d < c.ndims; d++) {
     s->dx_off[d] = off;
@@ -838,11 +834,14 @@ extern "C" int gb_solver_get_launch(gb_solver* s, int dir, int* seg, int* block)
 }
 
 // Launch-shape autotuner: each candidate is timed on `reps` steps of the resident
-// solution, which is restored afterwards.  The float-pair kernels take the most threads
-// per block from the shape (pair_cap_of); the FP64 ones (gravity, Steger-Warming, CRWENO5)
-// walk segments, where an even spread over the SMs (a partial last wave idles SMs) stands
-// against the per-segment overhead (a six-cell window warm-up and one extra interface):
-// segment lengths that give 1..4 full waves of 4 warps per SM, plus fixed lengths.
+// solution, which is restored afterwards.  The float-pair kernels first, with blocks of the
+// grid's size, 64 and 128 threads.  The FP64 kernels are the faster where most interfaces
+// leave the pairs' bound (3-D turbulence of 24^3: tiles 0.93 ms per step against 1.30) and up
+// to six times slower elsewhere, so one of their tiles and one of their walkers are tried, and
+// the rest only where one of the two is within three times the best pair form.  Walkers spread
+// evenly over the SMs (a partial last wave idles SMs) against the per-segment overhead (a
+// six-cell window warm-up and one extra interface): segment lengths that give 1..4 full waves
+// of 4 warps per SM, plus fixed lengths.
 extern "C" int gb_solver_autotune(gb_solver* s, int reps) {
   if (!s) { gbh_set_error("null solver"); return GB_ERR_ARG; }
   if (reps < 1) reps = 1;
@@ -871,58 +870,71 @@ extern "C" int gb_solver_autotune(gb_solver* s, int reps) {
     long long ntrans = 1;
     for (int e = 0; e < c.ndims; e++)
       if (e != d) ntrans *= c.dim[e];
-    std::vector<int> segs;
     const bool pairs = c.hyp_scheme == GB_SCHEME_WENO5 && c.upwind != UPW_SWFS;
-    for (int w = 1; w <= 4 && !pairs; w++) {
+    // no tiles with gravity or CRWENO5
+    const bool tiles = !s->gravity && c.hyp_scheme == GB_SCHEME_WENO5;
+    float best = 1e30f;
+    HypLaunch bestL = s->hl[d];
+    // Times one shape; a tile's block is the tile.
+    auto timed = [&](int seg, int block) {
+      double ms[GB_PROF_CLASSES] = {};
+      long long nl[GB_PROF_CLASSES];
+      s->hl[d].seg = seg;
+      s->hl[d].block = block;
+      // every candidate on the same solution: the float pairs' time depends on it
+      if (!rc && cudaMemcpyAsync(s->d_u, save, bytes, cudaMemcpyDeviceToDevice, s->stream) != cudaSuccess) {
+        gbh_set_error("gb_solver_autotune: restoring the solution failed");
+        rc = GB_ERR_CUDA;
+      }
+      s->t = t0;
+      if (!rc) rc = gbh_rk_step(s);  // warm
+      if (!rc) rc = gb_solver_profile(s, 1);
+      for (int r = 0; r < reps && !rc; r++) rc = gbh_rk_step(s);
+      if (!rc) rc = gb_solver_profile_read(s, ms, nl);
+      const float t = rc ? 1e30f : (float)ms[GB_PROF_HYP_X + d];
+      if (t < best) {
+        best = t;
+        bestL = s->hl[d];
+      }
+      return t;
+    };
+    std::vector<int> segs;
+    for (int w = 1; w <= 4; w++) {
       double lanes = (double)w * sms * 4 * 32;
       long long nseg = (long long)(lanes / (double)ntrans + 0.5);
       if (nseg < 1) nseg = 1;
-      int sg = (int)((N + nseg - 1) / nseg);
-      segs.push_back(sg);
+      segs.push_back((int)((N + nseg - 1) / nseg));
     }
-    if (pairs) segs = {32, -128};  // (32, 128): by the grid's size; (32, 64): 64; -128: 128
-    else
-      for (int sg : {8, 16, 24, 32, 48, 64}) segs.push_back(sg);
+    bool fp64 = true;
+    if (pairs) {
+      for (int cap : {0, 64, 128}) timed(GB_SEG_AUTO + cap, 128);
+      const float pair = best;
+      best /= 1.1f;  // another form rounds differently: not for less than a tenth
+      // lane groups of 8 / 16 interfaces (Euler1D component-wise: short lines)
+      if (!s->gravity && c.model == GB_MODEL_EULER1D && c.interp == GB_INTERP_COMPONENTS)
+        for (int ti : {8, 16}) timed(-ti, 128);
+      float probe = timed(segs[0], 128);
+      if (tiles) probe = std::min(probe, timed(N < 32 ? -32 : -64, 128));
+      fp64 = probe <= 3.0f * pair;
+    } else if (c.hyp_scheme == GB_SCHEME_CRWENO5) {
+      timed(GB_SEG_AUTO, 128);
+    }
+    for (int sg : {8, 16, 24, 32, 48, 64}) segs.push_back(sg);
     // Small grids (at most four waves of 4 warps per SM at one interface per
     // thread) cannot fill the SMs with long segments: there, also 1-3
     // interfaces per thread and 32-thread blocks, spreading the few threads
     // over more SMs at the price of recomputing the segments' first interfaces.
-    const bool small = !pairs && (double)ntrans * N <= 4.0 * sms * 4 * 32;
+    const bool small = (double)ntrans * N <= 4.0 * sms * 4 * 32;
     if (small)
       for (int sg : {1, 2, 3}) segs.push_back(sg);
     std::vector<int> blocks = {128, 64};
     if (small) blocks.push_back(32);
-    // shared-memory tiles of 32 / 64 / 128 interfaces (seg = -tile; not with gravity
-    // or CRWENO5, whose kernels have no tile form)
-    if (!pairs && !s->gravity && c.hyp_scheme == GB_SCHEME_WENO5)
-      for (int ti : {32, 64, 128}) segs.push_back(-ti);
-    // lane groups of 8 / 16 interfaces (Euler1D component-wise: short lines)
-    if (!s->gravity && c.hyp_scheme == GB_SCHEME_WENO5 && c.model == GB_MODEL_EULER1D &&
-        c.interp == GB_INTERP_COMPONENTS)
-      for (int ti : {8, 16}) segs.push_back(-ti);
-    double best = 1e30;
-    HypLaunch bestL = s->hl[d];
     for (int sg : segs) {
-      if (!pairs && sg > 0 && (sg < (small ? 1 : 4) || sg > N)) continue;
-      if (!pairs && sg < 0 && -sg > 2 * (N + 1)) continue;
-      for (int blk : blocks) {
-        if (sg < 0 && blk != blocks[0]) continue;  // a tile's block is the tile
-        s->hl[d].seg = sg;
-        s->hl[d].block = blk;
-        rc = gbh_rk_step(s);  // warm
-        if (!rc) rc = gb_solver_profile(s, 1);
-        for (int r = 0; r < reps && !rc; r++) rc = gbh_rk_step(s);
-        double ms[GB_PROF_CLASSES];
-        long long nl[GB_PROF_CLASSES];
-        if (!rc) rc = gb_solver_profile_read(s, ms, nl);
-        if (rc) break;
-        if (ms[GB_PROF_HYP_X + d] < best) {
-          best = ms[GB_PROF_HYP_X + d];
-          bestL = s->hl[d];
-        }
-      }
-      if (rc) break;
+      if (!fp64 || sg < (small ? 1 : 4) || sg > N) continue;
+      for (int blk : blocks) timed(sg, blk);
     }
+    for (int ti : {32, 64, 128})
+      if (fp64 && tiles && ti <= 2 * (N + 1)) timed(-ti, 128);
     s->hl[d] = bestL;
   }
   gb_solver_profile(s, prof_was ? 1 : 0);

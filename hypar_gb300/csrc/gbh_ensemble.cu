@@ -6,10 +6,10 @@
 // All members share the model, schemes, time step and Butcher table (as in the
 // reference, where they share solver.inp); sizes, boundaries and initial data
 // are per member.  Their arrays are concatenated; every Runge-Kutta stage is
-// one launch per direction over all members (each block finds its member in a
-// table of block offsets), and a whole step is captured once in a CUDA graph
-// and replayed.  The launch shape (segment length, tile, block) sets the most threads
-// per block (pair_cap_of).
+// one launch per direction over all members (each block, or a walker's thread, finds its
+// member in a table of offsets), and a whole step is captured once in a CUDA graph and
+// replayed.  The form per direction -- float pairs (the default), FP64 segment walkers, FP64
+// tiles in a grid or a persistent launch -- is set by gb_ensemble_set_launch.
 #include <algorithm>
 #include <cstring>
 #include <vector>
@@ -19,11 +19,14 @@
 
 namespace gbh {
 cudaError_t launch_batched_euler1d(int, int, int, const MemberDev*, int, long long, int, const double*, double*,
-                                   const double*, const PhysParams&, const StageEpi&, cudaStream_t);
+                                   const double*, const PhysParams&, const StageEpi&, const HypLaunch&,
+                                   unsigned long long*, cudaStream_t);
 cudaError_t launch_batched_euler2d(int, int, int, const MemberDev*, int, long long, int, const double*, double*,
-                                   const double*, const PhysParams&, const StageEpi&, cudaStream_t);
+                                   const double*, const PhysParams&, const StageEpi&, const HypLaunch&,
+                                   unsigned long long*, cudaStream_t);
 cudaError_t launch_batched_ns3d(int, int, int, const MemberDev*, int, long long, int, const double*, double*,
-                                const double*, const PhysParams&, const StageEpi&, cudaStream_t);
+                                const double*, const PhysParams&, const StageEpi&, const HypLaunch&,
+                                unsigned long long*, cudaStream_t);
 cudaError_t launch_pack(double*, const double*, const DevGeom&, int, int, cudaStream_t);
 }  // namespace gbh
 
@@ -53,10 +56,13 @@ struct gb_ensemble {
   double* d_stage = nullptr;
   size_t stage_vals = 0;
   long long total_vals = 0, total_dx = 0;
-  long long total_blk[3] = {0, 0, 0};
-  int threads[3] = {0, 0, 0};  // per block: the largest of the members' shapes
-  int seg[3] = {32, 32, 32}, block[3] = {128, 128, 128};
-  bool persist[3] = {false, false, false};  // block = -1 was asked for (the same blocks)
+  long long total[3] = {0, 0, 0};  // blocks, or the walkers' threads
+  int threads[3] = {0, 0, 0};  // pairs: per block, the largest of the members' shapes
+  HypLaunch hl[3];
+  // tile forms only: the persistent work-list kernel (one counter per stage and
+  // direction, cleared at the start of every step) instead of one block per tile
+  bool persist[3] = {false, false, false};
+  unsigned long long* d_ctr = nullptr;
   double* d_u = nullptr;
   double* d_acc = nullptr;
   double* d_P[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -84,21 +90,31 @@ static void rebuild_table(gb_ensemble* e) {
     cells += n;
   }
   for (int d = 0; d < 3; d++) {
-    e->total_blk[d] = 0;
+    e->total[d] = 0;
     e->threads[d] = 0;
   }
   for (int m = 0; m < e->nm; m++) {
     MemberDev& md = e->mem[m];
     for (int d = 0; d < 3; d++) {
-      md.start[d] = e->total_blk[d];
+      const int seg = e->hl[d].seg;
+      md.start[d] = e->total[d];
       md.ntrans[d] = 0;
       md.L[d] = md.XL[d] = 1;
+      md.seg[d] = seg;
+      md.nseg[d] = 0;
       if (d >= e->base.ndims) continue;
       long long ntr = 1;
       for (int k = 0; k < e->base.ndims; k++)
         if (k != d) ntr *= md.G.dim[k];
       md.ntrans[d] = ntr;
-      int cap = pair_cap_of(e->seg[d], e->block[d]);
+      if (!e->hl[d].pairs()) {
+        // walker: threads (segments x lines); tiles: blocks (tiles x lines)
+        const int ti = -seg;
+        md.nseg[d] = seg > 0 ? (md.G.dim[d] + seg - 1) / seg : (md.G.dim[d] + ti - 2) / (ti - 1);
+        e->total[d] += ntr * md.nseg[d];
+        continue;
+      }
+      int cap = e->hl[d].cap();
       if (cap <= 0) cap = pair_cap(cells);
       const int most = pair_threads(e->base.model == GB_MODEL_NS3D, e->base.interp == GB_INTERP_CHARACTERISTIC);
       if (cap > most) cap = most;
@@ -106,7 +122,7 @@ static void rebuild_table(gb_ensemble* e) {
       md.L[d] = p.L;
       md.XL[d] = p.XL;
       if (p.T > e->threads[d]) e->threads[d] = p.T;
-      e->total_blk[d] += (ntr + p.XL - 1) / p.XL * ((md.G.dim[d] + p.L - 1) / p.L);
+      e->total[d] += (ntr + p.XL - 1) / p.XL * ((md.G.dim[d] + p.L - 1) / p.L);
     }
   }
 }
@@ -121,15 +137,15 @@ static int upload_table(gb_ensemble* e) {
 
 static cudaError_t launch_dir(gb_ensemble* e, int st, int d, const double* U, const StageEpi& ep) {
   const gb_config& c = e->base;
-  (void)st;
-  if (c.model == GB_MODEL_EULER1D)
-    return launch_batched_euler1d(d, c.interp, c.upwind, e->d_mem, e->nm, e->total_blk[d], e->threads[d], U, e->d_H,
-                                  e->d_dx, e->pp, ep, e->stream);
-  if (c.model == GB_MODEL_EULER2D)
-    return launch_batched_euler2d(d, c.interp, c.upwind, e->d_mem, e->nm, e->total_blk[d], e->threads[d], U, e->d_H,
-                                  e->d_dx, e->pp, ep, e->stream);
-  return launch_batched_ns3d(d, c.interp, c.upwind, e->d_mem, e->nm, e->total_blk[d], e->threads[d], U, e->d_H,
-                             e->d_dx, e->pp, ep, e->stream);
+  const HypLaunch& L = e->hl[d];
+  unsigned long long* ctr = (L.seg < 0 && e->persist[d]) ? e->d_ctr + 3 * st + d : nullptr;
+  // one block per tile
+  if (L.seg < 0 && !ctr && e->total[d] > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+  auto launch = c.model == GB_MODEL_EULER1D   ? launch_batched_euler1d
+                : c.model == GB_MODEL_EULER2D ? launch_batched_euler2d
+                                              : launch_batched_ns3d;
+  return launch(d, c.interp, c.upwind, e->d_mem, e->nm, e->total[d], e->threads[d], U, e->d_H, e->d_dx, e->pp, ep, L,
+                ctr, e->stream);
 }
 
 // The launches of one Runge-Kutta step (ns stages x ndims directions).
@@ -137,6 +153,8 @@ static int step_launches(gb_ensemble* e) {
   const gb_config& c = e->base;
   const int ns = c.rk_nstages;
   int touched[4] = {0, 0, 0, 0};
+  if (e->persist[0] || e->persist[1] || e->persist[2])
+    CK(cudaMemsetAsync(e->d_ctr, 0, sizeof(unsigned long long) * 12, e->stream));
   for (int st = 0; st < ns; st++) {
     double* U = (st == 0 || !touched[st]) ? e->d_u : e->d_P[st];
     StageEpi ep;
@@ -267,6 +285,7 @@ extern "C" int gb_ensemble_create(const gb_config* cfgs, const double* const* dx
   if (e->base.ndims > 1) A(&e->d_H, bytes);
   A(&e->d_dx, dxo * sizeof(double));
   if (ce == cudaSuccess) ce = cudaMalloc((void**)&e->d_mem, sizeof(MemberDev) * nsims);
+  if (ce == cudaSuccess) ce = cudaMalloc((void**)&e->d_ctr, sizeof(unsigned long long) * 12);
   if (ce == cudaSuccess) ce = cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking);
   if (ce == cudaSuccess) e->own_stream = true;
   for (int m = 0; m < nsims && ce == cudaSuccess; m++) {
@@ -299,6 +318,7 @@ extern "C" void gb_ensemble_destroy(gb_ensemble* e) {
   cudaFree(e->d_H);
   cudaFree(e->d_dx);
   cudaFree(e->d_mem);
+  cudaFree(e->d_ctr);
   cudaFree(e->d_bnd);
   cudaFree(e->d_red);
   if (e->own_stream && e->stream) cudaStreamDestroy(e->stream);
@@ -434,7 +454,7 @@ extern "C" int gb_ensemble_set_launch(gb_ensemble* e, int dir, int seg, int bloc
     gbh_set_error("gb_ensemble_set_launch: a tile form is -32, -64 or -128 (got %d)", seg);
     return GB_ERR_ARG;
   }
-  const int nseg = seg != 0 ? seg : e->seg[dir];
+  const int nseg = seg != 0 ? seg : e->hl[dir].seg;
   if (block == -1 && nseg >= 0) {
     gbh_set_error("gb_ensemble_set_launch: the persistent work-list form (block -1) takes a tile form");
     return GB_ERR_ARG;
@@ -443,10 +463,10 @@ extern "C" int gb_ensemble_set_launch(gb_ensemble* e, int dir, int seg, int bloc
     gbh_set_error("gb_ensemble_set_launch: block %d (a multiple of 32 up to 128, or -1)", block);
     return GB_ERR_ARG;
   }
-  e->seg[dir] = nseg;
+  e->hl[dir].seg = nseg;
   if (block == -1) e->persist[dir] = true;
   if (block > 0) {
-    e->block[dir] = block;
+    e->hl[dir].block = block;
     e->persist[dir] = false;
   }
   if (nseg >= 0) e->persist[dir] = false;
@@ -455,15 +475,17 @@ extern "C" int gb_ensemble_set_launch(gb_ensemble* e, int dir, int seg, int bloc
 
 extern "C" int gb_ensemble_get_launch(gb_ensemble* e, int dir, int* seg, int* block) {
   if (!e || dir < 0 || dir >= e->base.ndims || !seg || !block) { gbh_set_error("bad argument"); return GB_ERR_ARG; }
-  *seg = e->seg[dir];
-  *block = e->persist[dir] ? -1 : e->block[dir];
+  *seg = e->hl[dir].seg;
+  *block = e->persist[dir] ? -1 : e->hl[dir].block;
   return GB_OK;
 }
 
 extern "C" double gb_ensemble_time(const gb_ensemble* e) { return e ? e->t : 0.0; }
 
-// Threads per block and direction by timing whole graph-replayed steps
-// (directions tuned one after the other); the state is restored afterwards.
+// Block size of the float-pair kernels per direction by timing whole graph-replayed steps
+// (directions tuned one after the other); the state is restored afterwards.  The FP64 forms
+// are left to gb_ensemble_set_launch: they round differently, and tuning an ensemble does not
+// change its results.
 extern "C" int gb_ensemble_autotune(gb_ensemble* e, int reps) {
   if (!e) { gbh_set_error("null ensemble"); return GB_ERR_ARG; }
   if (reps < 1) reps = 1;
@@ -479,14 +501,16 @@ extern "C" int gb_ensemble_autotune(gb_ensemble* e, int reps) {
   CK(cudaEventCreate(&a));
   CK(cudaEventCreate(&b));
   int rc = GB_OK;
-  // (32, 128): blocks of up to 256 threads on large ensembles; -128, -64: of up to 128 / 64
   for (int d = 0; d < e->base.ndims && !rc; d++) {
     float best = 1e30f;
-    int bs = e->seg[d];
-    e->block[d] = 128;
+    HypLaunch bl = e->hl[d];
     e->persist[d] = false;
-    for (int sg : {32, -128, -64}) {
-      e->seg[d] = sg;
+    for (int cap : {0, 128, 64}) {
+      e->hl[d] = HypLaunch();
+      e->hl[d].seg += cap;
+      // every candidate on the same solution, on which the time depends
+      CK(cudaMemcpyAsync(e->d_u, save, bytes, cudaMemcpyDeviceToDevice, e->stream));
+      e->t = t0;
       rc = upload_table(e);
       if (!rc) rc = gb_ensemble_step(e, 1);
       if (rc) break;
@@ -498,10 +522,10 @@ extern "C" int gb_ensemble_autotune(gb_ensemble* e, int reps) {
       cudaEventElapsedTime(&ms, a, b);
       if (!rc && ms < best) {
         best = ms;
-        bs = sg;
+        bl = e->hl[d];
       }
     }
-    e->seg[d] = bs;
+    e->hl[d] = bl;
     if (!rc) rc = upload_table(e);
   }
   cudaEventDestroy(a);

@@ -570,16 +570,23 @@ __device__ __forceinline__ void iface_flux(const double (&wu)[6][ModelTraits<M>:
 // One thread's share of a launch: interfaces [sg*seg, min((sg+1)*seg, N)] of
 // the grid line with transverse index `tr` (other dimensions ascending, first
 // fastest), and the flux difference / epilogue of the cells in between.
+// GRAV (NavierStokes3D with Rusanov): the well-balanced gravity treatment --
+// the modified solution uC = [f u_{0..3}, P/(gamma-1)/g + f rho|v|^2/2]
+// (NavierStokes3DModifiedSolution.c:52-66), the dissipation factor
+// max(g_L, g_R) (NavierStokes3DUpwind.c:407) and, along a direction with
+// gravity, the source term of NavierStokes3DSource.c:38-112 subtracted from
+// the hyperbolic term of this direction (except when only that term is asked for).
 // WT (Euler2D, component-wise, Jiang-Shu: the adjoint's configuration): the wide
 // tape -- per interface uL, uR and, per component, the smoothness terms and
 // normalisation reciprocals of the f and u pairs (TAPE_WIDE doubles).
-template <int M, bool CHAR, int UPW, int DIR, bool ALTW = false, bool WT = false>
+template <int M, bool CHAR, int UPW, int DIR, bool ALTW = false, bool GRAV = false, bool WT = false>
 __device__ __forceinline__ void hyp_segment(const double* __restrict__ U, double* __restrict__ H,
                                             const double* __restrict__ dxinv, const DevGeom& G,
                                             const PhysParams& pp, const StageEpi& ep, int seg, long long tr,
                                             int sg) {
   constexpr int NV = ModelTraits<M>::NV, ND = ModelTraits<M>::ND;
   constexpr bool CC = NeedCC<M, CHAR, UPW>::value;
+  constexpr bool REL = RelFlux<GRAV>::value;
   const long long line = tr;
 
   long long pbase = (long long)G.g * G.stride[DIR];
@@ -598,8 +605,9 @@ __device__ __forceinline__ void hyp_segment(const double* __restrict__ U, double
   const double eps4 = 4.0 * pp.eps;
 
   double wu[6][NV], wf[6][NV], wuc[6];
-  double wgf[6], wgg[6];  // (gravity fields: not used here)
+  double wgf[6], wgg[6];  // gravity fields f, g (GRAV)
   CellAux<M> ax[6];
+  const bool src_dir = GRAV && pp.grav[DIR] != 0.0 && (ep.mode != EPI_HYP || ep.with_source);
 
   auto load = [&](int i) {
     const long long pt = pbase + (long long)fold_index(i, N, lo, hi) * sd;
@@ -608,7 +616,13 @@ __device__ __forceinline__ void hyp_segment(const double* __restrict__ U, double
     for (int v = 0; v < NV; v++) wu[5][v] = src[v];
     Prim<M> q = to_prim<M>(wu[5], pp);
     cell_flux<M, DIR>(q, wf[5]);
-    wuc[5] = ufunc_energy<M>(q, pp, wu[5][NV - 1]);
+    if (GRAV) {
+      wgf[5] = pp.gf[pt];
+      wgg[5] = pp.gg[pt];
+      wuc[5] = modified_energy<M>(q, wu[5][NV - 1], wgf[5], wgg[5], pp);
+    } else {
+      wuc[5] = ufunc_energy<M>(q, pp, wu[5][NV - 1]);
+    }
     if (CC) ax[5].rs = roe_side<M>(q);
     if (UPW == UPW_RUS) ax[5].c = rusanov_speed<M, DIR>(q, pp);
     else if (M == MODEL_EULER1D && UPW != UPW_ROE) ax[5].c = sound_speed<M>(q, pp);
@@ -622,6 +636,10 @@ __device__ __forceinline__ void hyp_segment(const double* __restrict__ U, double
         wf[p][v] = wf[p + 1][v];
       }
       wuc[p] = wuc[p + 1];
+      if (GRAV) {
+        wgf[p] = wgf[p + 1];
+        wgg[p] = wgg[p + 1];
+      }
       ax[p] = ax[p + 1];
     }
   };
@@ -631,14 +649,14 @@ __device__ __forceinline__ void hyp_segment(const double* __restrict__ U, double
     shift();
   }
 
-  double fIp[NV], SI[NV];
+  double fIp[NV], SI[NV], SIp[NV];
 #pragma unroll
-  for (int v = 0; v < NV; v++) fIp[v] = SI[v] = 0.0;
+  for (int v = 0; v < NV; v++) fIp[v] = SI[v] = SIp[v] = 0.0;
 
   for (int I = I0; I <= I1; I++) {
     load(I + 2);
     double fI[NV];
-    iface_flux<M, CHAR, UPW, DIR, ALTW, false, WT>(wu, wf, wuc, wgf, wgg, ax, pp, ep, eps4, false,
+    iface_flux<M, CHAR, UPW, DIR, ALTW, GRAV, WT>(wu, wf, wuc, wgf, wgg, ax, pp, ep, eps4, src_dir,
                                                    line * (N + 1) + I, fI, SI);
     if (ep.bnd && (I == 0 || I == N)) {
       long long ntr = 1;
@@ -647,7 +665,7 @@ __device__ __forceinline__ void hyp_segment(const double* __restrict__ U, double
         if (e != DIR) ntr *= G.dim[e];
       double Fb[NV];
 #pragma unroll
-      for (int v = 0; v < NV; v++) Fb[v] = fI[v] + wf[2][v];
+      for (int v = 0; v < NV; v++) Fb[v] = REL ? fI[v] + wf[2][v] : fI[v];
       boundary_flux<NV>(ep, I, N, line, ntr, Fb);
     }
 
@@ -657,11 +675,21 @@ __device__ __forceinline__ void hyp_segment(const double* __restrict__ U, double
       const long long off = (pbase + (long long)c * sd) * NV;
       const double dxi = dxinv[G.g + c];
       const bool finish = ep.last && ep.mode != EPI_HYP;
-      double kv[NV];
+      double kv[NV], term[NV];
+      if (src_dir) {
+        // [0, rho RT e_DIR, rho RT v_DIR] f of the cell (NavierStokes3DSource.c:92-97)
+        const double rho = wu[2][0], rRT = rho * pp.RT, f = wgf[2];
+        const double vd = rho == 0.0 ? 0.0 : wu[2][1 + DIR] * nr_rcp(rho);
+#pragma unroll
+        for (int v = 0; v < NV; v++) term[v] = 0.0;
+        term[1 + DIR] = rRT * f;
+        term[NV - 1] = (rRT * vd) * f;
+      }
 #pragma unroll
       for (int v = 0; v < NV; v++) {
         // centre-relative fluxes: F_I - F_{I-1} = (f_c - f_{c-1}) + (fI_I - fI_{I-1})
-        const double h = dxi * ((wf[2][v] - wf[1][v]) + (fI[v] - fIp[v]));
+        double h = REL ? dxi * ((wf[2][v] - wf[1][v]) + (fI[v] - fIp[v])) : dxi * (fI[v] - fIp[v]);
+        if (src_dir) h = fma(-term[v] * (SI[v] - SIp[v]), dxi, h);  // rhs = -hyp + source
         double hyp = ep.first ? h : H[off + v] + h;
         if (!finish) {
           H[off + v] = hyp;
@@ -692,7 +720,10 @@ __device__ __forceinline__ void hyp_segment(const double* __restrict__ U, double
       }
     }
 #pragma unroll
-    for (int v = 0; v < NV; v++) fIp[v] = fI[v];
+    for (int v = 0; v < NV; v++) {
+      fIp[v] = fI[v];
+      SIp[v] = SI[v];
+    }
     shift();
   }
 }
@@ -982,17 +1013,18 @@ hyp_tile_kernel(const double* __restrict__ U, double* __restrict__ H, const doub
   hyp_tile_body<M, CHAR, UPW, DIR, ALTW, TI, WT>(U, H, dxinv, G, pp, ep, ntrans, blockIdx.x);
 }
 
-template <int M, bool CHAR, int UPW, int DIR, bool ALTW, bool WT = false>
+template <int M, bool CHAR, int UPW, int DIR, bool ALTW, bool GRAV = false, bool WT = false>
 __global__ void __launch_bounds__(128)
 hyp_dir_kernel(const double* __restrict__ U, double* __restrict__ H, const double* __restrict__ dxinv,
                DevGeom G, PhysParams pp, StageEpi ep, int seg, int nseg, long long ntrans) {
   long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (tid >= ntrans * (long long)nseg) return;
-  hyp_segment<M, CHAR, UPW, DIR, ALTW, WT>(U, H, dxinv, G, pp, ep, seg, tid % ntrans, (int)(tid / ntrans));
+  hyp_segment<M, CHAR, UPW, DIR, ALTW, GRAV, WT>(U, H, dxinv, G, pp, ep, seg, tid % ntrans, (int)(tid / ntrans));
 }
 
-// All members of an ensemble advanced by one launch per direction: a block finds its
-// member by binary search over the start offsets, then works as in the single-grid kernel.
+// All members of an ensemble advanced by one launch per direction: a block (walkers: a
+// thread) finds its member by binary search over the start offsets, then works as in the
+// single-grid kernel.
 // The member that owns work item `w` of direction DIR (members' first items
 // ascending), with the stage pointers moved to its arrays.
 template <int DIR>
@@ -1018,23 +1050,135 @@ __device__ __forceinline__ const MemberDev& batched_member(const MemberDev* __re
   return m;
 }
 
-// All members in one launch (gbh_pair_flux.cuh): nblk blocks of T threads.
+// The float-pair form (gbh_pair_flux.cuh): nblk blocks of T threads.
 template <int M, bool CHAR, int UPW, int DIR>
-cudaError_t launch_batched_dir(const MemberDev* mem, int nmem, long long nblk, int T, const double* U, double* H,
-                               const double* dxinv, const PhysParams& pp, const StageEpi& ep, cudaStream_t s);
+cudaError_t launch_batched_pair(const MemberDev* mem, int nmem, long long nblk, int T, const double* U, double* H,
+                                const double* dxinv, const PhysParams& pp, const StageEpi& ep, cudaStream_t s);
+
+template <int M, bool CHAR, int UPW, int DIR>
+__global__ void __launch_bounds__(128)
+hyp_batched_kernel(const MemberDev* __restrict__ mem, int nmem, long long total, const double* __restrict__ U,
+                   double* __restrict__ H, const double* __restrict__ dxinv, PhysParams pp, StageEpi ep) {
+  long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (tid >= total) return;
+  StageEpi e = ep;
+  const MemberDev& m = batched_member<DIR>(mem, nmem, tid, e);
+  long long lt = tid - m.start[DIR];
+  long long ntr = m.ntrans[DIR];
+  const long long o = m.off;
+  hyp_segment<M, CHAR, UPW, DIR>(U + o, H ? H + o : nullptr, dxinv + m.dx_off[DIR], m.G, pp, e, m.seg[DIR],
+                                 lt % ntr, (int)(lt / ntr));
+}
+
+// Tile form of the batched kernel: one block per tile of TI interfaces of one
+// member's grid line; the members' tables count blocks instead of threads.
+template <int M, bool CHAR, int UPW, int DIR, int TI>
+__global__ void __launch_bounds__(TI)
+hyp_batched_tile_kernel(const MemberDev* __restrict__ mem, int nmem, const double* __restrict__ U,
+                        double* __restrict__ H, const double* __restrict__ dxinv, PhysParams pp, StageEpi ep) {
+  StageEpi e = ep;
+  const long long b = blockIdx.x;
+  const MemberDev& m = batched_member<DIR>(mem, nmem, b, e);
+  const long long o = m.off;
+  hyp_tile_body<M, CHAR, UPW, DIR, false, TI, false>(U + o, H ? H + o : nullptr, dxinv + m.dx_off[DIR], m.G, pp,
+                                                     e, m.ntrans[DIR], b - m.start[DIR]);
+}
+
+// Persistent work-list form of the batched tile kernel: a grid of as many blocks as
+// the SMs hold at once pulls tile indices from a work counter (one atomicAdd per
+// tile, by one thread of the block) until the launch's `total` tiles are taken.  The
+// loop is bounded: every fetch takes a new index, so a block stops after at most
+// total / gridDim + 1 fetches.  `counter` is zero when the launch starts.
+template <int M, bool CHAR, int UPW, int DIR, int TI>
+__global__ void __launch_bounds__(TI)
+hyp_batched_worklist_kernel(const MemberDev* __restrict__ mem, int nmem, long long total,
+                            unsigned long long* __restrict__ counter, const double* __restrict__ U,
+                            double* __restrict__ H, const double* __restrict__ dxinv, PhysParams pp, StageEpi ep) {
+  __shared__ long long s_tile;
+  for (;;) {
+    if (threadIdx.x == 0) s_tile = (long long)atomicAdd(counter, 1ULL);
+    __syncthreads();
+    const long long b = s_tile;
+    __syncthreads();  // every thread holds b before thread 0 fetches the next one
+    if (b >= total) return;
+    StageEpi e = ep;
+    const MemberDev& m = batched_member<DIR>(mem, nmem, b, e);
+    const long long o = m.off;
+    hyp_tile_body<M, CHAR, UPW, DIR, false, TI, false>(U + o, H ? H + o : nullptr, dxinv + m.dx_off[DIR], m.G, pp,
+                                                       e, m.ntrans[DIR], b - m.start[DIR]);
+  }
+}
+
+template <typename K>
+unsigned worklist_grid(K kernel, int threads, long long total) {
+  int dev = 0, sms = 0, per = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, 0);
+  long long g = (long long)(per > 0 ? per : 1) * (sms > 0 ? sms : 1);
+  return (unsigned)(g < total ? g : total);
+}
+
+// total = threads (walker, tile == 0) or blocks (tiles of `tile` interfaces).
+// counter != nullptr with a tile form: the persistent work-list kernel.
+template <int M, bool CHAR, int UPW, int DIR>
+cudaError_t launch_batched_fp64(const MemberDev* mem, int nmem, long long total, const double* U, double* H,
+                               const double* dxinv, const PhysParams& pp, const StageEpi& ep, int block, int tile,
+                               unsigned long long* counter, cudaStream_t s) {
+  if (total <= 0) return cudaSuccess;
+  if (counter && tile) {
+#define GBH_WL(TI)                                                                                       \
+  do {                                                                                                   \
+    auto k = hyp_batched_worklist_kernel<M, CHAR, UPW, DIR, TI>;                                         \
+    k<<<worklist_grid(k, TI, total), TI, 0, s>>>(mem, nmem, total, counter, U, H, dxinv, pp, ep);        \
+  } while (0)
+    if (tile == 32) GBH_WL(32);
+    else if (tile == 64) GBH_WL(64);
+    else if (tile == 128) GBH_WL(128);
+    else return cudaErrorInvalidValue;
+#undef GBH_WL
+    return cudaGetLastError();
+  }
+  if (tile == 32)
+    hyp_batched_tile_kernel<M, CHAR, UPW, DIR, 32><<<(unsigned)total, 32, 0, s>>>(mem, nmem, U, H, dxinv, pp, ep);
+  else if (tile == 64)
+    hyp_batched_tile_kernel<M, CHAR, UPW, DIR, 64><<<(unsigned)total, 64, 0, s>>>(mem, nmem, U, H, dxinv, pp, ep);
+  else if (tile == 128)
+    hyp_batched_tile_kernel<M, CHAR, UPW, DIR, 128><<<(unsigned)total, 128, 0, s>>>(mem, nmem, U, H, dxinv, pp, ep);
+  else if (tile != 0)
+    return cudaErrorInvalidValue;
+  else {
+    if (block <= 0) block = 128;
+    long long grid = (total + block - 1) / block;
+    hyp_batched_kernel<M, CHAR, UPW, DIR><<<(unsigned)grid, block, 0, s>>>(mem, nmem, total, U, H, dxinv, pp, ep);
+  }
+  return cudaGetLastError();
+}
+
+// The form of L: float pairs in blocks of T threads, else as launch_batched_fp64 (counter: the
+// work list).  total: blocks, or the walkers' threads.
+template <int M, bool CHAR, int UPW, int DIR>
+cudaError_t launch_batched_dir(const MemberDev* mem, int nmem, long long total, int T, const double* U, double* H,
+                               const double* dxinv, const PhysParams& pp, const StageEpi& ep, const HypLaunch& L,
+                               unsigned long long* counter, cudaStream_t s) {
+  if (L.pairs()) return launch_batched_pair<M, CHAR, UPW, DIR>(mem, nmem, total, T, U, H, dxinv, pp, ep, s);
+  return launch_batched_fp64<M, CHAR, UPW, DIR>(mem, nmem, total, U, H, dxinv, pp, ep, L.block,
+                                                L.seg < 0 ? -L.seg : 0, counter, s);
+}
 
 template <int M>
-cudaError_t launch_batched_model(int dir, int chr, int upw, const MemberDev* mem, int nmem, long long nblk, int T,
+cudaError_t launch_batched_model(int dir, int chr, int upw, const MemberDev* mem, int nmem, long long total, int T,
                                  const double* U, double* H, const double* dxinv, const PhysParams& pp,
-                                 const StageEpi& ep, cudaStream_t s) {
+                                 const StageEpi& ep, const HypLaunch& L, unsigned long long* counter, cudaStream_t s) {
   constexpr int ND = ModelTraits<M>::ND;
 #define GBH_B(C, W)                                                                                          \
   do {                                                                                                       \
-    if (dir == 0) return launch_batched_dir<M, C, W, 0>(mem, nmem, nblk, T, U, H, dxinv, pp, ep, s);         \
+    if (dir == 0)                                                                                            \
+      return launch_batched_dir<M, C, W, 0>(mem, nmem, total, T, U, H, dxinv, pp, ep, L, counter, s);        \
     if (ND > 1 && dir == 1)                                                                                  \
-      return launch_batched_dir<M, C, W, (ND > 1 ? 1 : 0)>(mem, nmem, nblk, T, U, H, dxinv, pp, ep, s);      \
+      return launch_batched_dir<M, C, W, (ND > 1 ? 1 : 0)>(mem, nmem, total, T, U, H, dxinv, pp, ep, L, counter, s); \
     if (ND > 2 && dir == 2)                                                                                  \
-      return launch_batched_dir<M, C, W, (ND > 2 ? 2 : 0)>(mem, nmem, nblk, T, U, H, dxinv, pp, ep, s);      \
+      return launch_batched_dir<M, C, W, (ND > 2 ? 2 : 0)>(mem, nmem, total, T, U, H, dxinv, pp, ep, L, counter, s); \
     return cudaErrorInvalidValue;                                                                            \
   } while (0)
   // Rusanov: Euler1D and NavierStokes3D (Euler2D offers none); the template
@@ -1054,7 +1198,7 @@ cudaError_t launch_batched_model(int dir, int chr, int upw, const MemberDev* mem
 #undef GBH_B
 }
 
-// The float-pair form (gbh_pair_flux.cuh), which the direction launcher prefers.
+// The float-pair form (gbh_pair_flux.cuh), the default.
 template <int M, bool CHAR, int UPW, int DIR, bool ALTW, bool GRAV>
 cudaError_t launch_pair(const double* U, double* H, const double* dxinv_dir, const DevGeom& G, const PhysParams& pp,
                         const StageEpi& ep, long long ntrans, int cap, cudaStream_t s);
@@ -1076,38 +1220,44 @@ cudaError_t launch_dir(const double* U, double* H, const double* dxinv_dir, cons
       return launch_pdl(hyp_lane_kernel<M, UPW, ALTW, 16>, nblk, 256, 0, s, U, H, dxinv_dir, G, pp, ep);
     }
   }
-  // Steger-Warming and the adjoint's tapes: the FP64 kernels.
+  // Float pairs unless a shape of the FP64 kernels is asked for; Steger-Warming and the
+  // adjoint's tapes have these only.
   constexpr bool PAIR = !WT && UPW != UPW_SWFS;
   constexpr bool TAPE = M == MODEL_EULER2D && !CHAR && UPW == UPW_ROE && !ALTW && !GRAV;
   if constexpr (PAIR) {
-    if (!TAPE || !ep.tape)
-      return launch_pair<M, CHAR, UPW, DIR, ALTW, GRAV>(U, H, dxinv_dir, G, pp, ep, ntrans, pair_cap_of(L.seg, L.block), s);
+    if (L.pairs() && (!TAPE || !ep.tape))
+      return launch_pair<M, CHAR, UPW, DIR, ALTW, GRAV>(U, H, dxinv_dir, G, pp, ep, ntrans, L.cap(), s);
   }
-  if constexpr (!PAIR || TAPE) {
-    if (L.seg < 0) {
-      // tiles of -seg interfaces (32, 64 or 128), one block each
-      const int ti = -L.seg;
-      const long long nblk = ntrans * ((N + ti - 2) / (ti - 1));
-      if (ti == 32)
-        hyp_tile_kernel<M, CHAR, UPW, DIR, ALTW, 32, WT><<<(unsigned)nblk, 32, 0, s>>>(U, H, dxinv_dir, G, pp, ep,
+  if (L.seg < 0 && !GRAV) {
+    // tiles of -seg interfaces (32, 64 or 128), one block each
+    const int ti = -L.seg;
+    const long long nblk = ntrans * ((N + ti - 2) / (ti - 1));
+    if (ti == 32)
+      hyp_tile_kernel<M, CHAR, UPW, DIR, ALTW, 32, WT><<<(unsigned)nblk, 32, 0, s>>>(U, H, dxinv_dir, G, pp, ep,
+                                                                                     ntrans);
+    else if (ti == 64)
+      hyp_tile_kernel<M, CHAR, UPW, DIR, ALTW, 64, WT><<<(unsigned)nblk, 64, 0, s>>>(U, H, dxinv_dir, G, pp, ep,
+                                                                                     ntrans);
+    else
+      hyp_tile_kernel<M, CHAR, UPW, DIR, ALTW, 128, WT><<<(unsigned)nblk, 128, 0, s>>>(U, H, dxinv_dir, G, pp, ep,
                                                                                        ntrans);
-      else if (ti == 64)
-        hyp_tile_kernel<M, CHAR, UPW, DIR, ALTW, 64, WT><<<(unsigned)nblk, 64, 0, s>>>(U, H, dxinv_dir, G, pp, ep,
-                                                                                       ntrans);
-      else
-        hyp_tile_kernel<M, CHAR, UPW, DIR, ALTW, 128, WT><<<(unsigned)nblk, 128, 0, s>>>(U, H, dxinv_dir, G, pp, ep,
-                                                                                         ntrans);
-      return cudaGetLastError();
-    }
-    const int seg = L.seg > 0 ? L.seg : 32;
-    const int nseg = (N + seg - 1) / seg;
-    const long long nthr = ntrans * nseg;
-    const int block = L.block > 0 ? L.block : 128;
-    const long long grid = (nthr + block - 1) / block;
-    hyp_dir_kernel<M, CHAR, UPW, DIR, ALTW, WT><<<(unsigned)grid, block, 0, s>>>(U, H, dxinv_dir, G, pp, ep, seg, nseg,
-                                                                                 ntrans);
     return cudaGetLastError();
   }
+  // a tile shape asked of a kernel without the tile form (gravity): segments that
+  // spread the line over about four warps per SM
+  int seg = L.seg > 0 && !L.pairs() ? L.seg : 32;
+  if (L.seg < 0) {
+    const long long want = sm_count() * 4LL * 32;
+    seg = (int)((ntrans * N + want - 1) / want);
+    seg = seg < 1 ? 1 : (seg > 64 ? 64 : seg);
+  }
+  const int nseg = (N + seg - 1) / seg;
+  const long long nthr = ntrans * nseg;
+  const int block = L.block > 0 ? L.block : 128;
+  const long long grid = (nthr + block - 1) / block;
+  hyp_dir_kernel<M, CHAR, UPW, DIR, ALTW, GRAV, WT><<<(unsigned)grid, block, 0, s>>>(U, H, dxinv_dir, G, pp, ep, seg,
+                                                                                     nseg, ntrans);
+  return cudaGetLastError();
 }
 
 template <int M, bool CHAR, int UPW, bool ALTW, bool GRAV = false>

@@ -100,22 +100,40 @@ struct ViscParams {
   int order;  // first derivatives: 4 (fourth-order central) or 2 (first-order one-sided)
 };
 
-// Per-launch configuration of the hyperbolic kernels.
+// SMs of the current device.
+inline int sm_count() {
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return 1;
+  return n > 0 ? n : 1;
+}
+
+// Per-launch configuration of the hyperbolic kernels: their form and its shape.
+//   seg >= GB_SEG_AUTO  the float-pair kernels of WENO5 (gbh_pair_flux.cuh); Steger-Warming
+//                       and CRWENO5: their default segments
+//   seg > 0             FP64 kernels, one thread per segment of that many interfaces
+//   seg = -t            FP64 kernels, tiles of t interfaces (32, 64, 128); -8, -16: lane groups
 struct HypLaunch {
-  int seg;         // interfaces walked by one thread
-  int block;       // threads per block
+  int seg = GB_SEG_AUTO;
+  int block = 128;  // threads per block
+  bool pairs() const { return seg >= GB_SEG_AUTO; }
+  // The most threads of a float-pair block: GB_SEG_AUTO + n asks for n, a block below 128 for
+  // itself, 0: by the grid's size.
+  int cap() const { return seg > GB_SEG_AUTO ? seg - GB_SEG_AUTO : (block > 0 && block < 128 ? block : 0); }
 };
 
 // Ensemble member as seen by the batched kernel: its geometry, where its
-// arrays start inside the batched arrays, which blocks of a launch along each direction
-// are its (from start[d]) and their shape (PairPlan in gbh_pair_flux.cuh).
+// arrays start inside the batched arrays, and which blocks (segment walkers: threads) of a
+// launch along each direction are its (from start[d]) with their shape: PairPlan's L, XL
+// (gbh_pair_plan.h) or the FP64 forms' nseg pieces of seg interfaces.
 struct MemberDev {
   DevGeom G;
   long long off;         // first value of the member in every state array
   long long dx_off[3];   // first dxinv value of each direction
-  long long start[3];    // first block of the member per direction
+  long long start[3];    // first block (walkers: thread) of the member per direction
   long long ntrans[3];
   int L[3], XL[3];
+  int nseg[3], seg[3];
   long long bnd_off[3];  // the member's conservation-check accumulators per direction
 };
 

@@ -152,9 +152,7 @@ extern "C" int gb_rhs_explicit_noalloc(const gb_config* cfg, const double* dxinv
   pp.wtype = c.weno_weights;
   pp.gf = pp.gg = nullptr;
   pp.RT = 1.0;  // no gravity here: grav[] stays zero, as in a solver without gravity
-  HypLaunch hl;
-  hl.seg = 32;
-  hl.block = 128;
+  const HypLaunch hl;
   StageEpi ep;
   memset(&ep, 0, sizeof(ep));
   ep.mode = EPI_RHS;

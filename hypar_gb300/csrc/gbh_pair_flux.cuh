@@ -1252,8 +1252,8 @@ hyp_batched_pair_kernel(const MemberDev* __restrict__ mem, int nmem, const doubl
 }
 
 template <int M, bool CHAR, int UPW, int DIR>
-cudaError_t launch_batched_dir(const MemberDev* mem, int nmem, long long nblk, int T, const double* U, double* H,
-                               const double* dxinv, const PhysParams& pp, const StageEpi& ep, cudaStream_t s) {
+cudaError_t launch_batched_pair(const MemberDev* mem, int nmem, long long nblk, int T, const double* U, double* H,
+                                const double* dxinv, const PhysParams& pp, const StageEpi& ep, cudaStream_t s) {
   if (nblk <= 0) return cudaSuccess;
   if (nblk > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
   auto k = hyp_batched_pair_kernel<M, CHAR, UPW, DIR>;

@@ -44,8 +44,5 @@ inline int pair_cap(long long cells) { return cells >= 150000 ? 256 : (cells >= 
 // SM leave 96 registers per thread, which their evaluation of flagged interfaces needs; the
 // others are the faster with 256 and 80 registers (vortex 1024^2 2.25 ms against 2.45).
 inline int pair_threads(bool ns3d, bool chr) { return ns3d && !chr ? 224 : 256; }
-// Threads per block asked for by a launch shape: a tile of t interfaces (seg = -t) or a
-// block below 128 threads is taken as the cap, anything else leaves it to pair_cap (0).
-inline int pair_cap_of(int seg, int block) { return seg <= -32 ? -seg : (block > 0 && block < 128 ? block : 0); }
 
 }  // namespace gbh

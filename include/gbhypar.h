@@ -251,17 +251,26 @@ int gb_solver_error(gb_solver *s, const double *uex, int layout, int mem, double
  * areas (BoundaryIntegral.c, CalculateConservationError.c). */
 int gb_solver_conservation_begin(gb_solver *s);
 int gb_solver_conservation_error(gb_solver *s, double *err);
-/* Launch shape of the fused kernels, per direction (values <= 0 keep the current
- * ones).  The WENO5 kernels choose the lines and cells of a block by the grid's size;
- * seg = -32, -64 or -128, or a block below 128, is the most threads a block may take.
- * Steger-Warming splitting and CRWENO5's flux pass walk seg interfaces per thread in
- * blocks of `block` threads (Steger-Warming with seg = -32, -64 or -128: tiles of that
- * many interfaces).  seg = -8 or -16 (Euler1D, component-wise WENO5, no gravity): tiles
- * of that many interfaces with 16 lanes per interface (for short 1-D lines). */
+/* Launch shape of the fused kernels, per direction (values <= 0 but the codes below keep the
+ * current ones).
+ *   seg >= GB_SEG_AUTO (the default): the library's choice.  WENO5: the float-pair kernels,
+ *     whose blocks take lines and cells by the grid's size; GB_SEG_AUTO + 32, 64, 96 or 128,
+ *     or a block below 128, is the most threads a block may take.  Steger-Warming: segments
+ *     of 32 interfaces; CRWENO5's flux pass: segments by the grid's size.
+ *   0 < seg < GB_SEG_AUTO: FP64 kernels in which a thread walks seg interfaces, in blocks of
+ *     `block` threads.
+ *   seg = -32, -64, -128: FP64 kernels in tiles of that many interfaces per block, one
+ *     interface per thread (the block is then the tile; gravity and CRWENO5 walk segments).
+ *   seg = -8, -16 (Euler1D, component-wise WENO5, no gravity): FP64 tiles of that many
+ *     interfaces with 16 lanes per interface (for short 1-D lines).
+ * The FP64 kernels agree with the float-pair ones to rounding and are the faster where most
+ * interfaces are rough (noise, a few points per wavelength). */
+#define GB_SEG_AUTO (1 << 30)
 int gb_solver_set_launch(gb_solver *s, int dir, int seg, int block);
 int gb_solver_get_launch(gb_solver *s, int dir, int *seg, int *block);
-/* Choose seg/block per direction by timing candidates on `reps` steps of the
- * resident solution (restored afterwards). */
+/* Choose form and shape per direction by timing candidates on `reps` steps of the
+ * resident solution (restored afterwards): the float-pair kernels, and the FP64 ones where
+ * they are faster by a tenth. */
 int gb_solver_autotune(gb_solver *s, int reps);
 /* 1 if every value of the resident interior solution is finite, else 0. */
 int gb_solver_check_finite(gb_solver *s, int *finite);
@@ -292,14 +301,16 @@ int gb_ensemble_set_state(gb_ensemble *e, int member, const double *u, int layou
 int gb_ensemble_get_state(gb_ensemble *e, int member, double *u, int layout, int mem);
 int gb_ensemble_step(gb_ensemble *e, int nsteps);
 double gb_ensemble_time(const gb_ensemble *e);
-/* Launch shape per direction, as gb_solver_set_launch (seg 0 keeps the current value):
- * one launch per stage and direction over all members (HyPar's ensemble mode,
- * src/TimeIntegration/TimeRK.c:164-170).  block = -1 with seg = -32, -64 or -128 asked
- * for a persistent launch; it is accepted and reported, and runs the same blocks. */
+/* Launch shape per direction, as gb_solver_set_launch (seg 0 keeps the current value): one
+ * launch per stage and direction over all members.  With a tile form, block = -1 selects the
+ * persistent work-list kernel (HyPar's ensemble mode, src/TimeIntegration/TimeRK.c:164-170, as
+ * one launch per stage and direction of as many blocks as the SMs hold, taking the members'
+ * tiles from an atomic counter), block > 0 the grid launch of one block per tile; get_launch
+ * reports -1 for the persistent form. */
 int gb_ensemble_set_launch(gb_ensemble *e, int dir, int seg, int block);
 int gb_ensemble_get_launch(gb_ensemble *e, int dir, int *seg, int *block);
-/* Choose the most threads per block per direction by timing graph-replayed steps
- * (state restored). */
+/* Choose the block size of the float-pair kernels per direction by timing graph-replayed
+ * steps (state restored); the results do not change. */
 int gb_ensemble_autotune(gb_ensemble *e, int reps);
 /* CalculateError of one member against its exact solution (as gb_solver_error). */
 int gb_ensemble_error(gb_ensemble *e, int member, const double *uex, int layout, int mem, double *err);
