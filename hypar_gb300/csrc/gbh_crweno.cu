@@ -35,6 +35,7 @@
 // Layout of the interface values (and of the elimination scratch):
 // [interface I][reconstruction k][component v][line], so that the threads of a
 // warp, which take consecutive lines, read and write consecutive addresses.
+#include "gbh_cr_plan.h"
 #include "gbh_hyp_impl.cuh"
 
 // Threads per block of the component-wise solve launch (a multiple of 32, at most 128).
@@ -784,11 +785,7 @@ static cudaError_t cr_dir(bool chr, const double* U, double* H, const double* dx
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  int seg = L.seg > 0 ? L.seg : 32;
-  // The back half walks short segments: 16 warps per SM hide the latency of its reads
-  // (64^3: two segments of 32 per line left 256 warps in all, 117 / 162 / 247 us).
-  const long long fill = G.dim[DIR] * ntrans / (152LL * 16 * 32);
-  if (seg > fill) seg = fill < 2 ? 2 : (int)fill;
+  const int seg = cr_segment(L.pairs() || L.seg < 0 ? 0 : L.seg, G.dim[DIR], ntrans, sm_count());
   const int nseg = (G.dim[DIR] + seg - 1) / seg;
   const long long nthr = ntrans * nseg;
   const int block = L.block > 0 ? L.block : 128;
