@@ -917,7 +917,10 @@ extern "C" int gb_solver_autotune(gb_solver* s, int reps) {
       if (tiles) probe = std::min(probe, timed(N < 32 ? -32 : -64, 128));
       fp64 = probe <= 3.0f * pair;
     } else if (c.hyp_scheme == GB_SCHEME_CRWENO5) {
-      timed(GB_SEG_AUTO, 128);
+      // the line solves, most of the time, do not depend on the segment
+      const float pair = timed(GB_SEG_AUTO, 128);
+      best /= 1.1f;
+      fp64 = timed(segs[0], 64) <= 1.3f * pair;
     }
     for (int sg : {8, 16, 24, 32, 48, 64}) segs.push_back(sg);
     // Small grids (at most four waves of 4 warps per SM at one interface per

@@ -109,8 +109,8 @@ inline int sm_count() {
 }
 
 // Per-launch configuration of the hyperbolic kernels: their form and its shape.
-//   seg >= GB_SEG_AUTO  the float-pair kernels of WENO5 (gbh_pair_flux.cuh); Steger-Warming
-//                       and CRWENO5: their default segments
+//   seg >= GB_SEG_AUTO  the float-pair kernels of WENO5 (gbh_pair_flux.cuh) and CRWENO5;
+//                       Steger-Warming: segments of 32
 //   seg > 0             FP64 kernels, one thread per segment of that many interfaces
 //   seg = -t            FP64 kernels, tiles of t interfaces (32, 64, 128); -8, -16: lane groups
 struct HypLaunch {

@@ -255,10 +255,10 @@ int gb_solver_conservation_error(gb_solver *s, double *err);
  * current ones).
  *   seg >= GB_SEG_AUTO (the default): the library's choice.  WENO5: the float-pair kernels,
  *     whose blocks take lines and cells by the grid's size; GB_SEG_AUTO + 32, 64, 96 or 128,
- *     or a block below 128, is the most threads a block may take.  Steger-Warming: segments
- *     of 32 interfaces; CRWENO5's flux pass: segments by the grid's size.
- *   0 < seg < GB_SEG_AUTO: FP64 kernels in which a thread walks seg interfaces, in blocks of
- *     `block` threads.
+ *     or a block below 128, is the most threads a block may take.  CRWENO5: float pairs,
+ *     the flux pass in segments by the grid's size.  Steger-Warming: segments of 32 interfaces.
+ *   0 < seg < GB_SEG_AUTO: FP64 kernels in which a thread walks seg interfaces (CRWENO5: in
+ *     the flux pass), in blocks of `block` threads.
  *   seg = -32, -64, -128: FP64 kernels in tiles of that many interfaces per block, one
  *     interface per thread (the block is then the tile; gravity and CRWENO5 walk segments).
  *   seg = -8, -16 (Euler1D, component-wise WENO5, no gravity): FP64 tiles of that many

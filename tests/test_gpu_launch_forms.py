@@ -37,9 +37,15 @@ def rough(case, a, seed=5):
     return case
 
 
+def with_scheme(case, scheme):
+    case.hyp_scheme = scheme
+    return case
+
+
 MAKE = {"euler1d": lambda: C.sod(128, n_iter=2), "euler2d": lambda: C.vortex(40, n_iter=2),
         "navierstokes3d": lambda: C.isotropic_turbulence(14, n_iter=2),
-        "gravity": lambda: C.rising_thermal_bubble(16, n_iter=2)}
+        "gravity": lambda: C.rising_thermal_bubble(16, n_iter=2),
+        "crweno5": lambda: with_scheme(C.vortex(40, n_iter=2), "crweno5")}
 
 
 @pytest.mark.parametrize("shape", [(16, 64), (-32, 0), (-128, 0)], ids=["walker", "tile32", "tile128"])
