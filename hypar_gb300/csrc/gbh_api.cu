@@ -836,12 +836,12 @@ extern "C" int gb_solver_get_launch(gb_solver* s, int dir, int* seg, int* block)
 // Launch-shape autotuner: each candidate is timed on `reps` steps of the resident
 // solution, which is restored afterwards.  The float-pair kernels first, with blocks of the
 // grid's size, 64 and 128 threads.  The FP64 kernels are the faster where most interfaces
-// leave the pairs' bound (3-D turbulence of 24^3: tiles 0.93 ms per step against 1.30) and up
-// to six times slower elsewhere, so one of their tiles and one of their walkers are tried, and
-// the rest only where one of the two is within three times the best pair form.  Walkers spread
-// evenly over the SMs (a partial last wave idles SMs) against the per-segment overhead (a
-// six-cell window warm-up and one extra interface): segment lengths that give 1..4 full waves
-// of 4 warps per SM, plus fixed lengths.
+// leave the pairs' bound (3-D turbulence of 24^3: tiles 0.63 ms per step against 0.93) and up
+// to six times slower elsewhere, so one of their shapes is tried, and the rest only where it
+// takes at most three times the best pair form.  Walkers spread evenly over the SMs (a partial
+// last wave idles SMs) against the per-segment overhead (a six-cell window warm-up and one
+// extra interface): segment lengths that give 1..4 full waves of 4 warps per SM, plus fixed
+// lengths.
 extern "C" int gb_solver_autotune(gb_solver* s, int reps) {
   if (!s) { gbh_set_error("null solver"); return GB_ERR_ARG; }
   if (reps < 1) reps = 1;
@@ -913,9 +913,7 @@ extern "C" int gb_solver_autotune(gb_solver* s, int reps) {
       // lane groups of 8 / 16 interfaces (Euler1D component-wise: short lines)
       if (!s->gravity && c.model == GB_MODEL_EULER1D && c.interp == GB_INTERP_COMPONENTS)
         for (int ti : {8, 16}) timed(-ti, 128);
-      float probe = timed(segs[0], 128);
-      if (tiles) probe = std::min(probe, timed(N < 32 ? -32 : -64, 128));
-      fp64 = probe <= 3.0f * pair;
+      fp64 = timed(tiles ? (N < 32 ? -32 : -64) : segs[0], 128) <= 3.0f * pair;
     } else if (c.hyp_scheme == GB_SCHEME_CRWENO5) {
       // the line solves, most of the time, do not depend on the segment
       const float pair = timed(GB_SEG_AUTO, 128);

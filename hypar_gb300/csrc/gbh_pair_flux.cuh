@@ -14,7 +14,7 @@
 // interface takes the FP64 evaluation (iface_flux) instead where
 //   - its terms exceed a bound times its flux scale (rho lam, rho lam^2, rho lam H with
 //     lam = |u_n| + a; pair_bound, dissipation terms at the dissipation's own speed),
-//   - what the characteristic projections add up exceeds one (proj_bound): a field may cancel
+//   - what the characteristic projections add up exceeds one (PROJ_BOUND): a field may cancel
 //     out of large differences, their rounding does not,
 //   - a scale of the states or the fluxes leaves the range 2^-44 .. 2^100 (scales_in_range), a
 //     weight's sum leaves its own, or anything is not finite:
@@ -36,14 +36,14 @@ struct PEig {
 // Set so that a right-hand side is no further from one in extended precision than that of
 // the FP64 kernels: over waves of 6 to 100 cells and noise of 0.1 to 8 %, root mean square in
 // units of 2^-53 of the flux scale over the spacing, 1-D 0.22-0.63 (FP64 kernels 0.27-0.63),
-// 2-D 0.20-0.51 (0.21-0.51), 3-D component-wise 0.23-0.40 (0.44-0.57; there 2^-7 is enough),
+// 2-D 0.20-0.51 (0.21-0.51; at worst 3 % more, 0.263 for 0.256), 3-D component-wise 0.23-0.40 (0.44-0.57; there 2^-7 is enough),
 // 3-D characteristic 0.31-0.60 (0.45-0.73).  With 2^-7 and without the projections' bound a
-// wave of 6 cells was 0.67 off for 0.37.  Time: Euler2D ensemble 16.9 -> 20.2 ms, the other
-// workloads within 3 %.
+// wave of 6 cells was 0.67 off for 0.37, one of 24 cells (characteristic) 0.45 for 0.24.
+// Time: Euler2D ensemble 16.9 -> 19.0 ms, the other workloads within 5 %.
 __host__ __device__ constexpr float pair_bound(int model, bool chr) {
   return 12.0f * (model == MODEL_NS3D ? (chr ? 0.001953125f : 0.0078125f) : 0.0009765625f);  // 2^-9, 2^-7, 2^-10
 }
-__host__ __device__ constexpr float proj_bound(int model) { return model == MODEL_NS3D ? 3.0e38f : 1.0f; }
+constexpr float PROJ_BOUND = 1.0f;  // 1-D and 2-D (3-D needs none)
 
 // Whether an interface's scales (density, speed, enthalpy) are such that pairs hold its terms:
 // to_pair drops what lies below 2^-103, which has to be below 2^-53 of the states and the
@@ -640,7 +640,8 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
   constexpr bool CC = LY::CC, NEEDC = LY::NEEDC, STATES = LY::STATES;
   // a block evaluates its flagged interfaces together, else each thread its own
   constexpr bool COOP = !GRAV && !(M == MODEL_NS3D && CHAR);
-  constexpr float BOUND = pair_bound(M, CHAR), PROJ_BOUND = proj_bound(M);
+  constexpr float BOUND = pair_bound(M, CHAR);
+  constexpr bool PROJ = M != MODEL_NS3D;
   const int T = blockDim.x, S = T + 4, t = threadIdx.x;
   double* sf = sm;
   ff* sd = (ff*)(sf + NV * S);  // rows 0..NV-1: f, NV..2NV-1: u, then the modified solution and g
@@ -946,8 +947,8 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
           if (h) parts(xc + k, gc[GRAV ? k : 0], tc[GRAV ? k : 0]);
         }
       }
-      float p1, p2, p3;  // of the third differences
-      {
+      float p1 = 0.0f, p2 = 0.0f, p3 = 0.0f;  // of the third differences
+      if (PROJ) {
         const ff* y = GRAV && h ? xc : x;
         const float q0 = terms(y), q1 = terms(y + 1), q2 = terms(y + 2), q3 = terms(y + 3), q4 = terms(y + 4);
         p1 = q0 + 2.0f * q1 + q2;
@@ -981,7 +982,7 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
         if (v < 2) mag = mag * sc01;
         ok = ok & (mag <= 3.0e38f);  // (the maxima below drop a NaN)
         const float w2 = h == 0 ? W.r3.h - W.l3.h : W.r3.h + W.l3.h - 1.0f;
-        const float proj = ffma(W.r1.h, p3, ffma(W.l1.h, p1, fabsf(w2) * p2));
+        const float proj = PROJ ? ffma(W.r1.h, p3, ffma(W.l1.h, p1, fabsf(w2) * p2)) : 0.0f;
         if (h == 0) {
           pf = fmaxf(pf, proj);
           sx[v * S + w] = weno_sum6(W, t1, t2, t3);
@@ -1066,7 +1067,8 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
     // the fields' strengths are densities (shear: momenta) times a speed for f
     const float s0 = rho * lam, sm1 = s0 * lam;
     ok = ok & scales_in_range(rho, lam, Hs, GRAV ? kap.h : 1.0f) & (ffma(alm, ua, ma) <= BOUND * s0) &
-         (ffma(alm, us, ms) <= BOUND * sm1) & (ffma(alm, pu, pf) <= PROJ_BOUND * s0);
+         (ffma(alm, us, ms) <= BOUND * sm1);
+    if (PROJ) ok = ok & (ffma(alm, pu, pf) <= PROJ_BOUND * s0);
     if (grav_dir) {
       const float rt = (float)term[0];
       ok = ok & (magg * rt <= BOUND * s0) & source_in_range(rt, lam, sm1, s0 * Hs);
