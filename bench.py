@@ -51,14 +51,19 @@ UNIT = "cell-component updates/s"
 # with the launch shapes the autotuner picks at full size, whose per-cell work is
 # that of the full grid to within the segment-boundary share).
 FP64_PER_CELL_STEP = {
-    "vortex": {"pairs": {"flops": 492.7, "instr": 447.5, "captured": "1024^2 (the full grid)"}},
+    "vortex": {"pairs": {"flops": 519.2, "instr": 460.7, "captured": "1024^2 (the full grid)"}},
     "sod": {"lanes": {"flops": 3654.7, "instr": 2455.2, "captured": "1024 (the full grid), lane groups of 16"}},
-    "tgv": {"pairs": {"flops": 1395.0, "instr": 1238.3, "captured": "128^3"}},
-    "rtb": {"pairs": {"flops": 1360.7, "instr": 1188.4, "captured": "128^3"}},
-    "rtb64": {"pairs": {"flops": 1864.3, "instr": 1618.3, "captured": "64^3 (the full grid)"}},
-    "dns": {"pairs": {"flops": 1053.8, "instr": 932.5, "captured": "128^3"}},
-    "dns64cr": {"pairs": {"flops": 11671.3, "instr": 7694.7, "captured": "64^3 (the full grid)"}},
+    "tgv": {"pairs": {"flops": 1479.9, "instr": 1279.1, "captured": "128^3"}},
+    "rtb": {"pairs": {"flops": 1382.4, "instr": 1208.7, "captured": "128^3"}},
+    "rtb64": {"pairs": {"flops": 1892.9, "instr": 1646.8, "captured": "64^3 (the full grid)"}},
+    "dns": {"pairs": {"flops": 1117.4, "instr": 964.9, "captured": "128^3"}},
+    "dns64cr": {"pairs": {"flops": 11702.7, "instr": 7710.4, "captured": "64^3 (the full grid)"}},
 }
+def kernel_form(seg):
+    """The form a launch shape selects (GB_SEG_AUTO and above: float pairs)."""
+    return "lanes" if seg in (-8, -16) else "pairs" if seg >= 1 << 30 else "fp64"
+
+
 # DRAM bytes (read + write) per cell of one launch (x launch / y launch with the RK
 # update), from a capture of the default 1024^2 run (the 34 MB state partly stays in L2).
 DRAM_BYTES_PER_CELL = {"vortex": {("hyp_x", "pairs"): 32.68, ("hyp_y", "pairs"): 128.78}}
@@ -327,8 +332,7 @@ def run_ours(args, case, desc, ws, rank, local):
         bytes_per_launch = cells * 8.0 * nv * 2  # read U, write the partial hyperbolic term
     achieved_gbs = bytes_per_launch / avg_launch_s / 1e9
     cls_dir = "xyz".index(cls[-1]) if cls.startswith("hyp_") else 0
-    seg0 = tuned[cls_dir][0] if tuned else 0
-    form = "lanes" if seg0 in (-8, -16) else "pairs"
+    form = kernel_form(tuned[cls_dir][0])
     traffic = DRAM_BYTES_PER_CELL.get(args.workload, {}).get((cls, form))
     roofline = {"bound": "hbm", "achieved": achieved_gbs, "peak": hbm_peak, "unit": "GB/s",
                 "frac": achieved_gbs / hbm_peak, "traffic": traffic * cells if traffic else None,
@@ -339,7 +343,7 @@ def run_ours(args, case, desc, ws, rank, local):
                 "algorithmic_bytes_per_launch": bytes_per_launch}
     step_bytes = cells * sum(stage_bytes(cfg, st) + (8.0 * nv * 2) * (cfg.ndims - 1)
                              for st in range(cfg.rk_nstages))
-    forms = ["lanes" if sg in (-8, -16) else "pairs" for sg, _ in tuned]
+    forms = [kernel_form(sg) for sg, _ in tuned]
     known = FP64_PER_CELL_STEP.get(args.workload, {}) if not args.size else {}
     fw = None
     if known and all(f in known for f in forms):

@@ -1205,13 +1205,11 @@ __device__ __forceinline__ void pair_body(const double* __restrict__ U, double* 
   }
 }
 
-// Blocks of 256 threads (3-D component-wise: 224, pair_threads) per SM the kernels are held
-// to.  Bound by issue slots and latency
-// (some 6000 mostly FP32 instructions per thread against 75 FP64 ones): two blocks (128
-// registers) left the schedulers idle half of the time; three (80 registers; spills in the
-// FP64 evaluation only) take the Taylor-Green 256^3 directions from 75.9 to 61.4 ms per RK4
-// step and the 1024^2 vortex from 3.12 to 2.56 ms per step, four (64 registers) are no
-// faster (61.7 and 2.54 ms; shared memory allows three).
+// Blocks (pair_threads) per SM the kernels are held to.  Bound by issue slots and latency
+// (6,000 to 10,000 mostly FP32 instructions per thread against 60-150 FP64 ones): two blocks
+// (128 registers) left the schedulers idle half of the time; three (80 registers; spills in
+// the FP64 evaluation only) took the 1024^2 vortex from 3.12 to 2.56 ms per step when they were
+// brought in, four (64 registers) were no faster (2.54 ms; shared memory allows three).
 constexpr int PAIR_MINB = 3;
 template <int M, bool CHAR, int UPW, int DIR, bool ALTW, bool GRAV>
 __global__ void __launch_bounds__((M == MODEL_NS3D && !CHAR ? 224 : 256), PAIR_MINB)

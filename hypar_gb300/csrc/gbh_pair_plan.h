@@ -40,9 +40,9 @@ inline PairPlan pair_plan(int N, long long nlines, int dir, int cap, bool fixed 
 // 157 / 181, 320^2 343 / 331 / 346, 384^2 432 / 419 / 406, 640^2 1096 / 1058 / 989.
 inline int pair_cap(long long cells) { return cells >= 150000 ? 256 : (cells >= 30000 ? 128 : 64); }
 
-// Most threads of a block.  The 3-D component-wise kernels take 224: three such blocks per
-// SM leave 96 registers per thread, which their evaluation of flagged interfaces needs; the
-// others are the faster with 256 and 80 registers (vortex 1024^2 2.25 ms against 2.45).
+// Most threads of a block: 224 in the 3-D component-wise kernels (Taylor-Green 256^3 71.1 ms per
+// step against 72.2 with 256, bubble 64^3 1.93 against 1.96), 256 in the others (vortex 1024^2
+// 2.25 ms against 2.45 with 224).
 inline int pair_threads(bool ns3d, bool chr) { return ns3d && !chr ? 224 : 256; }
 
 }  // namespace gbh

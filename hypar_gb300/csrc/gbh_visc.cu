@@ -23,7 +23,7 @@
 // that is below a quarter of the rounding of the convective flux (rho a^2) it is added to.
 // visc_q checks this, and any point that fails (or leaves the pairs' range, or is not
 // finite) turns the whole evaluation to FP64.  Temperature derivatives stay in FP64.
-// 256^3: 8.30 -> 2.5 ms per evaluation.
+// 256^3: 8.30 -> 2.6 ms per evaluation.
 #include "gbh_internal.h"
 #include "gbh_pair.cuh"
 
